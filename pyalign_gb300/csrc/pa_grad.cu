@@ -28,29 +28,57 @@ struct GradParams {
 	float *dgap;  // 4 per pair: open_s, extend_s, open_t, extend_t
 };
 
-__global__ void path_grad_kernel(GradParams p) {
-	const int64_t k = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-	if (k >= p.batch) return;
+// A warp per pair, 32 path steps at a time.  The path is read once and nothing depends on the
+// previous step, so what bounds the kernel is the round trips to memory of one pair's chain:
+// a thread per pair paid one for each of its few hundred steps (8-byte loads of 32 different
+// paths per warp), a warp pays one per 32 steps, with coalesced loads, and the next 32 points
+// are in flight while these are handled.  The visited cells of a path are distinct, so the
+// lanes add to dS without atomics; the gap counts are integers, summed over the lanes at the
+// end.  1,024 pairs of 100..400 with dS: 429 -> 46 us; 4,096 pairs of 64..256, gap counts only:
+// 104 -> 8 us.
+__global__ void __launch_bounds__(128) path_grad_kernel(GradParams p) {
+	const int64_t k = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+	const int lane = threadIdx.x & 31;
+	if (k >= p.batch) return;  // whole warps
 	const float g = p.grad[k];
 	const int n = p.path_len[k];
 	const int32_t *P = p.paths + p.path_off[k];
 	float *d = p.dS ? p.dS + p.ds_off[k] : nullptr;
 	int open_s = 0, ext_s = 0, open_t = 0, ext_t = 0;
-	for (int q = 0; q + 1 < n; q++) {
-		const int u0 = P[2 * q], v0 = P[2 * q + 1], u1 = P[2 * q + 2], v1 = P[2 * q + 3];
-		if (u0 < 0 || v0 < 0) break;
-		if (p.dtw) {
-			if (d) d[int64_t(u0) * p.ss + int64_t(v0) * p.st] += g;
-		} else if (u1 == u0 - 1 && v1 == v0 - 1) {
-			if (d) d[int64_t(u0) * p.ss + int64_t(v0) * p.st] += g;
-		} else if (v1 == v0 && u1 < u0) {
-			open_s += 1;
-			ext_s += u0 - u1 - 1;
-		} else if (u1 == u0 && v1 < v0) {
-			open_t += 1;
-			ext_t += v0 - v1 - 1;
+	// lane l holds point q0 + l; its successor comes from lane l + 1, lane 31's from memory
+	auto point = [&](int q) { return q < n ? make_int2(P[2 * q], P[2 * q + 1]) : make_int2(-1, -1); };
+	int2 cur = point(lane);
+	for (int q0 = 0; q0 + 1 < n; q0 += 32) {
+		const int2 ahead = point(q0 + 32 + lane);
+		int u1 = __shfl_down_sync(0xffffffffu, cur.x, 1), v1 = __shfl_down_sync(0xffffffffu, cur.y, 1);
+		const int ux = __shfl_sync(0xffffffffu, ahead.x, 0), vx = __shfl_sync(0xffffffffu, ahead.y, 0);
+		if (lane == 31) {
+			u1 = ux;
+			v1 = vx;
 		}
+		const int u0 = cur.x, v0 = cur.y;
+		const bool step = q0 + lane + 1 < n;
+		const uint32_t neg = __ballot_sync(0xffffffffu, step && (u0 < 0 || v0 < 0));
+		if (step && (neg == 0 || lane < __ffs(int(neg)) - 1)) {  // steps before the first negative point
+			if (p.dtw || (u1 == u0 - 1 && v1 == v0 - 1)) {
+				if (d) d[int64_t(u0) * p.ss + int64_t(v0) * p.st] += g;
+			} else if (v1 == v0 && u1 < u0) {
+				open_s += 1;
+				ext_s += u0 - u1 - 1;
+			} else if (u1 == u0 && v1 < v0) {
+				open_t += 1;
+				ext_t += v0 - v1 - 1;
+			}
+		}
+		if (neg) break;
+		cur = ahead;
 	}
+	if (!p.dgap) return;
+	open_s = __reduce_add_sync(0xffffffffu, open_s);
+	ext_s = __reduce_add_sync(0xffffffffu, ext_s);
+	open_t = __reduce_add_sync(0xffffffffu, open_t);
+	ext_t = __reduce_add_sync(0xffffffffu, ext_t);
+	if (lane != 0) return;
 	if (n > 0 && p.global && !p.dtw) {
 		const int ul = P[2 * (n - 1)], vl = P[2 * (n - 1) + 1];
 		if (ul < 0 && vl >= 0) {  // D(-1, vl) = w_t(vl + 1)
@@ -61,13 +89,11 @@ __global__ void path_grad_kernel(GradParams p) {
 			ext_s += ul;
 		}
 	}
-	if (p.dgap) {
-		const float c = p.gap_sign * g;
-		p.dgap[4 * k + 0] = c * float(open_s);
-		p.dgap[4 * k + 1] = c * float(ext_s);
-		p.dgap[4 * k + 2] = c * float(open_t);
-		p.dgap[4 * k + 3] = c * float(ext_t);
-	}
+	const float c = p.gap_sign * g;
+	p.dgap[4 * k + 0] = c * float(open_s);
+	p.dgap[4 * k + 1] = c * float(ext_s);
+	p.dgap[4 * k + 2] = c * float(open_t);
+	p.dgap[4 * k + 3] = c * float(ext_t);
 }
 
 }  // namespace
@@ -93,7 +119,7 @@ extern "C" pa_status pa_path_gradients(int32_t type, int32_t locality, int32_t d
 	p.ss = stride_s;
 	p.st = stride_t;
 	p.dgap = dgap;
-	path_grad_kernel<<<int((batch + 127) / 128), 128, 0, reinterpret_cast<cudaStream_t>(stream)>>>(p);
+	path_grad_kernel<<<unsigned((batch + 3) / 4), 128, 0, reinterpret_cast<cudaStream_t>(stream)>>>(p);
 	return cudaGetLastError() == cudaSuccess ? PA_OK : PA_ERR_CUDA;
 }
 
