@@ -1197,6 +1197,133 @@ pa_status run_wsb(pa_solver *s, const Input &in, const std::vector<int32_t> &ls,
 	return PA_OK;
 }
 
+// General gap costs without the cell matrices: the tiled sweep (pa_wsb_tile.cu), scores and
+// (with `maps`) one alignment per pair.  Everything the kernels read besides the inputs -- gap
+// costs, borders, offsets, the tile list -- is staged in one pinned block and one copy.
+pa_status run_wsb_tiles(pa_solver *s, const Input &in, const std::vector<int32_t> &ls, const std::vector<int32_t> &lt,
+                        int *launches, int32_t *maps) {
+	cudaStream_t st = s->stream;
+	const int64_t B = in.batch;
+	constexpr int T = WSB_TILE;
+	const size_t ns = s->left_D.size(), nt = s->top_D.size();
+	// tiles by anti-diagonal of tiles, all pairs' tiles of one before the next: a tile waits on
+	// its left and upper neighbours only, which come earlier
+	std::vector<int64_t> voff(size_t(B) + 1, 0);
+	std::vector<int32_t> poff(size_t(B) + 1, 0);
+	std::vector<int64_t> first;  // tiles of each anti-diagonal, then its first place in the list
+	for (int64_t k = 0; k < B; k++) {
+		const int64_t NI = (ls[size_t(k)] + T - 1) / T, NJ = (lt[size_t(k)] + T - 1) / T;
+		const bool cells = NI > 0 && NJ > 0;
+		voff[size_t(k) + 1] = voff[size_t(k)] + (cells ? NI * NJ * T * T : 0);
+		poff[size_t(k) + 1] = int32_t(poff[size_t(k)] + (cells ? NI + NJ : 0));
+		if (!cells) continue;
+		if (int64_t(first.size()) < NI + NJ) first.resize(size_t(NI + NJ), 0);
+		for (int64_t d = 0; d < NI + NJ - 1; d++)
+			first[size_t(d) + 1] += std::min(NI - 1, d) - std::max<int64_t>(0, d - (NJ - 1)) + 1;
+	}
+	for (size_t d = 1; d < first.size(); d++) first[d] += first[d - 1];
+	const int64_t ntiles = first.empty() ? 0 : first.back();
+	if (ntiles >= (int64_t(1) << 31) - 4096) return fail(PA_ERR_LENGTH, "too many tiles in one launch");
+	size_t o = 0;
+	auto room = [&](size_t nbytes) {
+		const size_t at = o;
+		o = (o + nbytes + 15) & ~size_t(15);
+		return at;
+	};
+	const size_t o_left = room(ns * 4), o_top = room(nt * 4), o_gs = room((ns + T) * 4), o_gt = room((nt + T) * 4),
+	             o_voff = room(size_t(B + 1) * 8), o_poff = room(size_t(B + 1) * 4), o_tiles = room(size_t(ntiles) * 8),
+	             o_tab = room(in.form == F_INDEXED ? size_t(in.table_rows * in.table_cols) * 4 : 0);
+	PA_CUDA(s->h_stage.ensure(o));  // free again: every general-gap solve ends with a wait for its stream
+	PA_CUDA(s->d_gen.ensure(o));
+	unsigned char *h = s->h_stage.as<unsigned char>(), *d = s->d_gen.as<unsigned char>();
+	std::memcpy(h + o_left, s->left_D.data(), ns * 4);
+	std::memcpy(h + o_top, s->top_D.data(), nt * 4);
+	float *gs = reinterpret_cast<float *>(h + o_gs), *gt = reinterpret_cast<float *>(h + o_gt);
+	for (size_t k = 0; k < ns + T; k++) gs[k] = k < ns ? -s->gen_s[k] : 0.0f;
+	for (size_t k = 0; k < nt + T; k++) gt[k] = k < nt ? -s->gen_t[k] : 0.0f;
+	std::memcpy(h + o_voff, voff.data(), size_t(B + 1) * 8);
+	std::memcpy(h + o_poff, poff.data(), size_t(B + 1) * 4);
+	int2 *tiles = reinterpret_cast<int2 *>(h + o_tiles);
+	for (int64_t k = 0; k < B; k++) {
+		if (ls[size_t(k)] == 0 || lt[size_t(k)] == 0) continue;
+		const int NI = (ls[size_t(k)] + T - 1) / T, NJ = (lt[size_t(k)] + T - 1) / T;
+		for (int dg = 0; dg < NI + NJ - 1; dg++)
+			for (int I = std::max(0, dg - (NJ - 1)); I <= std::min(NI - 1, dg); I++)
+				tiles[first[size_t(dg)]++] = make_int2(int(k), (I << 16) | (dg - I));
+	}
+	// (device-resident tables join by a copy of their own below)
+	if (in.form == F_INDEXED && in.location == PA_HOST && o > o_tab)
+		std::memcpy(h + o_tab, in.table, size_t(in.table_rows * in.table_cols) * 4);
+	PA_CUDA(pa_copy(s, d, h, o, cudaMemcpyHostToDevice, st));
+	if (in.form == F_INDEXED && in.location == PA_DEVICE)
+		PA_CUDA(pa_copy(s, d + o_tab, in.table, size_t(in.table_rows * in.table_cols) * 4, cudaMemcpyDeviceToDevice, st));
+	PA_CUDA(s->d_wsb_vals.ensure(size_t(voff[size_t(B)]) * 4));
+	PA_CUDA(s->d_wsb_vals_t.ensure(size_t(voff[size_t(B)]) * 4));
+	// zeroed per call: the optimum keys, the tile counters, the work counter
+	const size_t zb = size_t(B) * 8 + size_t(poff[size_t(B)]) * 4 + 4;
+	PA_CUDA(s->d_progress.ensure(zb));
+	PA_CUDA(cudaMemsetAsync(s->d_progress.p, 0, zb, st));
+	WsbTileParams w{};
+	w.npairs = int32_t(B);
+	w.len_s = s->m.ls;
+	w.len_t = s->m.lt;
+	w.local = s->loc;
+	w.sub_kind = in.form == F_DENSE ? SUB_DENSE : (in.form == F_BINARY ? SUB_BINARY : SUB_TABLE);
+	if (in.form != F_DENSE) {
+		w.a = in.location == PA_DEVICE ? in.a : s->d_a.as<uint32_t>();
+		w.b = in.location == PA_DEVICE ? in.b : s->d_b.as<uint32_t>();
+		w.a_stride = in.n_s;
+		w.b_stride = in.n_t;
+	} else {
+		w.dense = in.location == PA_DEVICE ? in.sim : s->d_dense.as<float>();
+		w.dense_si = in.n_t * in.batch;
+		w.dense_sj = in.batch;
+	}
+	w.table = reinterpret_cast<const float *>(d + o_tab);
+	w.table_rows = int32_t(in.table_rows);
+	w.table_cols = int32_t(in.table_cols);
+	w.eq = in.eq;
+	w.ne = in.ne;
+	w.sign = s->sign;
+	w.left_D = reinterpret_cast<const float *>(d + o_left);
+	w.top_D = reinterpret_cast<const float *>(d + o_top);
+	w.ngap_s = reinterpret_cast<const float *>(d + o_gs);
+	w.ngap_t = reinterpret_cast<const float *>(d + o_gt);
+	w.vals = s->d_wsb_vals.as<float>();
+	w.vals_t = s->d_wsb_vals_t.as<float>();
+	w.vals_off = reinterpret_cast<const int64_t *>(d + o_voff);
+	w.tiles = reinterpret_cast<const int2 *>(d + o_tiles);
+	w.ntiles = int32_t(ntiles);
+	w.best = s->d_progress.as<unsigned long long>();
+	w.progress = reinterpret_cast<int32_t *>(s->d_progress.as<unsigned char>() + size_t(B) * 8);
+	w.work_counter = w.progress + poff[size_t(B)];
+	w.prog_off = reinterpret_cast<const int32_t *>(d + o_poff);
+	w.score = s->d_score.as<float>();
+	w.seed = s->d_seed.as<int32_t>();
+	w.has_seed = s->d_has.as<int32_t>();
+	w.status = s->d_status.as<int32_t>();
+	w.map_off = s->m.map_off;
+	w.maps = maps;
+	PA_CUDA(launch_wsb_tiles(w, s->sm_count, st));
+	*launches += 1 + int(ntiles > 0);
+	return PA_OK;
+}
+
+// Whether the tiled sweep takes a general-gap solve that needs no cell matrices: always, but
+// for pairs of 2^32 cells (its local seeds pack a position in 32 bits) or 2^20 rows (the tile
+// list packs tile coordinates in 16 bits), and when one of the switches that pick a split of
+// wsb_kernel is set.  It beats that kernel at every size measured (call times, this
+// sweep against wsb_kernel's: 1 pair of 20 x 20 85 / 120 us, 512 of 50 x 50 172 / 552 us, 2048 of
+// 30 x 30 204 / 618 us, 64 of 20 x 900 0.45 / 3.5 ms, 64 of 300 x 300 0.56 / 4.2 ms, 2 of
+// 600 x 600 0.88 / 11.3 ms, 16 of 1000 x 1000 3.1 / 39 ms).
+bool wsb_tiles_ok(const std::vector<int32_t> &ls, const std::vector<int32_t> &lt) {
+	for (const char *e : {"PA_WSB_THREADS", "PA_WSB_CLUSTER", "PA_WSB_SMEM", "PA_WSB_WARP_CELLS"})
+		if (std::getenv(e)) return false;
+	for (size_t k = 0; k < ls.size(); k++)
+		if (int64_t(ls[k]) * lt[k] >= (int64_t(1) << 32) || std::max(ls[k], lt[k]) >= (1 << 20)) return false;
+	return true;
+}
+
 pa_status download_wsb(pa_solver *s, ResultData &res) {
 	cudaStream_t st = s->stream;
 	const int64_t B = res.batch;
@@ -1914,7 +2041,11 @@ pa_status solve_impl(pa_solver *s, const Input &in, int method, float *scores_ou
 					wmaps = s->d_maps.as<int32_t>();
 				}
 			}
-			if (pa_status e = run_wsb(s, in, ls, lt, &launches, res, wmaps)) return e;
+			if (!wsb_host && wsb_tiles_ok(ls, lt)) {
+				if (pa_status e = run_wsb_tiles(s, in, ls, lt, &launches, wmaps)) return e;
+			} else if (pa_status e = run_wsb(s, in, ls, lt, &launches, res, wmaps)) {
+				return e;
+			}
 		} else {
 			if (tb == TB_ALL && s->loc == LOC_LOCAL) {
 				// the optimum is needed to mark the seeds (solver.h:2066-2091): a score pass first

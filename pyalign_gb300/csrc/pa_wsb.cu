@@ -1,4 +1,6 @@
-// General gap cost solve (GeneralGapCostSolver, solver.h:3056-3184): O(n m (n + m)).
+// General gap cost solve (GeneralGapCostSolver, solver.h:3056-3184): O(n m (n + m)), with every
+// cell's value, traceback code and similarity left in memory for the iterators, solutions and
+// all-optimal searches (scores and single alignments need none of them: pa_wsb_tile.cu).
 //
 // A CTA, or a cluster of 2 or 4 CTAs when there are fewer pairs than SMs, per pair sweeps
 // anti-diagonals.  Cell (u, v) takes the best of its head candidates -- (local zero), the
