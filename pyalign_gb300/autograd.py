@@ -440,8 +440,12 @@ class EmbeddingAlignmentScore(torch.autograd.Function):
         Esb, inv_s = normalized_bf16(Es, normalize, ln[:, 0], tiled=True)
         Etb, inv_t = normalized_bf16(Et, normalize, ln[:, 1], tiled=True)
         # S^T = en_t en_s^T on the tensor cores, only the cells inside the lengths; its
-        # transposed view is S with stride 1 along s
-        S = similarity_bf16(Esb, Etb, lengths)
+        # transposed view is S with stride 1 along s; its columns are padded to whole 16-byte
+        # words (rows no pair reaches) for the DP's loads
+        B, n_s, n_t = Es.shape[0], Es.shape[1], Et.shape[1]
+        St = torch.empty((B, n_t, (n_s + 3) // 4 * 4), dtype=torch.float32, device=Es.device)
+        similarity_bf16(Esb, Etb, lengths, out=St[:, :, :n_s])
+        S = St.transpose(1, 2)
         gap = (float(gap_open), None) if linear else (float(gap_open), float(gap_extend))
         scores, paths, plen, poff, _ = _forward_paths(S, lengths, gap, locality, direction, False)
         ctx.save_for_backward(Es, Et, Esb, Etb, inv_s, inv_t, paths, plen, poff)

@@ -118,6 +118,10 @@ struct DpParams {
 	void *scratch;
 	int64_t scratch_stride;  // elements per slot
 	int32_t *work_counter;
+	// group mode: the first tasks spread over the SMs (next_task); null: one counter for all
+	int32_t *spread;         // SPREAD_CLASSES task counters, then SPREAD_SMS warp counters, zeroed
+	int32_t spread_classes;  // classes of spread_size tasks each, the costliest first
+	int32_t spread_size;     // SMs
 	int32_t *status;
 	// stripe-chained mode (units != 0): a ticket is one stripe of one pair; tickets are
 	// numbered stripe-major, level_start[q] is the first ticket of stripe q (nlevels + 1
@@ -180,6 +184,54 @@ static __device__ __noinline__ int32_t wait_progress(const int32_t *prog, int32_
 	}
 	atomicOr(status, ST_TIMEOUT);
 	return INT32_MAX;
+}
+
+// The next warp task of a group-mode launch (x; -1: none left), warp-uniform; y carries the
+// warp's cursor from call to call (-2 at first).
+//
+// Tasks are ordered costliest first and one counter hands them out.  That balances a launch of
+// many tasks per warp, but most launches have about one: all of them are taken within
+// microseconds of the start, in block order, so the SMs that start first hold the longest pairs
+// and run on when the others are done (8,192 pairs of 32..512 on G = 16: one SM's ALU pipe 97%
+// busy, the average 41%).  So the first tasks go out by classes of one task per SM, as equal in
+// cost as the order makes them: the r-th warp to start on an SM takes from class r, and every SM
+// holds one task of each class.  A warp whose class is used up takes from the next class that
+// has a task left (an SM shared with another kernel may start fewer warps than there are
+// classes), then from the counter, which holds the tasks past the classes.  Where those are
+// all in classes the surplus warps leave at once, so no SM takes more than its share.
+constexpr int SPREAD_CLASSES = 32;
+constexpr int SPREAD_SMS = 256;
+static __device__ __noinline__ int2 next_task(int32_t *counter, int32_t *spread, int nclass, int size, int ntasks,
+                                              int cursor) {
+	const int lane = threadIdx.x & 31;
+	int first = 0;
+	if (spread) {
+		first = nclass * size;
+		if (cursor == -2) {
+			uint32_t smid;
+			asm volatile("mov.u32 %0, %%smid;" : "=r"(smid));
+			int r = 0;
+			if (lane == 0) r = atomicAdd(spread + SPREAD_CLASSES + int(smid % SPREAD_SMS), 1);
+			r = __shfl_sync(0xffffffffu, r, 0);
+			if (r >= nclass && first >= ntasks) return make_int2(-1, -1);
+			cursor = r < nclass ? r : -1;
+		}
+		while (cursor >= 0) {
+			int k = 0;
+			if (lane == 0) k = atomicAdd(spread + cursor, 1);
+			k = __shfl_sync(0xffffffffu, k, 0);
+			if (k < min(size, ntasks - cursor * size)) return make_int2(cursor * size + k, cursor);
+			const int taken = lane < nclass ? *reinterpret_cast<volatile int32_t *>(spread + lane) : 0;
+			const uint32_t left =
+			    __ballot_sync(0xffffffffu, lane < nclass && taken < min(size, ntasks - lane * size));
+			const uint32_t later = left & ~((2u << cursor) - 1u);
+			cursor = left ? __ffs(int(later ? later : left)) - 1 : -1;
+		}
+	}
+	int t = 0;
+	if (lane == 0) t = atomicAdd(counter, 1);
+	t = __shfl_sync(0xffffffffu, t, 0) + first;
+	return make_int2(t < ntasks ? t : -1, -1);
 }
 
 template <typename V>
@@ -426,13 +478,21 @@ __global__ void __launch_bounds__(BLOCK, 4) dp_kernel(DpParams<V> p) {
 	const int rpp = G * R;  // rows per pass
 	const int sub_kind = p.sub_kind;
 	constexpr bool units = CHAIN;  // stripe-chained mode (G == 32)
-	const int ntickets = units ? p.ntickets : p.npairs;
+	int cursor = -2;
 
 	for (;;) {
 		int base = 0;
-		if (lane == 0) base = atomicAdd(p.work_counter, gpw);
-		base = __shfl_sync(0xffffffffu, base, 0);
-		if (base >= ntickets) break;
+		if constexpr (units) {
+			if (lane == 0) base = atomicAdd(p.work_counter, 1);
+			base = __shfl_sync(0xffffffffu, base, 0);
+			if (base >= p.ntickets) break;
+		} else {
+			const int2 t = next_task(p.work_counter, p.spread, p.spread_classes, p.spread_size,
+			                         (p.npairs + gpw - 1) / gpw, cursor);
+			if (t.x < 0) break;
+			base = t.x * gpw;
+			cursor = t.y;
+		}
 		// group mode: the pair at rank base + grp, all of its stripes.  Stripe-chained mode:
 		// stripe q_lo of the pair at rank w, waiting on ticket prod (stripe q_lo - 1).
 		int w = base + grp, q_lo = 0, prod = -1;
@@ -907,6 +967,12 @@ __global__ void __launch_bounds__(BLOCK, 4) dp_kernel(DpParams<V> p) {
 		                                    l_bj, row_best, row_bj, col_best, col_bi, glob, have_glob);
 	}
 }
+
+// A dense similarity with unit stride along s or t copied to the layout the float kernels read
+// 16 bytes at a time: S(k, i, j) = dst[dst_off[k] + i + j * pitch] for the cells inside the
+// lengths.
+__global__ void dense_copy_kernel(const float *src, const int64_t *src_off, int64_t si, int64_t sj, float *dst,
+                                  const int64_t *dst_off, int64_t pitch, const int32_t *len_s, const int32_t *len_t);
 
 // Largest code in a batch of sequences (host validation of the indexed form,
 // factory.h:602-614, done on the device for device-resident inputs).

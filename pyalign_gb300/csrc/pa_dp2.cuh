@@ -91,13 +91,21 @@ __global__ void __launch_bounds__(BLOCK, 4) dp2_kernel(DpParams<int32_t> p) {
 	const V NEG = p.neg_inf;
 	const int rpp = G * R;
 	const int sub_kind = p.sub_kind;
-	const int ntickets = CHAIN ? p.ntickets : p.npairs;
+	int cursor = -2;
 
 	for (;;) {
 		int base = 0;
-		if (lane == 0) base = atomicAdd(p.work_counter, gpw);
-		base = __shfl_sync(0xffffffffu, base, 0);
-		if (base >= ntickets) break;
+		if constexpr (CHAIN) {
+			if (lane == 0) base = atomicAdd(p.work_counter, 1);
+			base = __shfl_sync(0xffffffffu, base, 0);
+			if (base >= p.ntickets) break;
+		} else {
+			const int2 t = next_task(p.work_counter, p.spread, p.spread_classes, p.spread_size,
+			                         (p.npairs + gpw - 1) / gpw, cursor);
+			if (t.x < 0) break;
+			base = t.x * gpw;
+			cursor = t.y;
+		}
 		int w = base + grp, q_lo = 0, prod = -1;
 		if constexpr (CHAIN) {
 			int lo = 0, hi = p.nlevels - 1;

@@ -25,6 +25,7 @@
 #include "../../include/pyalign_gb300.h"
 #include "pa_dp.cuh"
 #include "pa_enum.h"
+#include "pa_dpf2.cuh"
 #include "pa_launch.h"
 #include "pa_wsb.h"
 
@@ -392,6 +393,7 @@ struct pa_solver {
 	struct {
 		int32_t *ls, *lt, *order, *level_start;
 		int64_t *mask_off, *map_off, *path_off, *val_off, *dense_off;
+		int64_t *dense_src;  // a copied similarity's offsets in the caller's tensor
 		int8_t *pair_G;  // per pair group width (length buckets)
 	} m{};
 	std::vector<std::pair<uint64_t, int>> occ_cache;  // (kernel variant, smem) -> blocks per SM
@@ -419,7 +421,9 @@ struct pa_solver {
 		std::vector<int64_t> user_map_off, user_path_off, dense_off;
 		// the plan and what the downloads need from it
 		int G = 0, C = 1, launches = 0, key_shift = 0, ntickets = 0, nlevels = 0;
-		bool units = false, use_int = false, h16 = false, blk = false, seg = false;
+		bool units = false, use_int = false, h16 = false, blk = false, seg = false, uneven = false;
+		int sub2 = -1;
+		int64_t copy_pitch = 0;
 		int bucket_G[PA_BUCKETS] = {};
 		SegInfo segs[PA_MAX_CHUNKS];
 		int32_t h_neg = 0;
@@ -510,6 +514,9 @@ struct Plan {
 	int bucket_G[PA_BUCKETS] = {16, 16, 16, 16};
 	SegInfo segs[PA_MAX_CHUNKS];
 	int32_t h_neg = 0;
+	bool uneven = false;       // the pairs' costs differ: group mode spreads the first tasks (run_dp)
+	int sub2 = -1;             // float: what dpf2_kernel reads (C = 2), or -1
+	int64_t copy_pitch = 0;    // float, dense: > 0, the similarity is copied first, with this pitch
 	int C32 = 1;               // columns per lane step of the int32/float kernels for this launch
 	int nchunks = 1;           // repeated host-buffer solves: pipeline of this many pair ranges
 };
@@ -608,6 +615,41 @@ int plan_words(const Plan &pl) { return pl.blk ? 2 : pl.C; }
 // Launches the two-column kernel can run: int32 tagged scoring without all-optimal masks
 // or Solution values.
 bool cols2_ok(const Plan &plan, bool want_values) { return plan.use_int && plan.tb != TB_ALL && !want_values; }
+
+// Columns per lane step of a launch outside the 16-bit kernel: the two-column kernels where they
+// take it, but float scoring's stripe-chained mode is the one-column kernel's.
+int cols_of(const Plan &plan, bool units) { return units && !plan.use_int ? 1 : plan.C32; }
+
+// The float form of a launch's similarities the two-column float kernel (pa_dpf2.cuh) reads, or
+// -1: scores or one traceback, without Solution values, of a table, of series, or of a dense
+// similarity whose columns can be read 16 bytes at a time (stride 1 along s, aligned, a multiple
+// of 4 rows).
+int dpf2_sub(const Input &in, int tb, bool want_values) {
+	if (tb == TB_ALL || want_values) return -1;
+	if (in.form == F_INDEXED) return SUBF_TABLE;
+	if (tb != TB_ONE) return -1;
+	if (in.form == F_SERIES) return SUBF_SERIES;
+	if (in.form != F_DENSE || in.location != PA_DEVICE || in.dense_si != 1 || (in.dense_sj & 3) || (in.n_s & 3) ||
+	    (reinterpret_cast<uintptr_t>(in.sim) & 15) || !in.dense_off_host)
+		return -1;
+	for (int64_t k = 0; k < in.batch; k++)
+		if (in.dense_off_host[k] & 3) return -1;
+	return SUBF_DENSE;
+}
+
+// Whether a dense similarity that kernel cannot read in place is copied to its layout first
+// (dense_copy_kernel): unit stride along s or t, and a copy of at most 4 GiB.  The copy moves 8
+// bytes a cell at the speed of HBM, and the DP then reads 32-byte rows instead of single floats of
+// eight rows: 1,024
+// pairs of 100..400 with stride 1 along t 0.98 ms in place (dp_kernel), 0.11 + 0.38 ms copied.
+constexpr int64_t DENSE_COPY_BYTES = int64_t(4) << 30;
+bool dense_copy_ok(const Input &in, int tb, bool want_values, const std::vector<int32_t> &lt, int64_t pitch) {
+	if (in.form != F_DENSE || in.location != PA_DEVICE || tb != TB_ONE || want_values || !in.dense_off_host) return false;
+	if (in.dense_si != 1 && in.dense_sj != 1) return false;
+	int64_t cells = 0;
+	for (int32_t t : lt) cells += t * pitch;
+	return cells * 4 <= DENSE_COPY_BYTES;
+}
 
 // Group width G (lanes per pair, R = 8 rows each; G = 1 is a lane per pair) that minimises the cells a launch
 // computes: the real cells plus the padding rows of each pair's last stripe and the G-1
@@ -813,6 +855,11 @@ pa_status run_dp(pa_solver *s, const Input &in, const Plan &plan, int tb, const 
 		p.dense_si = in.dense_si ? in.dense_si : in.n_t * in.batch;
 		p.dense_sj = in.dense_si ? in.dense_sj : in.batch;
 		p.dense_sign = s->sign;
+		if (plan.copy_pitch) {
+			p.dense = s->d_dense.as<float>();
+			p.dense_si = 1;
+			p.dense_sj = plan.copy_pitch;
+		}
 	}
 	// ---- gaps (negative addends, maximize form)
 	const pa_options &o = s->opt;
@@ -920,7 +967,8 @@ pa_status run_dp(pa_solver *s, const Input &in, const Plan &plan, int tb, const 
 	p.best_in = best_in_dev;
 	p.values = want_values ? s->d_vals.as<float>() : nullptr;
 	p.val_off = s->m.val_off;
-	PA_CUDA(counter.ensure(4));
+	constexpr size_t counter_bytes = size_t(1 + SPREAD_CLASSES + SPREAD_SMS) * 4;
+	PA_CUDA(counter.ensure(counter_bytes));
 	p.work_counter = counter.as<int32_t>();
 	p.status = s->d_status.as<int32_t>();
 	if (in.form == F_INDEXED) {
@@ -935,6 +983,7 @@ pa_status run_dp(pa_solver *s, const Input &in, const Plan &plan, int tb, const 
 	                  : 0;
 	if (p.sub_kind == SUB_COLPROF) smem = ((smem + 15) & ~size_t(15)) + size_t(in.table_cols) * BLOCK * 8;
 	if (p.sub_kind == SUB_DENSE) smem = size_t(BLOCK) * DENSE_RING * 32;  // the dense S ring (pa_dp.cuh)
+	const size_t smem0 = smem;
 	int bps = 0;
 	cudaError_t e = cudaSuccess;
 	const int loc = s->loc;
@@ -942,9 +991,11 @@ pa_status run_dp(pa_solver *s, const Input &in, const Plan &plan, int tb, const 
 	                      (uint64_t(tb) << 48) | (uint64_t(want_values) << 44) | uint64_t(smem);
 	const bool ch = plan.units;
 	const int cols = (ISINT && plan.C == 2 && tb != TB_ALL && !want_values) ? 2 : 1;
+	const int sub2 = !ISINT && plan.C == 2 ? plan.sub2 : -1;  // >= 0: dpf2_kernel
+	if (sub2 == SUBF_DENSE) smem = size_t(DPF2_RING) * 4 * BLOCK * 16;
 	const bool blk = h16 && plan.blk;
-	const uint64_t ckey = okey | (uint64_t(ch) << 40) | (uint64_t(cols == 2) << 41) | (uint64_t(h16) << 42) |
-	                      (uint64_t(blk) << 43);
+	const uint64_t ckey = (okey + smem - smem0) | (uint64_t(sub2 + 1) << 36) | (uint64_t(ch) << 40) |
+	                      (uint64_t(cols == 2) << 41) | (uint64_t(h16) << 42) | (uint64_t(blk) << 43);
 	for (const auto &kv : s->occ_cache)
 		if (kv.first == ckey) bps = kv.second;
 	if (bps == 0) {
@@ -952,6 +1003,9 @@ pa_status run_dp(pa_solver *s, const Input &in, const Plan &plan, int tb, const 
 		                              : occupancy_dp16b_affine(loc, tb, smem, &bps);
 		else if (h16) e = gk == GAP_LINEAR ? occupancy_dp16_linear(loc, tb, cols, smem, &bps)
 		                                   : occupancy_dp16_affine(loc, tb, cols, smem, &bps);
+		else if (sub2 >= 0) e = gk == GAP_LINEAR   ? occupancy_dpf2_linear(loc, tb, sub2, smem, &bps)
+		                        : gk == GAP_AFFINE ? occupancy_dpf2_affine(loc, tb, sub2, smem, &bps)
+		                                           : occupancy_dpf2_dtw(loc, tb, sub2, smem, &bps);
 		else e = dp_occupancy<V>(gk, ch, loc, tb, want_values, smem, &bps, cols);
 	}
 	PA_CUDA(e);
@@ -966,12 +1020,28 @@ pa_status run_dp(pa_solver *s, const Input &in, const Plan &plan, int tb, const 
 	grid = std::min<int64_t>(grid, (groups_needed + WARPS - 1) / WARPS);
 	// PA_GRID=exact: one block per WARPS work units, each warp takes one unit and exits -- the
 	// non-persistent launch of a plain per-bucket solve, kept for that comparison
-	if (const char *ge = std::getenv("PA_GRID"))
-		if (std::strcmp(ge, "exact") == 0) grid = (groups_needed + WARPS - 1) / WARPS;
+	bool exact = false;
+	if (const char *ge = std::getenv("PA_GRID")) exact = std::strcmp(ge, "exact") == 0;
+	if (exact) grid = (groups_needed + WARPS - 1) / WARPS;
 	grid = std::max<int64_t>(grid, 1);
+	// group mode: the first tasks one per SM and class (next_task), for which every SM needs its
+	// warps, so the launch fills the GPU.  Only where the tasks' costs differ and there are few of
+	// them per resident warp: the counter balances more (65,536 DNA pairs, 7 tasks a warp, run the
+	// same either way), and on equal tasks the classes only cost their atomics (4,096 pairs of
+	// 64 x 64: 28 against 21 us).  4,096 protein pairs of
+	// 50..600 (int32) 0.80 -> 0.73 ms, 8,192 dense pairs of 32..512 (float) 1.72 -> 1.53 ms, 4,096
+	// series pairs of 128..1024 1.75 -> 1.63 ms.
+	if (!plan.units && !h16 && !exact && plan.uneven && groups_needed > WARPS &&
+	    groups_needed <= 3 * int64_t(s->sm_count) * bps * WARPS) {
+		grid = int64_t(s->sm_count) * bps;
+		p.spread = p.work_counter + 1;
+		p.spread_size = s->sm_count;
+		p.spread_classes = int32_t(std::min<int64_t>(std::min(SPREAD_CLASSES, bps * WARPS),
+		                                             (groups_needed + s->sm_count - 1) / s->sm_count));
+	}
 	// scratch rows: per group slot, or per pair in the stripe-chained mode
 	const int64_t slots = plan.units ? std::max<int64_t>(npairs, 1) : grid * WARPS * gpw;
-	p.scratch_stride = 2 * std::max<int64_t>(plan.max_lt, 1);
+	p.scratch_stride = 2 * ((std::max<int64_t>(plan.max_lt, 1) + 1) & ~int64_t(1));  // two rows of column pairs
 	PA_CUDA(scratch.ensure(size_t(slots * p.scratch_stride) * 2 * sizeof(V)));
 	p.scratch = scratch.p;
 	if (plan.units) {
@@ -986,13 +1056,17 @@ pa_status run_dp(pa_solver *s, const Input &in, const Plan &plan, int tb, const 
 		PA_CUDA(cudaMemsetAsync(s->d_progress.p, 0, size_t(plan.ntickets) * 4, st));
 	}
 
-	PA_CUDA(cudaMemsetAsync(counter.p, 0, sizeof(int32_t), st));
+	PA_CUDA(cudaMemsetAsync(counter.p, 0, counter_bytes, st));
 	if constexpr (std::is_same<V, int32_t>::value) {
 		if (blk) e = gk == GAP_LINEAR ? launch_dp16b_linear(loc, tb, p, int(grid), smem, st)
 		                              : launch_dp16b_affine(loc, tb, p, int(grid), smem, st);
 		else if (h16) e = gk == GAP_LINEAR ? launch_dp16_linear(loc, tb, cols, p, int(grid), smem, st)
 		                                   : launch_dp16_affine(loc, tb, cols, p, int(grid), smem, st);
 		else e = dp_launch<V>(gk, ch, loc, tb, want_values, p, int(grid), smem, st, cols);
+	} else if (sub2 >= 0) {
+		e = gk == GAP_LINEAR   ? launch_dpf2_linear(loc, tb, sub2, p, int(grid), smem, st)
+		    : gk == GAP_AFFINE ? launch_dpf2_affine(loc, tb, sub2, p, int(grid), smem, st)
+		                       : launch_dpf2_dtw(loc, tb, sub2, p, int(grid), smem, st);
 	} else {
 		e = dp_launch<V>(gk, ch, loc, tb, want_values, p, int(grid), smem, st, cols);
 	}
@@ -1411,7 +1485,7 @@ pa_status tune_plan(pa_solver *s, const std::vector<int32_t> &ls, const std::vec
 				plan.units = t.units;
 				plan.h16 = plan.h16 && t.h16;  // the 16-bit kernel still needs this launch's bounds
 				plan.blk = plan.h16 && t.blk;
-				plan.C = plan.h16 ? t.C : plan.C32;
+				plan.C = plan.h16 ? t.C : cols_of(plan, plan.units);
 				plan.seg = plan.h16 && !plan.blk && t.seg;
 				for (int k = 0; k < PA_BUCKETS; k++) plan.bucket_G[k] = t.bucket_G[k];
 				return PA_OK;
@@ -1442,7 +1516,7 @@ pa_status tune_plan(pa_solver *s, const std::vector<int32_t> &ls, const std::vec
 	if (plan.h16 && C0 == 2)
 		for (int G : {32, 16, 8})
 			if (int64_t(G) * 4 <= 2 * plan.max_ls) cand.push_back({G, false, true, 4, true});
-	if (plan.max_ls > 2 * 32 * R) cand.push_back({32, true, false, C0, false});
+	if (plan.max_ls > 2 * 32 * R) cand.push_back({32, true, false, cols_of(plan, true), false});
 	if (cand.size() < 2) return PA_OK;
 	cudaStream_t st = s->stream;
 	float best = INFINITY;
@@ -1751,7 +1825,17 @@ pa_status solve_impl(pa_solver *s, const Input &in, int method, float *scores_ou
 	plan.max_ls = max_ls;
 	plan.max_lt = max_lt;
 	plan.tb = tb;
-	if (!hit) plan.G = choose_G(ls, lt, s->sm_count);
+	if (!hit) {
+		plan.G = choose_G(ls, lt, s->sm_count);
+		int64_t most = 0, sum = 0, n = 0;
+		for (int64_t k = 0; k < B; k++) {
+			const int64_t c = int64_t(ls[size_t(k)]) * lt[size_t(k)];
+			most = std::max(most, c);
+			sum += c;
+			n += c > 0;
+		}
+		plan.uneven = 2 * most * n > 3 * sum;  // the largest pair over 1.5 times the mean
+	}
 	if (!hit && s->gap != GAP_GENERAL) {
 		plan.units = choose_units(ls, lt, s->sm_count, plan.G);
 		if (plan.units) plan.G = 32;
@@ -1765,11 +1849,25 @@ pa_status solve_impl(pa_solver *s, const Input &in, int method, float *scores_ou
 			if ((bound * 4.0 + 4.0) * double(int64_t(1) << shift) >= 2147483647.0) use_int = false;
 		}
 		plan.use_int = use_int;
-		plan.C = cols2_ok(plan, want_values) ? 2 : 1;
+		if (!use_int) plan.sub2 = dpf2_sub(in, tb, want_values);
+		if (!use_int && plan.sub2 < 0) {
+			const int64_t pitch = (max_ls + 3) & ~int64_t(3);
+			int64_t cells = 0;
+			for (int32_t t : lt) cells += t * pitch;
+			if (cells > 0 && dense_copy_ok(in, tb, want_values, lt, pitch)) {
+				if (s->d_dense.ensure(size_t(cells) * 4) == cudaSuccess) {
+					plan.copy_pitch = pitch;
+					plan.sub2 = SUBF_DENSE;
+				} else {
+					cudaGetLastError();  // no room for the copy: the similarity is read in place
+				}
+			}
+		}
+		plan.C32 = cols2_ok(plan, want_values) || plan.sub2 >= 0 ? 2 : 1;
 		if (const char *e = std::getenv("PA_DP_COLS"))  // experiments and tests
-			if (std::atoi(e) == 1) plan.C = 1;
+			if (std::atoi(e) == 1) plan.C32 = 1;
+		plan.C = cols_of(plan, plan.units);
 		int32_t hneg = 0;
-		plan.C32 = plan.C;
 		plan.h16 = !plan.units && h16_plan(s, in, host_table.data(), ls, lt, tb, want_values, use_int, &hneg);
 		plan.h_neg = hneg;
 		if (plan.h16) plan.C = plan.C32;  // two columns per step unless PA_DP_COLS=1
@@ -1783,7 +1881,7 @@ pa_status solve_impl(pa_solver *s, const Input &in, int method, float *scores_ou
 	}
 	std::vector<int32_t> order, level_start;
 	std::vector<int8_t> pair_g;  // group width per pair (length buckets)
-	std::vector<int64_t> mask_off, map_off, path_off, val_off, dense_off;
+	std::vector<int64_t> mask_off, map_off, path_off, val_off, dense_off, copy_off;
 	struct Lend {  // a repeat's offsets lent to this call, returned however the call ends
 		pa_solver::Repeat *r = nullptr;
 		std::vector<int64_t> *mo, *mp, *po, *vo;
@@ -1897,6 +1995,8 @@ pa_status solve_impl(pa_solver *s, const Input &in, int method, float *scores_ou
 		path_off.assign(size_t(B) + 1, 0);
 		val_off.assign(size_t(B) + 1, 0);
 		dense_off.assign(size_t(B), 0);
+		copy_off.assign(plan.copy_pitch ? size_t(B) : 0, 0);
+		int64_t copied = 0;
 		for (int64_t k = 0; k < B; k++) {
 			const int64_t a = ls[size_t(k)], b = lt[size_t(k)];
 			const int64_t gk = pair_g[size_t(k)], rpp = gk * plan_rows(plan);
@@ -1907,11 +2007,15 @@ pa_status solve_impl(pa_solver *s, const Input &in, int method, float *scores_ou
 			path_off[size_t(k) + 1] = path_off[size_t(k)] + 2 * (a + b + 2);
 			val_off[size_t(k) + 1] = val_off[size_t(k)] + int64_t(res.layers) * (a + 1) * (b + 1);
 			dense_off[size_t(k)] = in.dense_off_host ? in.dense_off_host[k] : k;
+			if (plan.copy_pitch) {
+				copy_off[size_t(k)] = copied;
+				copied += b * plan.copy_pitch;
+			}
 		}
 		// pair metadata: packed into one pinned staging buffer, one host-to-device copy
 		{
 			const size_t n32 = size_t(B), n64 = size_t(B) + 1;
-			const size_t bytes = ((3 * n32 * 4 + level_start.size() * 4 + 7) & ~size_t(7)) + 5 * n64 * 8 + 16 + n32 + 8;
+			const size_t bytes = ((3 * n32 * 4 + level_start.size() * 4 + 7) & ~size_t(7)) + (5 * n64 + copy_off.size()) * 8 + 16 + n32 + 8;
 			if (s->meta_pending) {
 				PA_CUDA(cudaEventSynchronize(s->meta_ev));  // the previous call's copy has read it
 				s->meta_pending = false;
@@ -1943,6 +2047,8 @@ pa_status solve_impl(pa_solver *s, const Input &in, int method, float *scores_ou
 			s->m.val_off = reinterpret_cast<int64_t *>(put(val_off.data(), n64 * 8, 8));
 			s->m.dense_off = reinterpret_cast<int64_t *>(put(dense_off.data(), n32 * 8, 8));
 			o += 8;
+			s->m.dense_src = s->m.dense_off;
+			if (plan.copy_pitch) s->m.dense_off = reinterpret_cast<int64_t *>(put(copy_off.data(), n32 * 8, 8));
 			s->m.pair_G = reinterpret_cast<int8_t *>(put(pair_g.data(), n32, 1));
 			PA_CUDA(pa_copy(s, d, h, o, cudaMemcpyHostToDevice, st));
 			PA_CUDA(cudaEventRecord(s->meta_ev, st));
@@ -1951,7 +2057,6 @@ pa_status solve_impl(pa_solver *s, const Input &in, int method, float *scores_ou
 		PA_CUDA(s->d_score.ensure(size_t(B) * 4));
 		PA_CUDA(s->d_seed.ensure(size_t(B) * 8));
 		PA_CUDA(s->d_has.ensure(size_t(B) * 4));
-		PA_CUDA(s->d_counter.ensure(4));
 		PA_CUDA(s->d_status.ensure(4));
 		PA_CUDA(cudaMemsetAsync(s->d_status.p, 0, 4, st));
 		const size_t mask_elem = tb == TB_ALL ? 16 : 4;
@@ -1959,7 +2064,21 @@ pa_status solve_impl(pa_solver *s, const Input &in, int method, float *scores_ou
 		if (want_values) PA_CUDA(s->d_vals.ensure(size_t(val_off[size_t(B)]) * 4));
 		return PA_OK;
 	};
+	// a dense similarity into the layout the float kernels read (the staged offsets are in place)
+	auto dense_copy = [&](cudaStream_t sw) -> cudaError_t {
+		if (!plan.copy_pitch) return cudaSuccess;
+		dense_copy_kernel<<<dim3(unsigned(B), unsigned(std::min<int64_t>(8, (max_lt + 31) / 32))), 256, 0, sw>>>(in.sim, s->m.dense_src, in.dense_si, in.dense_sj,
+		                                                     s->d_dense.as<float>(), s->m.dense_off, plan.copy_pitch,
+		                                                     s->m.ls, s->m.lt);
+		launches++;
+		return cudaGetLastError();
+	};
+	bool tuning_copy = false;  // the tuner's runs need the copy once
 	auto dp = [&](const Plan &pl, int tbk, bool vals, const float *best_in) -> pa_status {
+		if (tuning_copy) {
+			PA_CUDA(dense_copy(s->stream));
+			tuning_copy = false;
+		}
 		if (pl.seg && pl.h16 && !pl.blk && pl.nchunks > 1) {
 			// length buckets of a chunk-major order: one launch per chunk, each over its own
 			// segments (a whole-bag launch has none: segments do not cross chunks)
@@ -2053,6 +2172,7 @@ pa_status solve_impl(pa_solver *s, const Input &in, int method, float *scores_ou
 				PA_CUDA(s->d_best.ensure(size_t(B) * 4));
 				PA_CUDA(pa_copy(s, s->d_best.p, s->d_score.p, size_t(B) * 4, cudaMemcpyDeviceToDevice, sw));
 			}
+			PA_CUDA(dense_copy(sw));
 			if (pa_status e2 = dp(plan, tb, want_values, s->d_best.as<float>())) return e2;
 		}
 		if (timed) PA_CUDA(record(s->ev[2], sw));
@@ -2197,6 +2317,9 @@ pa_status solve_impl(pa_solver *s, const Input &in, int method, float *scores_ou
 		plan.h16 = r.h16;
 		plan.blk = r.blk;
 		plan.seg = r.seg;
+		plan.uneven = r.uneven;
+		plan.sub2 = r.sub2;
+		plan.copy_pitch = r.copy_pitch;
 		for (int k = 0; k < PA_BUCKETS; k++) plan.bucket_G[k] = r.bucket_G[k];
 		for (int c = 0; c < PA_MAX_CHUNKS; c++) plan.segs[c] = r.segs[c];
 		plan.h_neg = r.h_neg;
@@ -2249,7 +2372,9 @@ pa_status solve_impl(pa_solver *s, const Input &in, int method, float *scores_ou
 		}
 	} else {
 		if (s->gap != GAP_GENERAL && tb != TB_ALL && !want_values) {
+			tuning_copy = true;
 			if (pa_status e = tune_plan(s, ls, lt, in, plan, stage, dp)) return e;
+			tuning_copy = false;
 		}
 		// host buffers and many pairs: the repeats of this solve run as a pipeline of chunks
 		// (3 chunks from 32K pairs, 2 from 8K; PA_CHUNKS overrides, up to 12); host maps use
@@ -2317,6 +2442,9 @@ pa_status solve_impl(pa_solver *s, const Input &in, int method, float *scores_ou
 		r.h16 = plan.h16;
 		r.blk = plan.blk;
 		r.seg = plan.seg;
+		r.uneven = plan.uneven;
+		r.sub2 = plan.sub2;
+		r.copy_pitch = plan.copy_pitch;
 		for (int k = 0; k < PA_BUCKETS; k++) r.bucket_G[k] = plan.bucket_G[k];
 		for (int c = 0; c < PA_MAX_CHUNKS; c++) r.segs[c] = plan.segs[c];
 		r.h_neg = plan.h_neg;

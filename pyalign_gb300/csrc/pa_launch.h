@@ -31,6 +31,15 @@ PA_DECL2(affine)
 PA_DECL2(dtw)
 #undef PA_DECL2
 
+#define PA_DECLF2(GAP)                                                                                \
+	cudaError_t launch_dpf2_##GAP(int loc, int tb, int sub, const DpParams<float> &p, int grid, size_t smem, \
+	                              cudaStream_t st);                                               \
+	cudaError_t occupancy_dpf2_##GAP(int loc, int tb, int sub, size_t smem, int *blocks_per_sm);
+PA_DECLF2(linear)
+PA_DECLF2(affine)
+PA_DECLF2(dtw)
+#undef PA_DECLF2
+
 #define PA_DECL16(GAP)                                                                                  \
 	cudaError_t launch_dp16_##GAP(int loc, int tb, int cols, const DpParams<int32_t> &p, int grid, size_t smem, \
 	                              cudaStream_t st);                                                 \

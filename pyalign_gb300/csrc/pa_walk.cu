@@ -164,6 +164,54 @@ __global__ void __launch_bounds__(WALK_WARPS * 32) walk_kernel(WalkParams p) {
 	if (p.path_len && lane == 0) p.path_len[pair] = np;
 }
 
+// See pa_dp.cuh.  A block takes every gridDim.y-th strip of 32 columns of one pair, 64 x 32 cells
+// at a time through shared memory, so that both the reads (along the source's unit stride) and the
+// writes (along s) are whole 128-byte lines.  HBM-bound, 8 bytes moved per cell, with eight loads
+// of a thread in flight: 1,024 pairs of 100..400 (64 M
+// cells) in 109 us (137 us with 32 x 32 tiles and four loads).
+__global__ void __launch_bounds__(256) dense_copy_kernel(const float *src, const int64_t *src_off, int64_t si,
+                                                         int64_t sj, float *dst, const int64_t *dst_off, int64_t pitch,
+                                                         const int32_t *len_s, const int32_t *len_t) {
+	constexpr int TI = 64;
+	__shared__ float tile[TI][33];
+	const int pair = blockIdx.x;
+	const int ls = len_s[pair], lt = len_t[pair];
+	const float *S = src + src_off[pair];
+	float *D = dst + dst_off[pair];
+	const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
+	for (int j0 = 32 * blockIdx.y; j0 < lt; j0 += 32 * gridDim.y)
+		for (int i0 = 0; i0 < ls; i0 += TI) {
+			float v[8];
+			if (si == 1) {  // only the pitch or the alignment differs
+#pragma unroll
+				for (int r = 0; r < 8; r++) {
+					const int i = i0 + x + 32 * (r & 1), j = j0 + y + 8 * (r >> 1);
+					v[r] = i < ls && j < lt ? S[i + int64_t(j) * sj] : 0.0f;
+				}
+#pragma unroll
+				for (int r = 0; r < 8; r++) {
+					const int i = i0 + x + 32 * (r & 1), j = j0 + y + 8 * (r >> 1);
+					if (i < ls && j < lt) D[i + int64_t(j) * pitch] = v[r];
+				}
+				continue;
+			}
+#pragma unroll
+			for (int r = 0; r < 8; r++) {
+				const int i = i0 + y + 8 * r, j = j0 + x;
+				v[r] = i < ls && j < lt ? S[int64_t(i) * si + j] : 0.0f;
+			}
+			__syncthreads();  // the previous tile has been written out
+#pragma unroll
+			for (int r = 0; r < 8; r++) tile[y + 8 * r][x] = v[r];
+			__syncthreads();
+#pragma unroll
+			for (int r = 0; r < 8; r++) {
+				const int i = i0 + x + 32 * (r & 1), j = j0 + y + 8 * (r >> 1);
+				if (i < ls && j < lt) D[i + int64_t(j) * pitch] = tile[i - i0][j - j0];
+			}
+		}
+}
+
 // Largest code of an array, folded into *out with atomicMax.  Streams 16-byte words with
 // four loads in flight per thread (the reads are the whole cost: 4 bytes per code), after a
 // scalar head up to the first 16-byte boundary and before a scalar tail.
