@@ -141,6 +141,10 @@ struct DpParams {
 	// holds value * 16 + 8
 	uint32_t h_ext_s, h_ext_t, h_neg;
 	uint32_t k_open_s, k_open_t, k_up, k_left;
+	// scores alone (dps16_kernel, pa_dps16.cuh): the same addends as plain packed values, what a
+	// stored value exceeds the real one by, and a packed real value below all others
+	int32_t h_off;
+	uint32_t h_low;
 	const uint32_t *left16;
 	const uint32_t *top16;
 	// indexed form: the largest code of a and of b (written by codes_max_kernel earlier in

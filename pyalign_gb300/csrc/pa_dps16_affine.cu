@@ -1,0 +1,4 @@
+// Instantiations of dps16_kernel<GAP_AFFINE, *, *, *> (packed 16-bit twin pairs, scores alone).
+#define PA_GAPK GAP_AFFINE
+#define PA_FN(x) x##_dps16_affine
+#include "pa_dps16_inst.inc"

@@ -26,6 +26,7 @@
 #include "pa_dp.cuh"
 #include "pa_enum.h"
 #include "pa_dpf2.cuh"
+#include "pa_dps16.cuh"
 #include "pa_launch.h"
 #include "pa_wsb.h"
 
@@ -424,6 +425,8 @@ struct pa_solver {
 		bool units = false, use_int = false, h16 = false, blk = false, seg = false, uneven = false;
 		int sub2 = -1;
 		int64_t copy_pitch = 0;
+		bool s16 = false;
+		int32_t s_neg = 0, h_off = 0, h_low = 0;
 		int bucket_G[PA_BUCKETS] = {};
 		SegInfo segs[PA_MAX_CHUNKS];
 		int32_t h_neg = 0;
@@ -515,6 +518,8 @@ struct Plan {
 	SegInfo segs[PA_MAX_CHUNKS];
 	int32_t h_neg = 0;
 	bool uneven = false;       // the pairs' costs differ: group mode spreads the first tasks (run_dp)
+	bool s16 = false;          // scores alone in packed 16-bit twins (dps16_kernel), before h16
+	int32_t s_neg = 0, h_off = 0, h_low = 0;
 	int sub2 = -1;             // float: what dpf2_kernel reads (C = 2), or -1
 	int64_t copy_pitch = 0;    // float, dense: > 0, the similarity is copied first, with this pitch
 	int C32 = 1;               // columns per lane step of the int32/float kernels for this launch
@@ -586,6 +591,60 @@ bool h16_plan(const pa_solver *s, const Input &in, const float *host_table, cons
 	const double neg = 16.0 * std::ceil(std::max(w1s, w1t) + std::max(us, ut) + 10.0) - 32768.0;
 	if (hi * 16.0 + 15.0 > 32767.0 || lo * 16.0 <= neg + 16.0) return false;
 	*neg_out = int32_t(neg);
+	return true;
+}
+
+// Scores alone in plain packed 16-bit values (pa_dps16.cuh): a launch whose every value fits an
+// int16 after an offset.  Bounds in value units over the launch's whole rectangle, padding rows
+// (at most 256 past the longest |s|) included: no D above the largest similarity times the
+// shorter side, plus the largest border; none below the cheapest gap from a border (semiglobal:
+// both borders are 0, so the cheaper of straight down and straight across; global: the lowest
+// border, then down and across; local: 0).  P and Q lie at most one opening and one extension
+// lower, a padding row's diagonal 128.  It also needs an indexed form of at most 32 letters of t,
+// int8 similarities, and gap costs of at least 0 (rows past |s| must not exceed the optimum).
+// PA_DP16=0 turns it off, as do the switches that pick a variant of dp16_kernel.
+bool s16_plan(const pa_solver *s, const Input &in, const float *host_table, int64_t mls, int64_t mlt, Plan &plan) {
+	for (const char *e : {"PA_DP_BLOCK", "PA_BUCKET_WIDTHS"})
+		if (std::getenv(e)) return false;
+	if (const char *e = std::getenv("PA_DP16"))
+		if (std::strcmp(e, "0") == 0) return false;
+	if (const char *e = std::getenv("PA_DP_COLS"))
+		if (std::atoi(e) == 1) return false;
+	if (!plan.use_int || plan.tb != TB_NONE || in.form != F_INDEXED) return false;
+	if (in.table_cols > MAX_COLPROF || in.table_rows > MAX_SMEM_TABLE || in.table_cols < 1) return false;
+	if (s->gap != GAP_LINEAR && s->gap != GAP_AFFINE) return false;
+	const pa_options &o = s->opt;
+	const bool affine = s->gap == GAP_AFFINE;
+	const double us = affine ? o.affine_u_s : o.linear_s, ut = affine ? o.affine_u_t : o.linear_t;
+	const double ws = affine ? double(o.affine_u_s) + o.affine_v_s : us, wt = affine ? double(o.affine_u_t) + o.affine_v_t : ut;
+	if (!(us >= 0 && ut >= 0 && ws >= 0 && wt >= 0)) return false;
+	double smax = 0;
+	for (int64_t k = 0; k < in.table_rows * in.table_cols; k++) {
+		const double v = double(host_table[k]) * s->sign;
+		if (v < -128 || v > 127) return false;
+		smax = std::max(smax, v);
+	}
+	double bmin = 0, bmax = 0;
+	for (int64_t k = 0; k <= mls && k < int64_t(s->left_D.size()); k++) {
+		if (!std::isfinite(s->left_D[size_t(k)])) return false;
+		bmin = std::min(bmin, double(s->left_D[size_t(k)]));
+		bmax = std::max(bmax, double(s->left_D[size_t(k)]));
+	}
+	for (int64_t k = 0; k <= mlt && k < int64_t(s->top_D.size()); k++) {
+		if (!std::isfinite(s->top_D[size_t(k)])) return false;
+		bmin = std::min(bmin, double(s->top_D[size_t(k)]));
+		bmax = std::max(bmax, double(s->top_D[size_t(k)]));
+	}
+	const double hi = smax * double(std::min(mls, mlt)) + bmax;
+	const double down = ws + us * double(mls + 256), across = wt + ut * double(mlt);
+	const double lo = s->loc == LOC_LOCAL ? 0.0 : s->loc == LOC_SEMI ? -std::min(down, across) : bmin - down - across;
+	const double step = std::max(ws, wt) + std::max(us, ut) + 128.0;
+	const double neg = -32767.0 + std::max({us, ut, ws, wt, 128.0});  // a gap below it stays in range
+	const double off = s->loc == LOC_LOCAL ? 0.0 : neg + step + 1.0 - lo;
+	if (lo + off - step < neg || hi + off > 32767.0) return false;
+	plan.s_neg = int32_t(neg);
+	plan.h_off = int32_t(off);
+	plan.h_low = int32_t((s->loc == LOC_GLOBAL ? lo : 0.0) + off);
 	return true;
 }
 
@@ -784,7 +843,8 @@ pa_status run_dp(pa_solver *s, const Input &in, const Plan &plan, int tb, const 
                  int codes_slot = 0, int side = 0, int seg_slot = -1) {
 	if (seg_slot < 0) seg_slot = codes_slot;  // the pipeline chunk whose segments this launch runs
 	const bool ISINT = std::is_same<V, int32_t>::value;
-	const bool tag = ISINT && tb != TB_ALL;
+	const bool s16 = ISINT && plan.s16;
+	const bool tag = ISINT && tb != TB_ALL && !s16;
 	const int scale = tag ? 4 : 1;
 	// side 1: a pipeline chunk on the second compute stream, with its own counter and scratch
 	cudaStream_t st = side ? s->cmp2 : s->stream;
@@ -824,7 +884,7 @@ pa_status run_dp(pa_solver *s, const Input &in, const Plan &plan, int tb, const 
 	p.out_sign = s->sign;
 	const int gk = s->gap;  // GAP_LINEAR / GAP_AFFINE / GAP_DTW
 	const int diag_tag = (tag && gk != GAP_DTW) ? 2 : 0;
-	const bool h16 = ISINT && plan.h16;
+	const bool h16 = ISINT && plan.h16 && !s16;
 
 	// ---- sequences and substitution
 	if (in.form == F_SERIES) {
@@ -887,6 +947,21 @@ pa_status run_dp(pa_solver *s, const Input &in, const Plan &plan, int tb, const 
 			p.h_ext_t = h16_pack(raw(-o.affine_u_t, 0));
 		}
 		p.h_neg = h16_value(plan.h_neg);
+	}
+	if (s16) {
+		auto both = [](float x) { return h16_pack(int32_t(std::nearbyint(x))); };
+		if (gk == GAP_LINEAR) {
+			p.k_up = both(-o.linear_s);
+			p.k_left = both(-o.linear_t);
+		} else {
+			p.k_open_s = both(-(o.affine_u_s + o.affine_v_s));
+			p.h_ext_s = both(-o.affine_u_s);
+			p.k_open_t = both(-(o.affine_u_t + o.affine_v_t));
+			p.h_ext_t = both(-o.affine_u_t);
+		}
+		p.h_off = plan.h_off;
+		p.h_neg = h16_pack(plan.s_neg);
+		p.h_low = h16_pack(plan.h_low);
 	}
 	// ---- borders: converted once per solver and arithmetic mode, then kept on the device
 	{
@@ -992,9 +1067,15 @@ pa_status run_dp(pa_solver *s, const Input &in, const Plan &plan, int tb, const 
 	const bool ch = plan.units;
 	const int cols = (ISINT && plan.C == 2 && tb != TB_ALL && !want_values) ? 2 : 1;
 	const int sub2 = !ISINT && plan.C == 2 ? plan.sub2 : -1;  // >= 0: dpf2_kernel
+	const int subs = in.table_cols <= 4 ? SUBS_PROFILE : SUBS_COLPROF;  // dps16_kernel
+	if (s16) {
+		smem = (size_t(in.table_rows * in.table_cols) + 15) & ~size_t(15);
+		smem += size_t(s16_smem(plan.G, subs == SUBS_COLPROF, plan.units));
+		if (subs == SUBS_COLPROF) smem += size_t(in.table_cols) * 32 * s16_warps(plan.units) * 16;
+	}
 	if (sub2 == SUBF_DENSE) smem = size_t(DPF2_RING) * 4 * BLOCK * 16;
 	const bool blk = h16 && plan.blk;
-	const uint64_t ckey = (okey + smem - smem0) | (uint64_t(sub2 + 1) << 36) | (uint64_t(ch) << 40) |
+	const uint64_t ckey = (okey + smem - smem0) | (uint64_t(s16 ? 7 : sub2 + 1) << 36) | (uint64_t(ch) << 40) |
 	                      (uint64_t(cols == 2) << 41) | (uint64_t(h16) << 42) | (uint64_t(blk) << 43);
 	for (const auto &kv : s->occ_cache)
 		if (kv.first == ckey) bps = kv.second;
@@ -1003,6 +1084,8 @@ pa_status run_dp(pa_solver *s, const Input &in, const Plan &plan, int tb, const 
 		                              : occupancy_dp16b_affine(loc, tb, smem, &bps);
 		else if (h16) e = gk == GAP_LINEAR ? occupancy_dp16_linear(loc, tb, cols, smem, &bps)
 		                                   : occupancy_dp16_affine(loc, tb, cols, smem, &bps);
+		else if (s16) e = gk == GAP_LINEAR ? occupancy_dps16_linear(loc, subs, ch, smem, &bps)
+		                                   : occupancy_dps16_affine(loc, subs, ch, smem, &bps);
 		else if (sub2 >= 0) e = gk == GAP_LINEAR   ? occupancy_dpf2_linear(loc, tb, sub2, smem, &bps)
 		                        : gk == GAP_AFFINE ? occupancy_dpf2_affine(loc, tb, sub2, smem, &bps)
 		                                           : occupancy_dpf2_dtw(loc, tb, sub2, smem, &bps);
@@ -1012,12 +1095,13 @@ pa_status run_dp(pa_solver *s, const Input &in, const Plan &plan, int tb, const 
 	bps = std::max(bps, 1);
 	if (s->occ_cache.size() < 64) s->occ_cache.push_back({ckey, bps});
 	const int gpw = segd ? p.slots_per_warp : 32 / plan.G;
-	const int64_t units_needed = h16 ? (npairs + 1) / 2 : npairs;  // twins or pairs
+	const int64_t units_needed = h16 || s16 ? (npairs + 1) / 2 : npairs;  // twins or pairs
 	const int64_t groups_needed = plan.units ? plan.ntickets
 	                              : segd     ? p.seg_task[p.nseg]  // warp tasks of the segments
 	                                         : (units_needed + gpw - 1) / gpw;  // warps needed
+	const int wpb = s16 ? s16_warps(plan.units) : WARPS;  // warps per block
 	int64_t grid = int64_t(s->sm_count) * bps;
-	grid = std::min<int64_t>(grid, (groups_needed + WARPS - 1) / WARPS);
+	grid = std::min<int64_t>(grid, (groups_needed + wpb - 1) / wpb);
 	// PA_GRID=exact: one block per WARPS work units, each warp takes one unit and exits -- the
 	// non-persistent launch of a plain per-bucket solve, kept for that comparison
 	bool exact = false;
@@ -1028,7 +1112,7 @@ pa_status run_dp(pa_solver *s, const Input &in, const Plan &plan, int tb, const 
 	// warps, so the launch fills the GPU.  Only where the tasks' costs differ and there are few of
 	// them per resident warp: the counter balances more (65,536 DNA pairs, 7 tasks a warp, run the
 	// same either way), and on equal tasks the classes only cost their atomics (4,096 pairs of
-	// 64 x 64: 28 against 21 us).  4,096 protein pairs of
+	// 64 x 64: 28 against 21 us), as on launches below SPREAD_MIN_CELLS, too short to gain them back.  4,096 protein pairs of
 	// 50..600 (int32) 0.80 -> 0.73 ms, 8,192 dense pairs of 32..512 (float) 1.72 -> 1.53 ms, 4,096
 	// series pairs of 128..1024 1.75 -> 1.63 ms.
 	if (!plan.units && !h16 && !exact && plan.uneven && groups_needed > WARPS &&
@@ -1062,6 +1146,8 @@ pa_status run_dp(pa_solver *s, const Input &in, const Plan &plan, int tb, const 
 		                              : launch_dp16b_affine(loc, tb, p, int(grid), smem, st);
 		else if (h16) e = gk == GAP_LINEAR ? launch_dp16_linear(loc, tb, cols, p, int(grid), smem, st)
 		                                   : launch_dp16_affine(loc, tb, cols, p, int(grid), smem, st);
+		else if (s16) e = gk == GAP_LINEAR ? launch_dps16_linear(loc, subs, ch, p, int(grid), smem, st)
+		                                   : launch_dps16_affine(loc, subs, ch, p, int(grid), smem, st);
 		else e = dp_launch<V>(gk, ch, loc, tb, want_values, p, int(grid), smem, st, cols);
 	} else if (sub2 >= 0) {
 		e = gk == GAP_LINEAR   ? launch_dpf2_linear(loc, tb, sub2, p, int(grid), smem, st)
@@ -1439,11 +1525,19 @@ struct TuneEntry {
 	int C;
 	bool blk;
 	bool seg;
+	bool s16;
 	int bucket_G[PA_BUCKETS];
 };
 std::mutex g_tune_mu;
 std::vector<TuneEntry> g_tune;
 constexpr double TUNE_MIN_CELLS = 4e6;  // smaller launches keep the analytic choice
+// Scores alone in 16 bits against int32 (pa_dps16.cuh): from here on the 16-bit kernel always won.
+// Below, a launch that leaves the GPU half empty gains nothing from two pairs per lane and pays for
+// two pairs' profiles at the head of a stripe, so the tuner times both, and below TUNE_MIN_CELLS
+// the int32 kernel runs (266 pairs of 13..27 x 51..102: 98 us a call in int32, 107 in 16 bits; 1,203
+// of 39..196 x 20..80 89 and 101; 2,647 of 35..350 x 36..144 211 and 171).
+constexpr double S16_SURE_CELLS = 2e8;
+constexpr int64_t SPREAD_MIN_CELLS = 50000000;  // smaller launches take their tasks from one counter
 
 uint64_t tune_key(const pa_solver *s, const Input &in, const Plan &plan, const std::vector<int32_t> &ls,
                   const std::vector<int32_t> &lt, double *cells) {
@@ -1465,7 +1559,8 @@ uint64_t tune_key(const pa_solver *s, const Input &in, const Plan &plan, const s
 	return oct(double(n)) | (half(n ? sls / n : 0) << 6) | (half(n ? slt / n : 0) << 12) | (oct(double(mls)) << 18) |
 	       (oct(double(mlt)) << 24) | (uint64_t(s->gap & 3) << 30) | (uint64_t(s->loc & 3) << 32) |
 	       (uint64_t(plan.tb & 3) << 34) | (uint64_t(plan.use_int) << 36) | (uint64_t(in.form & 3) << 37) |
-	       (tabk << 39) | (uint64_t(s->sm_count & 1023) << 41) | (uint64_t(s->device & 63) << 51);
+	       (tabk << 39) | (uint64_t(s->sm_count & 1023) << 41) | (uint64_t(s->device & 63) << 51) |
+	       (uint64_t(plan.s16) << 57);
 }
 
 template <typename Stage, typename Dp>
@@ -1485,15 +1580,21 @@ pa_status tune_plan(pa_solver *s, const std::vector<int32_t> &ls, const std::vec
 				plan.units = t.units;
 				plan.h16 = plan.h16 && t.h16;  // the 16-bit kernel still needs this launch's bounds
 				plan.blk = plan.h16 && t.blk;
+				plan.s16 = plan.s16 && t.s16;
 				plan.C = plan.h16 ? t.C : cols_of(plan, plan.units);
 				plan.seg = plan.h16 && !plan.blk && t.seg;
 				for (int k = 0; k < PA_BUCKETS; k++) plan.bucket_G[k] = t.bucket_G[k];
 				return PA_OK;
 			}
 	}
-	if (cells < TUNE_MIN_CELLS) return PA_OK;
+	if (cells < TUNE_MIN_CELLS) {
+		plan.s16 = false;  // (see S16_SURE_CELLS)
+		return PA_OK;
+	}
 	// candidates: every group width whose stripe is not far taller than the pairs, and the
 	// stripe-chained mode when the longest pairs span several 256-row stripes
+	// (scores alone that fit 16 bits: dps16_kernel, and beside it the int32 kernel while the
+	// launch is small)
 	// (G, chained, 16-bit twins, columns per step): the 16-bit kernel, with one or two columns
 	// per step, where this launch's bounds admit it
 	const int C0 = plan.C32;
@@ -1502,26 +1603,29 @@ pa_status tune_plan(pa_solver *s, const std::vector<int32_t> &ls, const std::vec
 		bool units, h16;
 		int C;
 		bool blk;
+		bool s16;
 	};
 	std::vector<Cand> cand;
+	const bool both = plan.s16 && cells < S16_SURE_CELLS;
 	for (int G : {32, 16, 8, 4, 2, 1})
 		if (G == 4 || (int64_t(G) * R <= 2 * plan.max_ls && (G >= 4 || plan.max_ls <= 256))) {
-			cand.push_back({G, false, false, C0, false});
-			if (plan.h16) {
-				cand.push_back({G, false, true, 1, false});
-				if (C0 == 2) cand.push_back({G, false, true, 2, false});
+			cand.push_back({G, false, false, C0, false, plan.s16});
+			if (both) cand.push_back({G, false, false, C0, false, false});
+			if (plan.h16 && !plan.s16) {
+				cand.push_back({G, false, true, 1, false, false});
+				if (C0 == 2) cand.push_back({G, false, true, 2, false, false});
 			}
 		}
 	// the 16-bit 4 x 4 block kernel (stripes of 4 G rows: the tile height 4 instead of 8)
-	if (plan.h16 && C0 == 2)
+	if (plan.h16 && !plan.s16 && C0 == 2)
 		for (int G : {32, 16, 8})
-			if (int64_t(G) * 4 <= 2 * plan.max_ls) cand.push_back({G, false, true, 4, true});
-	if (plan.max_ls > 2 * 32 * R) cand.push_back({32, true, false, cols_of(plan, true), false});
+			if (int64_t(G) * 4 <= 2 * plan.max_ls) cand.push_back({G, false, true, 4, true, false});
+	if (plan.max_ls > 2 * 32 * R) cand.push_back({32, true, false, cols_of(plan, true), false, plan.s16});
 	if (cand.size() < 2) return PA_OK;
 	cudaStream_t st = s->stream;
 	float best = INFINITY;
 	int bestG = plan.G, bestC = plan.C;
-	bool bestU = plan.units, bestH = plan.h16, bestB = plan.blk;
+	bool bestU = plan.units, bestH = plan.h16, bestB = plan.blk, bestS = plan.s16;
 	auto time_plan = [&](Plan &pl, int reps, float *ms) -> pa_status {
 		if (pa_status e = stage(pl)) return e;
 		*ms = INFINITY;
@@ -1544,6 +1648,7 @@ pa_status tune_plan(pa_solver *s, const std::vector<int32_t> &ls, const std::vec
 		pl.h16 = c.h16;
 		pl.C = c.C;
 		pl.blk = c.blk;
+		pl.s16 = c.s16;
 		pl.seg = false;
 		return pl;
 	};
@@ -1591,6 +1696,7 @@ pa_status tune_plan(pa_solver *s, const std::vector<int32_t> &ls, const std::vec
 			bestH = cand[ci].h16;
 			bestC = cand[ci].C;
 			bestB = cand[ci].blk;
+			bestS = cand[ci].s16;
 		}
 	}
 	plan.G = bestG;
@@ -1598,6 +1704,7 @@ pa_status tune_plan(pa_solver *s, const std::vector<int32_t> &ls, const std::vec
 	plan.h16 = bestH;
 	plan.C = bestC;
 	plan.blk = bestB;
+	plan.s16 = bestS;
 	plan.seg = false;
 	if (bestH && !bestB && !bestU) {
 		// a width per length bucket, by measurement: from the uniform plan, each populated
@@ -1648,7 +1755,7 @@ pa_status tune_plan(pa_solver *s, const std::vector<int32_t> &ls, const std::vec
 	}
 	std::lock_guard<std::mutex> lk(g_tune_mu);
 	if (g_tune.size() < 4096) {
-		TuneEntry t{key, bestG, bestU, bestH, bestC, bestB, plan.seg, {}};
+		TuneEntry t{key, bestG, bestU, bestH, bestC, bestB, plan.seg, bestS, {}};
 		for (int b = 0; b < PA_BUCKETS; b++) t.bucket_G[b] = plan.bucket_G[b];
 		g_tune.push_back(t);
 	}
@@ -1834,7 +1941,7 @@ pa_status solve_impl(pa_solver *s, const Input &in, int method, float *scores_ou
 			sum += c;
 			n += c > 0;
 		}
-		plan.uneven = 2 * most * n > 3 * sum;  // the largest pair over 1.5 times the mean
+		plan.uneven = 2 * most * n > 3 * sum && sum >= SPREAD_MIN_CELLS;  // the largest over 1.5 times the mean
 	}
 	if (!hit && s->gap != GAP_GENERAL) {
 		plan.units = choose_units(ls, lt, s->sm_count, plan.G);
@@ -1868,6 +1975,7 @@ pa_status solve_impl(pa_solver *s, const Input &in, int method, float *scores_ou
 			if (std::atoi(e) == 1) plan.C32 = 1;
 		plan.C = cols_of(plan, plan.units);
 		int32_t hneg = 0;
+		plan.s16 = s16_plan(s, in, host_table.data(), max_ls, max_lt, plan);
 		plan.h16 = !plan.units && h16_plan(s, in, host_table.data(), ls, lt, tb, want_values, use_int, &hneg);
 		plan.h_neg = hneg;
 		if (plan.h16) plan.C = plan.C32;  // two columns per step unless PA_DP_COLS=1
@@ -1971,17 +2079,20 @@ pa_status solve_impl(pa_solver *s, const Input &in, int method, float *scores_ou
 		// (an empty pair counts as one stripe, which writes its border result); the order puts
 		// those pairs first, so stripe q of rank w is ticket level_start[q] + w
 		level_start.clear();
+		// (scores in 16-bit twins: stripe q of the twin at rank w, which has as many stripes as its
+		// first, longer pair)
 		if (plan.units) {
-			const int64_t rpp_u = int64_t(plan.G) * R;
+			const int64_t rpp_u = int64_t(plan.G) * R, nunits = plan.s16 ? (B + 1) / 2 : B;
 			std::vector<int64_t> hist;
-			for (int64_t k = 0; k < B; k++) {
-				const int64_t np = std::max<int64_t>(1, (ls[size_t(k)] + rpp_u - 1) / rpp_u);
+			for (int64_t w = 0; w < nunits; w++) {
+				const size_t k = plan.s16 ? size_t(order[size_t(2 * w)]) : size_t(w);
+				const int64_t np = std::max<int64_t>(1, (ls[k] + rpp_u - 1) / rpp_u);
 				if (int64_t(hist.size()) <= np) hist.resize(size_t(np) + 1, 0);
 				hist[size_t(np)]++;
 			}
 			const int64_t nlev = int64_t(hist.size()) - 1;
 			level_start.assign(size_t(nlev) + 1, 0);
-			int64_t above = B;  // pairs with more than q stripes
+			int64_t above = nunits;  // pairs (twins) with more than q stripes
 			for (int64_t q = 0; q < nlev; q++) {
 				level_start[size_t(q) + 1] = int32_t(level_start[size_t(q)] + above);
 				above -= hist[size_t(q) + 1];
@@ -2319,6 +2430,10 @@ pa_status solve_impl(pa_solver *s, const Input &in, int method, float *scores_ou
 		plan.seg = r.seg;
 		plan.uneven = r.uneven;
 		plan.sub2 = r.sub2;
+		plan.s16 = r.s16;
+		plan.s_neg = r.s_neg;
+		plan.h_off = r.h_off;
+		plan.h_low = r.h_low;
 		plan.copy_pitch = r.copy_pitch;
 		for (int k = 0; k < PA_BUCKETS; k++) plan.bucket_G[k] = r.bucket_G[k];
 		for (int c = 0; c < PA_MAX_CHUNKS; c++) plan.segs[c] = r.segs[c];
@@ -2391,12 +2506,13 @@ pa_status solve_impl(pa_solver *s, const Input &in, int method, float *scores_ou
 	}
 	res.G = plan.G;
 	s->last_plan[0] = s->gap == GAP_GENERAL ? 4
+	                  : plan.s16 && !plan.units ? 5
 	                  : plan.h16  ? (plan.blk ? 6 : plan.C == 2 ? 5 : 3)
 	                  : plan.units ? 2
 	                  : plan.C == 2 ? 1
 	                               : 0;
 	s->last_plan[1] = plan.G;
-	s->last_plan[2] = plan.h16 ? 2 : plan.use_int ? 1 : 0;
+	s->last_plan[2] = plan.h16 || plan.s16 ? 2 : plan.use_int ? 1 : 0;
 	s->last_plan[3] = hit && s->rep.exec ? 1 : 0;
 	for (int k = 0; k < PA_BUCKETS; k++) s->last_widths[k] = plan.seg ? plan.bucket_G[k] : 0;
 	PA_CUDA(cudaEventRecord(s->ev[3], st));
@@ -2444,6 +2560,10 @@ pa_status solve_impl(pa_solver *s, const Input &in, int method, float *scores_ou
 		r.seg = plan.seg;
 		r.uneven = plan.uneven;
 		r.sub2 = plan.sub2;
+		r.s16 = plan.s16;
+		r.s_neg = plan.s_neg;
+		r.h_off = plan.h_off;
+		r.h_low = plan.h_low;
 		r.copy_pitch = plan.copy_pitch;
 		for (int k = 0; k < PA_BUCKETS; k++) r.bucket_G[k] = plan.bucket_G[k];
 		for (int c = 0; c < PA_MAX_CHUNKS; c++) r.segs[c] = plan.segs[c];
