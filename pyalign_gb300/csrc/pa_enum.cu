@@ -18,13 +18,21 @@
 // DP wrote (pa_dp.cuh layout: stripe q, step s, lane k, one uint4 of 8 rows of 16-bit cells).
 // The control flow is warp-uniform: every lane follows the same search, lane 0 alone reads
 // and writes the stack and the path (so it always sees its own writes), and the lanes
-// cooperate where the work is wide -- a 32-row x 32-column window of mask cells loaded into
+// cooperate where the work is wide -- a 64-row x 64-column window of mask cells loaded into
 // shared memory (one uint4 per lane and row block; the search walks up and left, so a
-// diagonal path reloads it every 32 steps), and at each yielded path the compression, the
+// diagonal path reloads it every 64 steps), and at each yielded path the compression, the
 // map (s_to_t or t_to_s, the reference's build_alignment from the compressed points,
 // solver.h:940-1086) and the de-duplication test, 32 path points per lane step.  The last
 // entry a point pushes is the next one popped, so it stays in registers and only the others
-// are written to the stack.  Local seeds come from enum_seed_kernel (every cell with the
+// are written to the stack.  Most cells of a path have the diagonal as their only entry: from
+// every cell the lanes test the 32 cells up its diagonal at once (one ballot), and a run of such
+// cells is appended to the path in one step; only the cells that branch go through the search.
+// What bounds it then is round trips: one per window and, per yielded path, those of reading the
+// path back, 256 points in flight together.  A yield differs from the one before it only past
+// the point where the search turned, mostly near the path's end: with the pair's current map in
+// shared memory (pairs of up to ENUM_SMEM_MAP) only that part of map and hash is worked out.  The
+// stack's lower 256 entries lie there too.  16 pairs of 2000..3000 x 3000..5000, the first 101
+// alignments of each: 9.66 -> 2.83 ms.  Local seeds come from enum_seed_kernel (every cell with the
 // seed bit, one block per pair), sorted on the host in the order the reference's stack
 // pops them: increasing row, then increasing column.
 //
@@ -74,29 +82,37 @@ __global__ void __launch_bounds__(256) enum_seed_kernel(SeedScanParams p) {
 	}
 }
 
+constexpr int WIN_B = 8;    // row blocks (of 8 rows) and columns of a warp's window: the searches of
+constexpr int WIN_C = 64;   // neighbouring yields differ near the path's end and mostly stay inside
+constexpr int SMEM_STACK = 256;  // entries of the stack kept in shared memory
+
 struct Window {
-	int gb0, j0;  // row blocks [gb0, gb0 + 4), columns [j0, j0 + 32)
+	int gb0, j0;  // row blocks [gb0, gb0 + WIN_B), columns [j0, j0 + WIN_C)
 };
 
 // cell (i, j) of the pair's masks through the warp's shared window (warp-uniform call)
-__device__ __forceinline__ uint32_t enum_cell(const EnumParams &p, uint4 (*win)[32], Window &w, const uint4 *m,
+__device__ __forceinline__ uint32_t enum_cell(const EnumParams &p, uint4 (*win)[WIN_C], Window &w, const uint4 *m,
                                               int64_t S, int ls, int lt, int i, int j, int lane) {
 	const int gb = i >> 3;
-	if (gb < w.gb0 || gb >= w.gb0 + 4 || j < w.j0 || j >= w.j0 + 32) {
-		w.gb0 = max(0, gb - 3);
-		w.j0 = max(0, j - 31);
+	if (gb < w.gb0 || gb >= w.gb0 + WIN_B || j < w.j0 || j >= w.j0 + WIN_C) {
+		w.gb0 = max(0, gb - (WIN_B - 1));
+		w.j0 = max(0, j - (WIN_C - 1));
 		__syncwarp();  // every lane is done with the old window
-		const int jj = w.j0 + lane;
-		if (jj < lt) {
+		uint4 x[WIN_B][2];  // every load in flight together
 #pragma unroll
-			for (int r = 0; r < 4; r++) {
-				const int g = w.gb0 + r;
-				if (g * R < ls) {
-					const int q = g / p.G, sb = g - q * p.G;
-					win[r][lane] = m[(int64_t(q) * S + jj + sb) * p.G + sb];
-				}
+		for (int r = 0; r < WIN_B; r++) {
+			const int g = w.gb0 + r, q = g / p.G, sb = g - q * p.G;
+#pragma unroll
+			for (int h = 0; h < 2; h++) {
+				const int jj = w.j0 + lane + 32 * h;
+				if (jj < lt && g * R < ls) x[r][h] = m[(int64_t(q) * S + jj + sb) * p.G + sb];
 			}
 		}
+#pragma unroll
+		for (int r = 0; r < WIN_B; r++)
+#pragma unroll
+			for (int h = 0; h < 2; h++)
+				if (w.j0 + lane + 32 * h < lt && (w.gb0 + r) * R < ls) win[r][lane + 32 * h] = x[r][h];
 		__syncwarp();
 	}
 	const uint4 e = win[gb - w.gb0][j - w.j0];
@@ -114,12 +130,14 @@ __device__ __forceinline__ unsigned long long enum_mix(int u, int v) {
 	return x ^ (x >> 31);
 }
 
-__global__ void __launch_bounds__(WARPS * 32) enum_kernel(EnumParams p) {
-	__shared__ uint4 win_all[WARPS][4][32];
-	const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-	uint4 (*win)[32] = win_all[wib];
-	const int wi = blockIdx.x * WARPS + wib;
-	if (wi >= p.nwork) return;
+// SM: the pair's current map is kept in shared memory (p.smem_map entries).  A block of one warp.
+template <bool SM>
+__global__ void __launch_bounds__(32) enum_kernel(EnumParams p) {
+	__shared__ uint4 win[WIN_B][WIN_C];
+	__shared__ int4 top[SMEM_STACK];  // stack entries 0 .. SMEM_STACK - 1 (the others in p.stack)
+	extern __shared__ int32_t smap[];
+	const int lane = threadIdx.x & 31;
+	const int wi = blockIdx.x;
 	const int L = p.work[wi];
 	const int ls = p.len_s[L], lt = p.len_t[L];
 	const int m = min(ls, lt);
@@ -133,7 +151,7 @@ __global__ void __launch_bounds__(WARPS * 32) enum_kernel(EnumParams p) {
 	unsigned long long *hash = p.hash + int64_t(L) * p.k;
 	int32_t *npts = p.npts + int64_t(L) * p.k;
 	const int plen_cap = ls + lt + 2;
-	Window w{-16, -64};
+	Window w{-WIN_B, -WIN_C};
 
 	int count = 0, sp = 0, si = 0, status = 0;
 	const int nseed = p.local ? p.seed_n[L] : 0;
@@ -145,15 +163,25 @@ __global__ void __launch_bounds__(WARPS * 32) enum_kernel(EnumParams p) {
 		ev = p.seed[2 * L + 1];
 		have = true;
 	}
+	// path points 0 .. low - 1 are those of the last complete path; its hash and point count
+	int low = 0, n = 0;
+	unsigned long long h = 0;
+	if (SM)
+		for (int x = lane; x < m; x += 32) smap[x] = -1;
 	while (count < p.k) {
 		if (!have) {
 			if (sp > 0) {
 				int4 t = make_int4(0, 0, 0, 0);
-				if (lane == 0) t = stk[sp - 1];
+				sp--;
+				if (sp < SMEM_STACK) {
+					__syncwarp();  // lane 0's write of it
+					t = top[sp];
+				} else if (lane == 0) {
+					t = stk[sp];
+				}
 				eu = __shfl_sync(0xffffffffu, t.x, 0);
 				ev = __shfl_sync(0xffffffffu, t.y, 0);
 				epl = __shfl_sync(0xffffffffu, t.z, 0);
-				sp--;
 			} else if (si < nseed) {
 				const int2 s = seeds[si++];
 				eu = s.x;
@@ -164,19 +192,39 @@ __global__ void __launch_bounds__(WARPS * 32) enum_kernel(EnumParams p) {
 			}
 		}
 		have = false;
+		low = min(low, epl);
 		int plen = epl;
 		if (plen >= plen_cap) {  // cannot happen: every step lowers u + v
 			status = ENUM_BAD_PATH;
 			break;
 		}
-		if (lane == 0) path[plen] = make_int2(eu, ev);
-		plen++;
 		bool cont = eu >= 0 && ev >= 0;
 		uint32_t c = 0;
 		if (cont) {
-			c = enum_cell(p, win, w, mk, S, ls, lt, eu, ev, lane);
+			c = enum_cell(p, win, w, mk, S, ls, lt, eu, ev, lane);  // the window holds (eu, ev)
+			// lane k: cell (eu - k, ev - k), while it lies in the window and its list is the diagonal
+			const int i = eu - lane, j = ev - lane;
+			bool simple = i >= 0 && j >= 0 && (i >> 3) >= w.gb0 && j >= w.j0;
+			if (simple) {
+				const uint32_t *e = reinterpret_cast<const uint32_t *>(&win[(i >> 3) - w.gb0][j - w.j0]);
+				simple = ((e[(i & 7) >> 1] >> (16 * (i & 1))) & 15u) == 2u;
+			}
+			const uint32_t b = __ballot_sync(0xffffffffu, simple);
+			const int run = min(b == 0xffffffffu ? 32 : __ffs(int(~b)) - 1, plen_cap - plen);
+			if (run > 0) {
+				__syncwarp();  // and may overwrite points of an earlier path
+				if (lane < run) path[plen + lane] = make_int2(i, j);
+				__syncwarp();  // a later path may overwrite these points from other lanes
+				eu -= run;
+				ev -= run;
+				epl = plen + run;
+				have = true;
+				continue;
+			}
 			if (p.local && (c & 1u)) cont = false;
 		}
+		if (lane == 0) path[plen] = make_int2(eu, ev);
+		plen++;
 		if (cont) {
 			// the list in push order; every entry but the last goes to the stack, the last is
 			// popped next and stays in registers
@@ -187,7 +235,7 @@ __global__ void __launch_bounds__(WARPS * 32) enum_kernel(EnumParams p) {
 				if (pend) {
 					if (sp >= cap) over = true;
 					else {
-						if (lane == 0) stk[sp] = make_int4(nu, nv, plen, 0);
+						if (lane == 0) (sp < SMEM_STACK ? top[sp] : stk[sp]) = make_int4(nu, nv, plen, 0);
 						sp++;
 					}
 				}
@@ -232,47 +280,100 @@ __global__ void __launch_bounds__(WARPS * 32) enum_kernel(EnumParams p) {
 			continue;
 		}
 
-		// ---- a complete path: path[0, plen).  Its map, hash and point count, 32 points per step
-		__syncwarp();  // lane 0's path writes are visible to the warp
+		// ---- a complete path: path[0, plen).  Its map, hash and point count.  With the map in
+		// shared memory only what differs from the last complete path is worked out: the points
+		// from low - 1 on, whose map entries are those at or below that point's coordinate (a path
+		// falls in both coordinates, and strictly at each aligned cell before it)
+		__syncwarp();  // the path's writes are visible to the warp
 		int32_t *mp = maps + int64_t(count) * m;
-		for (int x = lane; x < m; x += 32) mp[x] = -1;
-		__syncwarp();
-		unsigned long long h = 0;
-		int n = 0;
-		for (int t = lane; t + 1 < plen; t += 32) {
-			const int2 a = path[t], b = path[t + 1];
-			if (b.x != a.x && b.y != a.y && a.x >= 0 && a.y >= 0) {
-				if (s_side) mp[a.x] = a.y;
-				else mp[a.y] = a.x;
-				h += enum_mix(a.x, a.y);
-				n++;
+		unsigned long long dh = 0;  // this lane's change of the hash and the count
+		int dn = 0;
+		int first = 0;
+		if (SM) {
+			int bound = m - 1;
+			if (low > 0) {
+				const int2 a = path[low - 1];
+				bound = min(bound, s_side ? a.x : a.y);
+				first = low - 1;
+			}
+			for (int x = lane; x <= bound; x += 32) {
+				const int y = smap[x];
+				if (y >= 0) {
+					dh -= s_side ? enum_mix(x, y) : enum_mix(y, x);
+					dn--;
+					smap[x] = -1;
+				}
+			}
+			__syncwarp();
+		} else {
+			for (int x = lane; x < m; x += 32) mp[x] = -1;
+			h = 0;
+			n = 0;
+			__syncwarp();
+		}
+		for (int t0 = first; t0 + 1 < plen; t0 += 32 * 8) {
+			// lane l holds points t0 + 32 x + l; a point's successor comes from the next lane
+			int2 a[8];
+#pragma unroll
+			for (int x = 0; x < 8; x++) {
+				const int t = t0 + 32 * x + lane;
+				a[x] = t < plen ? path[t] : make_int2(0, 0);
+			}
+			const int2 past = t0 + 256 < plen ? path[t0 + 256] : make_int2(0, 0);
+#pragma unroll
+			for (int x = 0; x < 8; x++) {
+				int bx = __shfl_down_sync(0xffffffffu, a[x].x, 1), by = __shfl_down_sync(0xffffffffu, a[x].y, 1);
+				const int fx = x < 7 ? __shfl_sync(0xffffffffu, a[x < 7 ? x + 1 : 7].x, 0) : past.x;
+				const int fy = x < 7 ? __shfl_sync(0xffffffffu, a[x < 7 ? x + 1 : 7].y, 0) : past.y;
+				if (lane == 31) {
+					bx = fx;
+					by = fy;
+				}
+				if (t0 + 32 * x + lane + 1 < plen && bx != a[x].x && by != a[x].y && a[x].x >= 0 && a[x].y >= 0) {
+					int32_t *const to = SM ? smap : mp;
+					if (s_side) to[a[x].x] = a[x].y;
+					else to[a[x].y] = a[x].x;
+					dh += enum_mix(a[x].x, a[x].y);
+					dn++;
+				}
 			}
 		}
+		low = plen;
 #pragma unroll
 		for (int o = 16; o > 0; o >>= 1) {
-			h += __shfl_xor_sync(0xffffffffu, h, o);
-			n += __shfl_xor_sync(0xffffffffu, n, o);
+			dh += __shfl_xor_sync(0xffffffffu, dh, o);
+			dn += __shfl_xor_sync(0xffffffffu, dn, o);
 		}
+		h += dh;
+		n += dn;
 		__syncwarp();  // the map is complete
 		bool dup = false;
 		if (p.remove_dup) {
-			for (int r = 0; r < count && !dup; r++) {
-				if (hash[r] != h || npts[r] != n) continue;
-				const int32_t *mr = maps + int64_t(r) * m;
-				bool same = true;
-				for (int x = lane; x < m; x += 32) same &= mr[x] == mp[x];
-				dup = __all_sync(0xffffffffu, same);
+			for (int r0 = 0; r0 < count && !dup; r0 += 32) {
+				// 32 earlier yields at a time; those of equal hash and count are compared in full
+				const int rl = r0 + lane;
+				uint32_t like = __ballot_sync(0xffffffffu, rl < count && hash[rl] == h && npts[rl] == n);
+				for (; like && !dup; like &= like - 1) {
+					const int32_t *mr = maps + int64_t(r0 + __ffs(int(like)) - 1) * m;
+					bool same = true;
+					for (int x = lane; x < m; x += 32) same &= mr[x] == (SM ? smap[x] : mp[x]);
+					dup = __all_sync(0xffffffffu, same);
+				}
 			}
 		}
 		if (dup) continue;
+		if (SM)
+			for (int x = lane; x < m; x += 32) mp[x] = smap[x];
 		if (lane == 0) {
 			hash[count] = h;
 			npts[count] = n;
 		}
+		__syncwarp();  // the other lanes read them at the next yield
 		if (p.paths) {
 			int2 *po = p.paths + p.paths_off[L] + int64_t(count) * plen_cap;
 			for (int t = lane; t < plen; t += 32) po[t] = path[t];
 			if (lane == 0) p.path_len[int64_t(L) * p.k + count] = plen;
+			__syncwarp();  // the path may be overwritten
 		}
 		count++;
 	}
@@ -293,8 +394,17 @@ cudaError_t enum_seed_scan(const SeedScanParams &p, int grid, cudaStream_t st) {
 }
 
 cudaError_t enum_solve(const EnumParams &p, cudaStream_t st) {
-	const int grid = (p.nwork + WARPS - 1) / WARPS;
-	if (grid > 0) enum_kernel<<<grid, WARPS * 32, 0, st>>>(p);
+	if (p.nwork <= 0) return cudaSuccess;
+	if (p.smem_map > 0) {
+		const int bytes = p.smem_map * 4;
+		if (bytes > 32 * 1024)  // beside 12 KB of static shared memory
+			if (cudaError_t e = cudaFuncSetAttribute(enum_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+			                                         ENUM_SMEM_MAP * 4))
+				return e;
+		enum_kernel<true><<<p.nwork, 32, bytes, st>>>(p);
+	} else {
+		enum_kernel<false><<<p.nwork, 32, 0, st>>>(p);
+	}
 	return cudaGetLastError();
 }
 

@@ -37,7 +37,9 @@ struct EnumParams {
 	int32_t *npts;              // k per pair
 	int32_t *count;             // per pair: paths yielded (<= k)
 	int32_t *status;            // per pair: ENUM_OVERFLOW
+	int32_t smem_map;           // the largest map when it is kept in shared memory, else 0
 };
+constexpr int32_t ENUM_SMEM_MAP = 40960;  // at most (160 KB)
 
 struct SeedScanParams {
 	int32_t nwork;

@@ -3406,6 +3406,9 @@ void pa_iterator_destroy(pa_iterator *it) { delete it; }
 }  // extern "C"
 
 namespace pa {
+cudaError_t path_count_band(int32_t npairs, const int32_t *work, int32_t G, int32_t affine, const int32_t *len_s,
+                            const int32_t *len_t, const int64_t *mask_off, const void *masks, const int32_t *seed,
+                            unsigned long long *counts, int32_t *left, bool wide, cudaStream_t st);
 cudaError_t path_count_solve(int32_t npairs, int32_t G, int32_t local, int32_t affine, const int32_t *len_s,
                              const int32_t *len_t, const int64_t *mask_off, const void *masks, const int32_t *seed,
                              unsigned long long *counts, unsigned long long *scratch, int64_t scratch_stride,
@@ -3458,15 +3461,59 @@ pa_status pa_result_path_counts(const pa_result *r, uint64_t *counts) {
 			if (d.ls[size_t(k)] > 0 && d.lt[size_t(k)] > 0)
 				max_np = std::max<int64_t>(max_np, (d.ls[size_t(k)] + rpp32 - 1) / rpp32);
 		bool chain = d.G == 32 && max_np >= 3;
-		if (const char *e = std::getenv("PA_COUNT_MODE"))  // tests: "group" or "chain" (G = 32 only)
+		// one seed per pair (not local alignment): along the band of its co-optimal paths, which is
+		// the faster at every size measured, 64 x 64 to 4000 x 4000, one pair to 4000 (pa_count.cu)
+		std::vector<int32_t> ls_left(d.ls.begin(), d.ls.end()), lt_left(d.lt.begin(), d.lt.end());
+		bool band = !local;
+		if (const char *e = std::getenv("PA_COUNT_MODE")) {  // tests: "group" or "chain" (G = 32 only)
 			chain = std::strcmp(e, "chain") == 0 ? d.G == 32 : std::strcmp(e, "group") == 0 ? false : chain;
+			band = false;
+		}
 		std::vector<uint64_t> c(static_cast<size_t>(B), 0);
-		if (chain) {
+		std::vector<int32_t> work;
+		int64_t todo = 0;  // pairs that the band leaves to the kernels over whole matrices
+		for (int64_t k = 0; k < B; k++) {
+			if (d.ls[size_t(k)] == 0 || d.lt[size_t(k)] == 0 || (!local && !d.has[size_t(k)])) continue;
+			if (band) work.push_back(int32_t(k));
+			else todo++;
+		}
+		// in 64 rows, then those it was too narrow for in 256; a few pairs in 256 at once
+		for (int wide = int64_t(work.size()) <= sms ? 1 : 0; wide < 2 && !work.empty(); wide++) {
+			const size_t n = work.size();
+			PA_CUDA(dord.ensure(n * 4));
+			PA_CUDA(dprog.ensure(size_t(B) * 4));
+			PA_CUDA(cudaMemcpy(dord.p, work.data(), n * 4, cudaMemcpyHostToDevice));
+			PA_CUDA(pa::path_count_band(int32_t(n), dord.as<int32_t>(), d.G, d.gap == GAP_AFFINE ? 1 : 0, dl.as<int32_t>(),
+			                            dl.as<int32_t>() + B, dm.as<int64_t>(), d.dev_masks_all, dseed.as<int32_t>(),
+			                            dcnt.as<unsigned long long>(), dprog.as<int32_t>(), wide != 0, nullptr));
+			std::vector<int32_t> left(static_cast<size_t>(B)), again;
+			std::vector<uint64_t> bc(static_cast<size_t>(B));
+			PA_CUDA(cudaMemcpy(left.data(), dprog.p, size_t(B) * 4, cudaMemcpyDeviceToHost));
+			PA_CUDA(cudaMemcpy(bc.data(), dcnt.p, size_t(B) * 8, cudaMemcpyDeviceToHost));
+			for (int32_t k : work) {
+				if (left[size_t(k)] == 0) {
+					c[size_t(k)] = bc[size_t(k)];
+					ls_left[size_t(k)] = lt_left[size_t(k)] = 0;  // an empty pair for the kernels below
+				} else if (left[size_t(k)] == 1 && wide == 0) {
+					again.push_back(k);
+				} else {
+					todo++;
+				}
+			}
+			work.swap(again);
+		}
+		if (todo > 0) {
+			PA_CUDA(cudaMemcpy(dl.p, ls_left.data(), size_t(B) * 4, cudaMemcpyHostToDevice));
+			PA_CUDA(cudaMemcpy(dl.as<int32_t>() + B, lt_left.data(), size_t(B) * 4, cudaMemcpyHostToDevice));
+		}
+		if (todo == 0) {
+			// every pair is counted
+		} else if (chain) {
 			// tickets stripe-major: level q holds stripe q of every pair with more than q stripes
 			// (an empty pair counts as one), the pairs with the most stripes first
 			std::vector<int32_t> np(static_cast<size_t>(B)), order(static_cast<size_t>(B)), rank(static_cast<size_t>(B));
 			for (int64_t k = 0; k < B; k++) {
-				const int64_t a = d.ls[size_t(k)], b = d.lt[size_t(k)];
+				const int64_t a = ls_left[size_t(k)], b = lt_left[size_t(k)];
 				np[size_t(k)] = int32_t(std::max<int64_t>(1, (a == 0 || b == 0) ? 1 : (a + rpp32 - 1) / rpp32));
 				order[size_t(k)] = int32_t(k);
 			}
@@ -3506,6 +3553,7 @@ pa_status pa_result_path_counts(const pa_result *r, uint64_t *counts) {
 				return fail(PA_ERR_TIMEOUT, "a chained stripe of the path count timed out waiting for the stripe above it");
 			for (int64_t k = 0; k < B; k++)
 				for (int32_t q = 0; q < np[size_t(k)]; q++) {
+					if (ls_left[size_t(k)] == 0) break;
 					const uint64_t x = part[size_t(level_start[size_t(q)] + rank[size_t(k)])];
 					const uint64_t y = c[size_t(k)] + x;
 					c[size_t(k)] = y < x ? ~uint64_t(0) : y;
@@ -3522,7 +3570,10 @@ pa_status pa_result_path_counts(const pa_result *r, uint64_t *counts) {
 			                             dcnt.as<unsigned long long>(), dscr.as<unsigned long long>(), stride,
 			                             dctr.as<int32_t>(), int(grid), nullptr, 0, 0, nullptr, nullptr, nullptr, nullptr,
 			                             nullptr));
-			PA_CUDA(cudaMemcpy(c.data(), dcnt.p, size_t(B) * 8, cudaMemcpyDeviceToHost));
+			std::vector<uint64_t> whole(static_cast<size_t>(B));
+			PA_CUDA(cudaMemcpy(whole.data(), dcnt.p, size_t(B) * 8, cudaMemcpyDeviceToHost));
+			for (int64_t k = 0; k < B; k++)
+				if (ls_left[size_t(k)] > 0 && lt_left[size_t(k)] > 0) c[size_t(k)] = whole[size_t(k)];
 		}
 		for (int64_t k = 0; k < B; k++) {
 			const int ls = d.ls[size_t(k)], lt = d.lt[size_t(k)];
@@ -3739,6 +3790,11 @@ pa_status pa_result_first_alignments(const pa_result *r, int32_t k, int32_t *cou
 		ep.npts = dnpts.as<int32_t>();
 		ep.count = dcnt.as<int32_t>();
 		ep.status = dstat.as<int32_t>();
+		int64_t most = 0;
+		for (int32_t L : work) most = std::max<int64_t>(most, std::min(d.ls[size_t(L)], d.lt[size_t(L)]));
+		int64_t smem_most = pa::ENUM_SMEM_MAP;
+		if (const char *e = std::getenv("PA_ENUM_MAP")) smem_most = std::min<int64_t>(smem_most, std::atoll(e));  // tests
+		ep.smem_map = most <= smem_most ? int32_t(std::max<int64_t>(most, 1)) : 0;
 		PA_CUDA(pa::enum_solve(ep, nullptr));
 		PA_CUDA(cudaMemcpy(status.data(), dstat.p, size_t(B) * 4, cudaMemcpyDeviceToHost));
 		std::vector<int32_t> again;
