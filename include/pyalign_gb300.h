@@ -363,6 +363,15 @@ pa_status pa_path_embedding_gradients_full(int64_t batch, int32_t dim, int32_t n
                                            const float *inv_t, int64_t n_s, int64_t n_t, float *dEs, float *dEt,
                                            void *stream);
 
+/* pa_path_embedding_gradients_full from the float rows alone: the BF16 factors are Es[i] *
+ * inv_s[i] rounded.  dim a multiple of 4, at most 256; Es, Et, dEs, dEt 16-byte aligned; n_s
+ * and n_t together at most about 190,000 rows (PA_ERR_LENGTH). */
+pa_status pa_path_embedding_gradients_rows(int64_t batch, int32_t dim, int32_t normalize, const int32_t *paths,
+                                           const int64_t *path_offsets, const int32_t *path_len,
+                                           const float *grad_scores, const float *Es, const float *Et,
+                                           const float *inv_s, const float *inv_t, int64_t n_s, int64_t n_t,
+                                           float *dEs, float *dEt, void *stream);
+
 /* Fused backward of DTW on two series with d(u, v) = |x_u - y_v| (x: (batch, n_s),
  * y: (batch, n_t) float32): every visited cell adds grad * sign(x_u - y_v) to dx_u and
  * subtracts it from dy_v (per row and column: grad times the exact count of signs, adding to
@@ -387,6 +396,18 @@ pa_status pa_similarity_bf16(const void *Es, const void *Et, int64_t batch, int6
                              const int32_t *len_s, const int32_t *len_t, const int32_t *tile_start,
                              int64_t total_tiles, float *St, int64_t pitch_pair, int64_t pitch_row, float alpha,
                              float beta, int32_t *status, void *stream);
+
+/* pa_similarity_bf16 (alpha = 1, beta = 0) of the BF16 factors of pa_normalize_rows_bf16, from
+ * the float rows and without storing the factors: Es (batch, n_s, dim) and Et (batch, n_t, dim)
+ * float32, 16-byte aligned, dim a multiple of 4 and at most 256; inv_s (batch * n_s) and inv_t
+ * (batch * n_t) receive 1/|E| (1 when not normalising) of the rows inside the lengths of pairs
+ * with cells, the other entries are not written.  tile_start (batch + 1) holds the prefix sums
+ * of ceil(len_t / 256) * ceil(len_s / 128).  A wait that times out ORs 2 into *status.
+ * Allocates nothing; runs on `stream`. */
+pa_status pa_similarity_rows(const float *Es, const float *Et, int64_t batch, int64_t n_s, int64_t n_t, int32_t dim,
+                             int32_t normalize, const int32_t *len_s, const int32_t *len_t,
+                             const int32_t *tile_start, int64_t total_tiles, float *St, int64_t pitch_pair,
+                             int64_t pitch_row, float *inv_s, float *inv_t, int32_t *status, void *stream);
 
 /* Score of each pair's recovered path re-evaluated in FP64: the similarities of its aligned
  * cells (every visited cell for DTW) plus or minus its gap costs w(k) = open + extend (k - 1),

@@ -86,6 +86,10 @@ def _lib():
         L.pa_similarity_bf16.restype = i32
         f32 = ctypes.c_float
         L.pa_similarity_bf16.argtypes = [vp, vp, i64, i64, i64, i32, vp, vp, vp, i64, vp, i64, i64, f32, f32, vp, vp]
+        L.pa_similarity_rows.restype = i32
+        L.pa_similarity_rows.argtypes = [vp, vp, i64, i64, i64, i32, i32, vp, vp, vp, i64, vp, i64, i64, vp, vp, vp, vp]
+        L.pa_path_embedding_gradients_rows.restype = i32
+        L.pa_path_embedding_gradients_rows.argtypes = [i64, i32, i32, vp, vp, vp, vp, vp, vp, vp, vp, i64, i64, vp, vp, vp]
         L.pa_path_scores_f64.restype = i32
         L.pa_path_scores_f64.argtypes = [i32, i32, i32, i64, vp, vp, vp, vp, vp, i64, i64, vp, vp, vp, vp]
         L._pa_grad_bound = True
@@ -149,6 +153,35 @@ def _lengths(lengths, B):
     return ln
 
 
+def _tiles(lengths, B, n_s, n_t, tile_t, device):
+    """len_s, len_t and tile_start of a product in tiles of SIM_TILE rows of s and tile_t rows of
+    t, on the device without a host wait for the queued work, and the number of tiles."""
+    ln = _lengths(lengths, B)
+    if (ln[0] > n_s).any() or (ln[1] > n_t).any() or (ln < 0).any():
+        raise ValueError("lengths exceed the embeddings")
+    tiles = ((ln[1].astype(np.int64) + tile_t - 1) // tile_t) * ((ln[0].astype(np.int64) + SIM_TILE - 1) // SIM_TILE)
+    meta = np.zeros(3 * B + 1, np.int32)
+    meta[:B] = ln[0]
+    meta[B:2 * B] = ln[1]
+    meta[2 * B + 1:] = np.cumsum(tiles)
+    return _to_device(meta, device), int(meta[-1])
+
+
+def _similarity_rows(Es, Et, lengths, normalize, out):
+    """S^T of <en_s, en_t> into out (batch, n_t, n_s) from float rows of a width that is a
+    multiple of 4 up to ROWS_DIM (pa_similarity_rows), and 1 / |E| of the rows."""
+    B, n_s, dim = Es.shape
+    n_t = Et.shape[1]
+    dmeta, total = _tiles(lengths, B, n_s, n_t, ROWS_TILE, Es.device)
+    inv_s = torch.empty(B * n_s, dtype=torch.float32, device=Es.device)
+    inv_t = torch.empty(B * n_t, dtype=torch.float32, device=Es.device)
+    _alg.check(_lib().pa_similarity_rows(
+        Es.data_ptr(), Et.data_ptr(), B, n_s, n_t, dim, int(normalize), dmeta.data_ptr(), dmeta.data_ptr() + 4 * B,
+        dmeta.data_ptr() + 8 * B, total, out.data_ptr(), out.stride(0), out.stride(1), inv_s.data_ptr(),
+        inv_t.data_ptr(), _status(Es.device).data_ptr(), torch.cuda.current_stream().cuda_stream))
+    return inv_s, inv_t
+
+
 def similarity_bf16(Esb, Etb, lengths, out=None, alpha=1.0, beta=0.0):
     """S = beta + alpha <Es[i], Et[j]> per pair from BF16 factors (batch, n, dim), on the
     tensor cores (pa_similarity_bf16), FP32 accumulation (alpha = -1, beta = 1 gives the
@@ -162,16 +195,7 @@ def similarity_bf16(Esb, Etb, lengths, out=None, alpha=1.0, beta=0.0):
         raise ValueError("Es, Et must be contiguous BF16 (batch, n, dim) tensors of one batch and dim")
     if dim % 16:
         raise ValueError("dim must be a multiple of 16")
-    ln = _lengths(lengths, B)
-    if (ln[0] > n_s).any() or (ln[1] > n_t).any() or (ln < 0).any():
-        raise ValueError("lengths exceed the embeddings")
-    tiles = ((ln[1].astype(np.int64) + 127) // 128) * ((ln[0].astype(np.int64) + 127) // 128)
-    meta = np.zeros(3 * B + 1, np.int32)
-    meta[:B] = ln[0]
-    meta[B:2 * B] = ln[1]
-    meta[2 * B + 1:] = np.cumsum(tiles)
-    total = int(meta[-1])
-    dmeta = _to_device(meta, Esb.device)  # no host wait for the queued work
+    dmeta, total = _tiles(lengths, B, n_s, n_t, SIM_TILE, Esb.device)
     if out is None:
         out = torch.empty((B, n_t, n_s), dtype=torch.float32, device=Esb.device)
     elif out.shape != (B, n_t, n_s) or out.dtype != torch.float32 or out.stride(2) != 1 or not out.is_cuda:
@@ -347,6 +371,9 @@ def alignment_score(S, lengths, gap_open=None, gap_extend=None, locality="global
 
 
 SIM_TILE = 128  # rows of a tile of the tensor-core product (pa_simgemm.cu TM, TN)
+ROWS_TILE = 256  # rows of t of a tile of the product from float rows, and its largest width (FB, FDIM)
+ROWS_DIM = 256
+ROWS_MARKS = 190000  # rows of s and t whose marks fit the backward's shared memory
 
 
 def normalized_bf16(E, normalize=True, lengths=None, tiled=False):
@@ -433,18 +460,27 @@ class EmbeddingAlignmentScore(torch.autograd.Function):
     @staticmethod
     def forward(ctx, Es, Et, lengths, gap_open, gap_extend, locality, direction, linear, normalize):
         dim_in = Es.shape[-1]
-        Es = _pad16(Es.contiguous().float())
-        Et = _pad16(Et.contiguous().float())
-        ln = np.asarray(lengths).reshape(Es.shape[0], 2)
-        # rows past a pair's length: zero up to the product's tile, not read, not written beyond
-        Esb, inv_s = normalized_bf16(Es, normalize, ln[:, 0], tiled=True)
-        Etb, inv_t = normalized_bf16(Et, normalize, ln[:, 1], tiled=True)
+        Es, Et = Es.contiguous().float(), Et.contiguous().float()
+        # the product straight from the float rows where their width allows it; else through stored
+        # BF16 factors, of widths padded to the tensor cores' K step
+        rows = dim_in % 4 == 0 and 0 < dim_in <= ROWS_DIM and Es.shape[1] + Et.shape[1] <= ROWS_MARKS \
+            and Et.shape[0] == Es.shape[0] and Et.shape[2] == dim_in and (Es.data_ptr() | Et.data_ptr()) % 16 == 0
+        Esb = Etb = None
+        if not rows:
+            Es, Et = _pad16(Es), _pad16(Et)
+            ln = np.asarray(lengths).reshape(Es.shape[0], 2)
+            # rows past a pair's length: zero up to the product's tile, not read, not written beyond
+            Esb, inv_s = normalized_bf16(Es, normalize, ln[:, 0], tiled=True)
+            Etb, inv_t = normalized_bf16(Et, normalize, ln[:, 1], tiled=True)
         # S^T = en_t en_s^T on the tensor cores, only the cells inside the lengths; its
         # transposed view is S with stride 1 along s; its columns are padded to whole 16-byte
         # words (rows no pair reaches) for the DP's loads
         B, n_s, n_t = Es.shape[0], Es.shape[1], Et.shape[1]
         St = torch.empty((B, n_t, (n_s + 3) // 4 * 4), dtype=torch.float32, device=Es.device)
-        similarity_bf16(Esb, Etb, lengths, out=St[:, :, :n_s])
+        if rows:
+            inv_s, inv_t = _similarity_rows(Es, Et, lengths, normalize, St)
+        else:
+            similarity_bf16(Esb, Etb, lengths, out=St[:, :, :n_s])
         S = St.transpose(1, 2)
         gap = (float(gap_open), None) if linear else (float(gap_open), float(gap_extend))
         scores, paths, plen, poff, _ = _forward_paths(S, lengths, gap, locality, direction, False)
@@ -463,10 +499,14 @@ class EmbeddingAlignmentScore(torch.autograd.Function):
         d_in = ctx.dim_in
         dEs = torch.empty_like(Es)  # every row is written: the aligned ones, zeros elsewhere
         dEt = torch.empty_like(Et)
-        _alg.check(_lib().pa_path_embedding_gradients_full(
-            B, dim, int(normalize), paths.data_ptr(), poff.data_ptr(), plen.data_ptr(), grad.data_ptr(),
-            Es.data_ptr(), Et.data_ptr(), Esb.data_ptr(), Etb.data_ptr(), inv_s.data_ptr(), inv_t.data_ptr(),
-            n_s, n_t, dEs.data_ptr(), dEt.data_ptr(), torch.cuda.current_stream().cuda_stream))
+        walk = (B, dim, int(normalize), paths.data_ptr(), poff.data_ptr(), plen.data_ptr(), grad.data_ptr(),
+                Es.data_ptr(), Et.data_ptr())
+        out = (inv_s.data_ptr(), inv_t.data_ptr(), n_s, n_t, dEs.data_ptr(), dEt.data_ptr(),
+               torch.cuda.current_stream().cuda_stream)
+        if Esb is None:
+            _alg.check(_lib().pa_path_embedding_gradients_rows(*walk, *out))
+        else:
+            _alg.check(_lib().pa_path_embedding_gradients_full(*walk, Esb.data_ptr(), Etb.data_ptr(), *out))
         d_open, d_ext = _gap_grads(False, linear, locality, direction, B, paths, plen, poff, grad)
         return dEs[..., :d_in], dEt[..., :d_in], None, d_open, d_ext, None, None, None, None
 

@@ -134,24 +134,27 @@ __device__ __forceinline__ void stage(unsigned char *dst, const __nv_bfloat16 *X
 	}
 }
 
-// The pair of tile t -- the last k with tile_start[k] <= t -- and the tile's origin, by a
-// 32-way search of the whole warp (every lane probes one candidate per round, a ballot
-// picks the bracket): 3 rounds of dependent loads for 8192 pairs instead of 13 for a
-// binary search, which otherwise dominates the time per tile.  Call with all 32 lanes.
-__device__ __forceinline__ void tile_of(const SimParams &p, int64_t t, int64_t &k, int64_t &m0, int64_t &n0,
-                                        int64_t &ls, int64_t &lt) {
+// The pair of tile t -- the last k with tile_start[k] <= t -- by a 32-way search of the whole
+// warp (every lane probes one candidate per round, a ballot picks the bracket): 3 rounds of
+// dependent loads for 8192 pairs instead of 13 for a binary search, which otherwise dominates
+// the time per tile.  Call with all 32 lanes.
+__device__ __forceinline__ int64_t pair_of(const int32_t *tile_start, int64_t batch, int64_t t) {
 	const int lane = threadIdx.x & 31;
-	int64_t lo = 0, hi = p.batch - 1;  // tile_start[lo] <= t always holds (tile_start[0] = 0)
+	int64_t lo = 0, hi = batch - 1;  // tile_start[lo] <= t always holds (tile_start[0] = 0)
 	while (lo < hi) {
-		const int64_t step = (hi - lo + 32) / 32;  // ceil((hi - lo + 1) / 32)
-		const int64_t idx = lo + int64_t(lane) * step;
-		const bool le = idx <= hi && p.tile_start[idx] <= t;
-		const uint32_t m = __ballot_sync(0xffffffffu, le);
-		const int top = 31 - __clz(m);  // lane 0 always qualifies
-		lo = lo + int64_t(top) * step;
+		const int64_t step = (hi - lo + 32) / 32, idx = lo + int64_t(lane) * step;
+		const uint32_t m = __ballot_sync(0xffffffffu, idx <= hi && tile_start[idx] <= t);
+		// lane 0 always qualifies
+		lo = lo + int64_t(31 - __clz(int(m))) * step;
 		hi = min(hi, lo + step - 1);
 	}
-	k = lo;
+	return lo;
+}
+
+// and the tile's origin
+__device__ __forceinline__ void tile_of(const SimParams &p, int64_t t, int64_t &k, int64_t &m0, int64_t &n0,
+                                        int64_t &ls, int64_t &lt) {
+	k = pair_of(p.tile_start, p.batch, t);
 	ls = p.len_s[k];
 	lt = p.len_t[k];
 	const int64_t tiles_n = (ls + TN - 1) / TN;
@@ -468,6 +471,290 @@ __global__ void __launch_bounds__(PTHREADS, 1)
 	}
 }
 
+// ---------------------------------------------------------------------------------------
+// The product of float rows, normalised on the way: S^T of <en_s, en_t>, en = E / |E| or E,
+// straight from the float embeddings (widths that are a multiple of 4 up to FDIM).  Written in
+// two passes, BF16 factors are stored and read again: at 8,192 pairs of 32..512 rows of 256 that
+// is 5.6 of 12.5 GB; both kernels of that were at 65 % of the copy rate.  Here
+//   warps 0-15  (loaders) take 8 rows each of a 128-row operand tile into registers -- 8 rows'
+//               loads in flight per warp -- sum the squares as the normalising kernel of the two
+//               passes does (the same factors bit for bit), and store the BF16 factors into
+//               shared memory as the 128-byte-swizzled K-major operand that TMA would write;
+//   warp 0      also issues the MMAs of a tile, M = 128 rows of s, N = up to 256 rows of t (a
+//               warp of its own for that would leave the loaders 80 registers a thread, too few
+//               for their rows);
+//   warps 16-19 drain the accumulator.  A lane is a row of s and a register a row of t, so a
+//               store instruction writes 128 contiguous bytes of a row of S^T as it stands.
+// A CTA walks a contiguous range of tiles, pair by pair, 256 rows of t (operand B, kept) against
+// all tiles of s (operand A): a pair of at most 256 rows of t is read from memory once, a longer
+// one again from L2.  A's single buffer is free again after the MMAs of its tile, about 1 us,
+// less than the loads of the next tile take, which are under way meanwhile.  Product and
+// normalisation of 8,192 pairs of 32..512 rows of 256: 1,648 + 1,174 us in two passes, 1,640 us
+// here (7.0 GB, 4.3 TB/s); 4,096 pairs of 64..256 rows of 128: 319 + 249 -> 241 us.  It is bound
+// by the loaders' instructions as much as by memory: without any loads 1,160 us.  Measured and not
+// taken: prefetching the next tile to L2 (1,717 us), half of a warp's rows reloaded while the other
+// half is converted (2,179; 2,297 with 8 warps of 16 rows).
+constexpr int FDIM = 256;
+constexpr int FLOADERS = 16;
+constexpr int FTHREADS = (FLOADERS + 4) * 32;
+constexpr int FB = 256;                      // rows of t of a tile: MMA N
+constexpr int FA_CHUNK = TM * PK * 2;        // 64 K elements of operand A: 16 KB
+constexpr int FB_CHUNK = FB * PK * 2;        // and of B: 32 KB
+
+struct FusedParams {
+	const float *Es, *Et;
+	int64_t n_s, n_t;
+	int32_t dim, normalize;
+	const int32_t *len_s, *len_t;
+	const int32_t *tile_start;  // batch + 1
+	int64_t batch, total_tiles;
+	float *St;
+	int64_t pitch_pair, pitch_row;
+	float *inv_s, *inv_t;       // 1 / |E| of the rows inside the lengths
+	int32_t *status;
+};
+
+// A CTA's tiles: b counts the 256-row tiles of t, m inside it the 128-row tiles of s.  The lengths
+// of the next pair are loaded a pair ahead.
+struct FusedWalk {
+	int64_t k, left;
+	int ls, lt, next_ls, next_lt, b, m;
+	__device__ __forceinline__ void ahead(const FusedParams &p) {
+		const bool any = k + 1 < p.batch;
+		next_ls = any ? p.len_s[k + 1] : 0;
+		next_lt = any ? p.len_t[k + 1] : 0;
+	}
+	__device__ __forceinline__ void begin(const FusedParams &p, int64_t t0, int64_t t1) {
+		left = t1 - t0;
+		if (left <= 0) return;
+		k = pair_of(p.tile_start, p.batch, t0);
+		ls = p.len_s[k];
+		lt = p.len_t[k];
+		const int in = int(t0 - p.tile_start[k]), ms = (ls + TM - 1) / TM;
+		b = in / ms;
+		m = in - b * ms;
+		ahead(p);
+	}
+	__device__ __forceinline__ bool valid() const { return left > 0; }
+	__device__ __forceinline__ int rows_t() const { return min(FB, lt - b * FB); }
+	__device__ __forceinline__ int rows_s() const { return min(TM, ls - m * TM); }
+	__device__ __forceinline__ void next(const FusedParams &p) {
+		if (--left <= 0) return;
+		if (++m * TM < ls) return;
+		m = 0;
+		if (++b * FB < lt) return;
+		b = 0;
+		do {
+			k++;
+			ls = next_ls;
+			lt = next_lt;
+			ahead(p);
+		} while (ls == 0 || lt == 0);
+	}
+};
+
+// NV: 16-byte words of a row per lane
+template <int NV>
+__global__ void __launch_bounds__(FTHREADS, 1) sim_fused_kernel(FusedParams p) {
+	extern __shared__ __align__(1024) unsigned char smem_raw[];
+	const int chunks = (p.dim + PK - 1) / PK;
+	unsigned char *sA = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+	unsigned char *sB = sA + chunks * FA_CHUNK;
+	uint64_t *bars = reinterpret_cast<uint64_t *>(sB + chunks * FB_CHUNK);
+	uint32_t *tslot = reinterpret_cast<uint32_t *>(bars + 6);
+	const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+	const uint32_t bar0 = smem_addr(bars);
+	const uint32_t full = bar0, empty = bar0 + 8;  // both once per tile
+	auto ready = [&](int a) { return bar0 + 16u + 8u * a; };
+	auto freed = [&](int a) { return bar0 + 32u + 8u * a; };
+	if (threadIdx.x == 0) {
+		auto init = [](uint32_t bar, int count) {
+			asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
+		};
+		init(full, FLOADERS);
+		init(empty, 1);
+		for (int a = 0; a < 2; a++) {
+			init(ready(a), 1);
+			init(freed(a), 4);
+		}
+		asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+	}
+	if (warp == FLOADERS) {
+		asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(tslot)),
+		             "r"(2 * FB)
+		             : "memory");
+		asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+	}
+	asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+	__syncthreads();
+	asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+	const uint32_t tmem = *tslot;
+	const int64_t per = (p.total_tiles + gridDim.x - 1) / gridDim.x;
+	const int64_t t0 = min(int64_t(blockIdx.x) * per, p.total_tiles), t1 = min(t0 + per, p.total_tiles);
+	FusedWalk w;
+	w.begin(p, t0, t1);  // every warp, all lanes
+	uint32_t n = 0;      // tiles so far
+
+	if (warp < FLOADERS) {
+		constexpr int ROWS = TM / FLOADERS;
+		const int kdim = (p.dim + 15) & ~15;
+		bool waited = false;
+		// this lane's 8 bytes of row q of the warp's 8, in chunk 0 for j = 0: the 16-byte piece is
+		// swizzled by the row in its group of 8, which is q
+		const uint32_t put = ((uint32_t(lane) & 15u) >> 1 << 4) + ((uint32_t(lane) & 1u) << 3);
+		// rows 0 .. rows - 1 (128 at most) of X to rows d0.. of an operand in shared memory
+		auto fill = [&](const float *X, float *inv_out, int rows, unsigned char *dst, int d0, int chunk_bytes) {
+			const int w0 = warp * ROWS;
+			float4 v[ROWS][NV];
+			const float *x0 = X + int64_t(w0) * p.dim + 4 * lane;
+#pragma unroll
+			for (int q = 0; q < ROWS; q++)
+#pragma unroll
+				for (int j = 0; j < NV; j++)
+					v[q][j] = w0 + q < rows && 4 * lane + 128 * j < p.dim ? __ldg(reinterpret_cast<const float4 *>(x0 + q * p.dim + 128 * j))
+					                                                      : make_float4(0.f, 0.f, 0.f, 0.f);
+			float ss[ROWS];
+#pragma unroll
+			for (int q = 0; q < ROWS; q++) {
+				ss[q] = 0.0f;
+#pragma unroll
+				for (int j = 0; j < NV; j++) {
+					const float4 x = v[q][j];
+					ss[q] += x.x * x.x + x.y * x.y + x.z * x.z + x.w * x.w;
+				}
+			}
+			// the lanes' sums of 8 rows by halving: a lane keeps the rows its upper bits name and hands
+			// the others to its partner.  The pairs added are those of a butterfly over each row
+#pragma unroll
+			for (int h = ROWS / 2, o = 16; h > 0; h >>= 1, o >>= 1) {
+				const bool up = lane & o;
+#pragma unroll
+				for (int q = 0; q < h; q++) {
+					const float got = __shfl_xor_sync(0xffffffffu, up ? ss[q] : ss[q + h], o);
+					ss[q] = (up ? ss[q + h] : ss[q]) + got;
+				}
+			}
+			ss[0] += __shfl_xor_sync(0xffffffffu, ss[0], 2);
+			ss[0] += __shfl_xor_sync(0xffffffffu, ss[0], 1);
+			const float mine = p.normalize ? 1.0f / fmaxf(sqrtf(ss[0]), 1e-12f) : 1.0f;  // of row lane / 4
+			uint2 e[ROWS][NV];
+#pragma unroll
+			for (int q = 0; q < ROWS; q++) {
+				const float inv = __shfl_sync(0xffffffffu, mine, 4 * q);
+#pragma unroll
+				for (int j = 0; j < NV; j++) {
+					const float4 x = v[q][j];
+					const __nv_bfloat162 a = __floats2bfloat162_rn(x.x * inv, x.y * inv), b = __floats2bfloat162_rn(x.z * inv, x.w * inv);
+					e[q][j] = make_uint2(*reinterpret_cast<const uint32_t *>(&a), *reinterpret_cast<const uint32_t *>(&b));
+				}
+			}
+			if (!waited) {  // the MMAs of the tile before have read both operands
+				waited = true;
+				if (n > 0 && !mbar_wait(empty, (n - 1) & 1u)) return false;
+			}
+			if ((lane & 3) == 0 && w0 + (lane >> 2) < rows) inv_out[w0 + (lane >> 2)] = mine;
+			unsigned char *base = dst + (lane >> 4) * chunk_bytes + (d0 + w0) * 128;
+#pragma unroll
+			for (int q = 0; q < ROWS; q++) {
+				if (w0 + q >= rows) break;
+#pragma unroll
+				for (int j = 0; j < NV; j++)
+					if (4 * lane + 128 * j < kdim)
+						*reinterpret_cast<uint2 *>(base + (put ^ (q << 4)) + q * 128 + 2 * j * chunk_bytes) = e[q][j];
+			}
+			return true;
+		};
+		auto issue = [&](int a, uint32_t cols) {
+			asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+			const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((cols >> 3) << 17) | (uint32_t(TM >> 4) << 24);
+			const int steps = kdim / 16;
+			for (int kk = 0; kk < steps; kk++) {
+				const uint64_t da = desc_sw128(smem_addr(sA) + (kk >> 2) * FA_CHUNK + (kk & 3) * 32);
+				const uint64_t db = desc_sw128(smem_addr(sB) + (kk >> 2) * FB_CHUNK + (kk & 3) * 32);
+				asm volatile(
+				    "{\n\t.reg .pred p;\n\t"
+				    "setp.ne.b32 p, %4, 0;\n\t"
+				    "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tmem + uint32_t(a * FB)),
+				    "l"(da), "l"(db), "r"(idesc), "r"(kk > 0 ? 1u : 0u));
+			}
+			mma_commit(empty);
+			mma_commit(ready(a));
+		};
+		bool first = true;
+		for (; w.valid(); w.next(p), n++) {
+			bool ok = true;
+			waited = false;
+			if (first || w.m == 0) {  // operand B anew
+				const int rows = w.rows_t();
+				const int64_t r0 = w.k * p.n_t + int64_t(w.b) * FB;
+				for (int h = 0; h < rows && ok; h += TM)
+					ok = fill(p.Et + (r0 + h) * p.dim, p.inv_t + r0 + h, min(TM, rows - h), sB, h, FB_CHUNK);
+				first = false;
+			}
+			const int64_t r0 = w.k * p.n_s + int64_t(w.m) * TM;
+			ok = ok && fill(p.Es + r0 * p.dim, p.inv_s + r0, w.rows_s(), sA, 0, FA_CHUNK);
+			asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+			if (!__all_sync(0xffffffffu, ok)) {
+				if (lane == 0) atomicOr(p.status, ST_TIMEOUT);
+				break;
+			}
+			__syncwarp();
+			if (lane == 0) {
+				asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(full) : "memory");
+				if (warp == 0) {
+					const int a = int(n & 1u);
+					ok = mbar_wait(full, n & 1u) && mbar_wait(freed(a), ((n >> 1) & 1u) ^ 1u);
+					if (!ok) atomicOr(p.status, ST_TIMEOUT);
+					else issue(a, uint32_t(w.rows_t() + 15) & ~15u);
+				}
+			}
+			if (!__shfl_sync(0xffffffffu, ok, 0)) break;
+		}
+	} else {
+		const int rq = warp & 3;  // TMEM lanes 32 rq .. + 31
+		for (; w.valid(); w.next(p), n++) {
+			const int a = int(n & 1u);
+			if (!__all_sync(0xffffffffu, mbar_wait(ready(a), (n >> 1) & 1u))) {
+				if (lane == 0) atomicOr(p.status, ST_TIMEOUT);
+				break;
+			}
+			asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+			const int s = w.m * TM + rq * 32 + lane, cols = w.rows_t();
+			if (s - lane < w.ls) {
+				char *out = reinterpret_cast<char *>(p.St + w.k * p.pitch_pair + int64_t(w.b) * FB * p.pitch_row + s);
+				const int64_t pitch = p.pitch_row * 4;
+				for (int cc = 0; cc < cols; cc += 32) {
+					uint32_t v[32];
+					tmem_ld32(tmem + (uint32_t(rq * 32) << 16) + uint32_t(a * FB + cc), v);
+					if (s < w.ls) {
+						if (cc + 32 <= cols) {
+#pragma unroll
+							for (int q = 0; q < 32; q++) {
+								*reinterpret_cast<float *>(out) = __fadd_rn(__uint_as_float(v[q]), 0.0f);
+								out += pitch;
+							}
+						} else {
+#pragma unroll
+							for (int q = 0; q < 32; q++) {
+								if (cc + q < cols) *reinterpret_cast<float *>(out) = __fadd_rn(__uint_as_float(v[q]), 0.0f);
+								out += pitch;
+							}
+						}
+					}
+				}
+			}
+			asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+			__syncwarp();
+			if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(freed(a)) : "memory");
+		}
+	}
+	__syncthreads();
+	if (warp == FLOADERS) {
+		asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+		asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * FB) : "memory");
+	}
+}
+
 // cuTensorMapEncodeTiled through the runtime's driver entry point (no link against libcuda).
 typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
                                   const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
@@ -559,5 +846,37 @@ extern "C" pa_status pa_similarity_bf16(const void *Es, const void *Et, int64_t 
 	}
 	const int64_t grid = total_tiles < int64_t(3) * sms ? total_tiles : int64_t(3) * sms;
 	sim_bf16_kernel<<<int(grid), THREADS, SMEM_BYTES, static_cast<cudaStream_t>(stream)>>>(p);
+	return cudaGetLastError() == cudaSuccess ? PA_OK : PA_ERR_CUDA;
+}
+
+extern "C" pa_status pa_similarity_rows(const float *Es, const float *Et, int64_t batch, int64_t n_s, int64_t n_t,
+                                        int32_t dim, int32_t normalize, const int32_t *len_s, const int32_t *len_t,
+                                        const int32_t *tile_start, int64_t total_tiles, float *St,
+                                        int64_t pitch_pair, int64_t pitch_row, float *inv_s, float *inv_t,
+                                        int32_t *status, void *stream) {
+	if (batch < 0 || n_s < 0 || n_t < 0 || total_tiles < 0) return PA_ERR_INVALID_ARGUMENT;
+	if (batch == 0 || total_tiles == 0) return PA_OK;
+	if (!Es || !Et || !len_s || !len_t || !tile_start || !St || !inv_s || !inv_t || !status) return PA_ERR_INVALID_ARGUMENT;
+	if (dim <= 0 || dim % 4 != 0 || dim > FDIM) return PA_ERR_INVALID_ARGUMENT;
+	if ((reinterpret_cast<uintptr_t>(Es) | reinterpret_cast<uintptr_t>(Et)) & 15) return PA_ERR_INVALID_ARGUMENT;
+	int dev = 0, sms = 0;
+	if (cudaGetDevice(&dev) != cudaSuccess) return PA_ERR_NO_DEVICE;
+	if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return PA_ERR_CUDA;
+	FusedParams p{Es, Et, n_s, n_t, dim, normalize, len_s, len_t, tile_start, batch, total_tiles, St, pitch_pair, pitch_row,
+	              inv_s, inv_t, status};
+	const int chunks = (dim + PK - 1) / PK;
+	const int bytes = chunks * (FA_CHUNK + FB_CHUNK) + 128 + 1024;
+	constexpr int most = FDIM / PK * (FA_CHUNK + FB_CHUNK) + 128 + 1024;
+	const int grid = int(total_tiles < int64_t(sms) ? total_tiles : int64_t(sms));
+	cudaStream_t st = static_cast<cudaStream_t>(stream);
+	if (dim <= 128) {
+		if (cudaFuncSetAttribute(sim_fused_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, most) != cudaSuccess)
+			return PA_ERR_CUDA;
+		sim_fused_kernel<1><<<grid, FTHREADS, bytes, st>>>(p);
+	} else {
+		if (cudaFuncSetAttribute(sim_fused_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, most) != cudaSuccess)
+			return PA_ERR_CUDA;
+		sim_fused_kernel<2><<<grid, FTHREADS, bytes, st>>>(p);
+	}
 	return cudaGetLastError() == cudaSuccess ? PA_OK : PA_ERR_CUDA;
 }
