@@ -123,8 +123,48 @@ __global__ void __launch_bounds__(WALK_WARPS * 32) walk_kernel(WalkParams p) {
 			j -= dj * first_out;
 		}
 	};
+	// Step by step, for gaps without an open bit: the look at a run costs some 100 instructions
+	// whatever it finds, a single step 20, so where fewer than 7 of 8 steps are diagonal (a look
+	// found fewer than 8, or the last steps were mixed) up to 32 steps inside the window are taken
+	// one at a time by every lane alike; lane c keeps point c, and the points leave together.
+	// Steps on DTW paths rarely repeat: 4,096 pairs of 128..1024 points, 545 us by looks, 246 so.
+	bool single = false;
+	const int ushift = fmt16 ? 2 : 0;
 	while (u >= 0 && v >= 0) {
 		if (!inwin(u, v)) place(u, v);
+		if (single) {
+			const int ulo = max(0, 8 * (ub - (WIN_BLOCKS - 1))), vlo = max(0, vb - 31);
+			int cnt = 0, pu = 0, pv = 0;
+			bool pd = false, end = false;
+			do {
+				const uint32_t w = win[ub - (u >> 3)][vb - v];
+				const uint32_t c = (w >> (4 * (R - 1 - (u & (R - 1))) + ushift)) & 3u;
+				end = p.local && c == 3u;
+				if (end) break;
+				u -= int((c + 1u) >> 1) & 1;  // codes 1 (up) and 2 (diagonal)
+				v -= c != 1u;
+				if (lane == cnt) {
+					pu = u;
+					pv = v;
+					pd = c == 2u;
+				}
+				cnt++;
+			} while (cnt < 32 && u >= ulo && v >= vlo);
+			if (lane < cnt) {
+				if (map && pd) {  // from (pu + 1, pv + 1)
+					if (s2t) map[pu + 1] = pv + 1;
+					else map[pv + 1] = pu + 1;
+				}
+				if (path) {
+					path[2 * (np + lane)] = pu;
+					path[2 * (np + lane) + 1] = pv;
+				}
+			}
+			np += cnt;
+			if (end) break;
+			single = 8 * __popc(__ballot_sync(0xffffffffu, pd && lane < cnt)) < 7 * cnt;
+			continue;
+		}
 		// a run of diagonal steps: lane k looks at (u - k, v - k), one ballot finds how many
 		// consecutive cells from (u, v) have the diagonal code
 		const int iu = u - lane, iv = v - lane;
@@ -132,6 +172,7 @@ __global__ void __launch_bounds__(WALK_WARPS * 32) walk_kernel(WalkParams p) {
 		const uint32_t n = nib_at(iu, iv, ok);
 		const uint32_t bal = __ballot_sync(0xffffffffu, ok && (n & 3u) == 2u);
 		const int run = first_clear(bal);
+		single = !affine && run < 8;
 		if (run > 0) {
 			if (lane < run) {
 				if (map) {
