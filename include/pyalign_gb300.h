@@ -322,6 +322,17 @@ pa_status pa_path_gradients(int32_t type, int32_t locality, int32_t direction, i
                             const float *grad_scores, float *dS, const int64_t *ds_offsets, int64_t stride_s,
                             int64_t stride_t, float *dgap, void *stream);
 
+/* What the calls on per-pair lengths need of them, in one pass on the host.  lengths: (batch, 2)
+ * of |s|, |t|, int32 or (wide) int64; len (2, batch): the same pair-minor; tile_start (batch + 1): prefix sums of
+ * ceil(|s| / tile_s) * ceil(|t| / tile_t); path_offsets (batch): the packed start of each pair's
+ * path of 2 (|s| + |t| + 2) entries; totals[2]: all tiles, all path entries.  PA_ERR_LENGTH when
+ * a length is negative or above n_s, n_t.  Host memory. */
+pa_status pa_pair_plan(const void *lengths, int32_t wide, int64_t batch, int64_t n_s, int64_t n_t, int32_t tile_s,
+                       int32_t tile_t, int32_t *len, int32_t *tile_start, int64_t *path_offsets, int64_t *totals);
+
+/* A 64-bit hash of a host array, for tables keyed by content (equal hashes are not a proof). */
+uint64_t pa_content_hash(const void *data, int64_t bytes);
+
 /* Embedding similarity S(i, j) = <en_s[i], en_t[j]> with en = E / |E| (normalize != 0,
  * cosine) or en = E (dot).  pa_normalize_rows_bf16 writes the BF16 factor en (rows x dim)
  * and 1/|E| per row (1 when not normalising) in one pass over E (rows x dim float32).

@@ -13,6 +13,7 @@ the reference's optimal path.
 """
 
 import ctypes
+import functools
 import types
 
 import numpy as np
@@ -90,6 +91,10 @@ def _lib():
         L.pa_similarity_rows.argtypes = [vp, vp, i64, i64, i64, i32, i32, vp, vp, vp, i64, vp, i64, i64, vp, vp, vp, vp]
         L.pa_path_embedding_gradients_rows.restype = i32
         L.pa_path_embedding_gradients_rows.argtypes = [i64, i32, i32, vp, vp, vp, vp, vp, vp, vp, vp, i64, i64, vp, vp, vp]
+        L.pa_pair_plan.restype = i32
+        L.pa_pair_plan.argtypes = [vp, i32, i64, i64, i64, i32, i32, vp, vp, vp, vp]
+        L.pa_content_hash.restype = ctypes.c_uint64
+        L.pa_content_hash.argtypes = [vp, i64]
         L.pa_path_scores_f64.restype = i32
         L.pa_path_scores_f64.argtypes = [i32, i32, i32, i64, vp, vp, vp, vp, vp, i64, i64, vp, vp, vp, vp]
         L._pa_grad_bound = True
@@ -116,20 +121,20 @@ def tensor_core_status(device=None):
     return v
 
 
-_small_cache = {}   # (device, dtype, bytes) -> device tensor: index arrays seen before
+_small_cache = {}   # (device, dtype, shape, content hash) -> (host copy, device tensor): index arrays seen before
 _staging = {}       # (device, dtype) -> (pinned buffer, event of its last copy)
 
 
 def _to_device(arr, device):
     """A small host index array (lengths, offsets) on the device without blocking the host: a
-    content-keyed cache (a training loop passes the same lengths every step) and, for new
-    contents, a non-blocking copy out of a reused pinned buffer."""
+    content-keyed cache (a training loop passes the same lengths every step; equal hashes are
+    compared in full) and, for new contents, a non-blocking copy out of a reused pinned buffer."""
     arr = np.ascontiguousarray(arr)
     device = torch.device(device)
-    key = (str(device), arr.dtype.str, arr.shape, arr.tobytes())
+    key = (str(device), arr.dtype.str, arr.shape, _lib().pa_content_hash(arr.ctypes.data, arr.nbytes))
     hit = _small_cache.get(key)
-    if hit is not None:
-        return hit
+    if hit is not None and np.array_equal(hit[0], arr):
+        return hit[1]
     dtype = torch.from_numpy(arr[:0]).dtype
     buf, ev = _staging.get((str(device), arr.dtype.str), (None, None))
     if buf is None or buf.numel() < arr.size:
@@ -142,42 +147,45 @@ def _to_device(arr, device):
     ev = torch.cuda.Event()
     ev.record(torch.cuda.current_stream(device))
     _staging[(str(device), arr.dtype.str)] = (buf, ev)
-    if len(_small_cache) >= 32:
+    if key not in _small_cache and len(_small_cache) >= 32:
         _small_cache.pop(next(iter(_small_cache)))
-    _small_cache[key] = out
+    _small_cache[key] = (arr.copy(), out)
     return out
 
 
-def _lengths(lengths, B):
-    ln = np.ascontiguousarray(np.asarray(lengths).reshape(B, 2).T, dtype=np.int32)
-    return ln
+class _Plan:
+    """The lengths of a batch of pairs as the calls below take them (pa_pair_plan, one pass on the
+    host): ln (2, B) int32, meta = ln and the tile prefix of a product in tiles of SIM_TILE rows of
+    s and tile_t rows of t, the packed path offsets, and the totals."""
+
+    def __init__(self, lengths, B, n_s, n_t, what, tile_t=128):
+        raw = np.asarray(lengths).reshape(B, 2)
+        wide = raw.dtype == np.int64
+        if not wide or not raw.flags.c_contiguous:
+            raw, wide = np.ascontiguousarray(raw, dtype=np.int32), False
+        self.meta = np.empty(3 * B + 1, np.int32)
+        self.poff = np.empty(B, np.int64)
+        self.ln = self.meta[:2 * B].reshape(2, B)
+        tot = np.empty(2, np.int64)
+        m = self.meta.ctypes.data
+        if _lib().pa_pair_plan(raw.ctypes.data, int(wide), B, n_s, n_t, SIM_TILE, tile_t, m, m + 8 * B, self.poff.ctypes.data,
+                               tot.ctypes.data):
+            raise ValueError("lengths exceed " + what)
+        self.tiles, self.entries = int(tot[0]), int(tot[1])
 
 
-def _tiles(lengths, B, n_s, n_t, tile_t, device):
-    """len_s, len_t and tile_start of a product in tiles of SIM_TILE rows of s and tile_t rows of
-    t, on the device without a host wait for the queued work, and the number of tiles."""
-    ln = _lengths(lengths, B)
-    if (ln[0] > n_s).any() or (ln[1] > n_t).any() or (ln < 0).any():
-        raise ValueError("lengths exceed the embeddings")
-    tiles = ((ln[1].astype(np.int64) + tile_t - 1) // tile_t) * ((ln[0].astype(np.int64) + SIM_TILE - 1) // SIM_TILE)
-    meta = np.zeros(3 * B + 1, np.int32)
-    meta[:B] = ln[0]
-    meta[B:2 * B] = ln[1]
-    meta[2 * B + 1:] = np.cumsum(tiles)
-    return _to_device(meta, device), int(meta[-1])
-
-
-def _similarity_rows(Es, Et, lengths, normalize, out):
+def _similarity_rows(Es, Et, lengths, normalize, out, plan=None):
     """S^T of <en_s, en_t> into out (batch, n_t, n_s) from float rows of a width that is a
     multiple of 4 up to ROWS_DIM (pa_similarity_rows), and 1 / |E| of the rows."""
     B, n_s, dim = Es.shape
     n_t = Et.shape[1]
-    dmeta, total = _tiles(lengths, B, n_s, n_t, ROWS_TILE, Es.device)
+    plan = plan or _Plan(lengths, B, n_s, n_t, "the embeddings", ROWS_TILE)
+    dmeta = _to_device(plan.meta, Es.device)
     inv_s = torch.empty(B * n_s, dtype=torch.float32, device=Es.device)
     inv_t = torch.empty(B * n_t, dtype=torch.float32, device=Es.device)
     _alg.check(_lib().pa_similarity_rows(
         Es.data_ptr(), Et.data_ptr(), B, n_s, n_t, dim, int(normalize), dmeta.data_ptr(), dmeta.data_ptr() + 4 * B,
-        dmeta.data_ptr() + 8 * B, total, out.data_ptr(), out.stride(0), out.stride(1), inv_s.data_ptr(),
+        dmeta.data_ptr() + 8 * B, plan.tiles, out.data_ptr(), out.stride(0), out.stride(1), inv_s.data_ptr(),
         inv_t.data_ptr(), _status(Es.device).data_ptr(), torch.cuda.current_stream().cuda_stream))
     return inv_s, inv_t
 
@@ -195,7 +203,8 @@ def similarity_bf16(Esb, Etb, lengths, out=None, alpha=1.0, beta=0.0):
         raise ValueError("Es, Et must be contiguous BF16 (batch, n, dim) tensors of one batch and dim")
     if dim % 16:
         raise ValueError("dim must be a multiple of 16")
-    dmeta, total = _tiles(lengths, B, n_s, n_t, SIM_TILE, Esb.device)
+    plan = _Plan(lengths, B, n_s, n_t, "the embeddings")
+    dmeta, total = _to_device(plan.meta, Esb.device), plan.tiles  # no host wait for the queued work
     if out is None:
         out = torch.empty((B, n_t, n_s), dtype=torch.float32, device=Esb.device)
     elif out.shape != (B, n_t, n_s) or out.dtype != torch.float32 or out.stride(2) != 1 or not out.is_cuda:
@@ -245,9 +254,17 @@ def path_scores_f64(S, lengths, gap_open=None, gap_extend=None, locality="global
     return (scores, out, scale) if with_scale else (scores, out)
 
 
-def _forward_paths(S, lengths, gap, locality, direction, dtw):
+@functools.lru_cache(maxsize=32)
+def _pair_offsets(B, first, stride):
+    """Where the pairs' matrices begin (elements), as the host array a dense solve takes."""
+    off = first + np.arange(B, dtype=np.int64) * stride
+    off.flags.writeable = False
+    return off
+
+
+def _forward_paths(S, lengths, gap, locality, direction, dtw, plan=None):
     """Scores and optimal paths of the pairs of S (device); returns (scores, paths, path
-    lengths, device path offsets, layout flag)."""
+    lengths, device path offsets, layout flag).  plan: the _Plan of the lengths if there is one."""
     if not S.is_cuda or S.dtype != torch.float32 or S.dim() != 3:
         raise ValueError("S must be a (batch, len_s, len_t) float32 CUDA tensor")
     # any layout with unit stride along s or t is read in place; a transposed view
@@ -256,9 +273,9 @@ def _forward_paths(S, lengths, gap, locality, direction, dtw):
         S = S.contiguous()
     B, n_s, n_t = S.shape
     ss, st_ = S.stride(1), S.stride(2)
-    solver, ln, scores, paths, plen, poff = _path_buffers(B, n_s, n_t, lengths, locality, direction, dtw, gap,
-                                                          S.device, "the similarity tensor")
-    offsets = S.storage_offset() + np.arange(B, dtype=np.int64) * S.stride(0)
+    plan = plan or _Plan(lengths, B, n_s, n_t, "the similarity tensor")
+    solver, ln, scores, paths, plen, poff = _path_buffers(B, n_s, n_t, plan, locality, direction, dtw, gap, S.device)
+    offsets = _pair_offsets(B, S.storage_offset(), S.stride(0))
     base = S.data_ptr() - S.storage_offset() * S.element_size()
     _alg.check(_lib().pa_solve_dense_paths(
         solver.handle, base, offsets.ctypes.data, ss, st_, B, n_s, n_t, ln.ctypes.data,
@@ -266,23 +283,17 @@ def _forward_paths(S, lengths, gap, locality, direction, dtw):
     return scores, paths, plen, _to_device(poff, S.device), ss == 1
 
 
-def _path_buffers(B, n_s, n_t, lengths, locality, direction, dtw, gap, device, what):
+def _path_buffers(B, n_s, n_t, plan, locality, direction, dtw, gap, device):
     """The solver on the current stream, the (2, B) int32 lengths and the output buffers of a
     paths solve: scores, packed paths (2 (|s| + |t| + 2) entries per pair), path lengths and
     the host path offsets."""
-    ln = np.ascontiguousarray(np.asarray(lengths).reshape(B, 2).T, dtype=np.int32)
-    if (ln[0] > n_s).any() or (ln[1] > n_t).any() or (ln < 0).any():
-        raise ValueError("lengths exceed " + what)
     solver = _solver(B, n_s, n_t, locality, direction, dtw, gap)
     stream = torch.cuda.current_stream()
     _alg.check(_lib().pa_solver_set_stream(solver.handle, ctypes.c_void_p(stream.cuda_stream)))
-    sizes = 2 * (ln[0].astype(np.int64) + ln[1] + 2)
-    poff = np.zeros(B, np.int64)
-    poff[1:] = np.cumsum(sizes)[:-1]
-    paths = torch.empty(int(sizes.sum()), dtype=torch.int32, device=device)
+    paths = torch.empty(plan.entries, dtype=torch.int32, device=device)
     plen = torch.zeros(B, dtype=torch.int32, device=device)
     scores = torch.empty(B, dtype=torch.float32, device=device)
-    return solver, ln, scores, paths, plen, poff
+    return solver, plan.ln, scores, paths, plen, plan.poff
 
 
 def _series_paths(x, y, lengths, gap, locality, direction, dtw):
@@ -290,18 +301,17 @@ def _series_paths(x, y, lengths, gap, locality, direction, dtw):
     float32 CUDA tensors): the kernel computes each cell, no matrix is formed."""
     B, n_s = x.shape
     n_t = y.shape[1]
-    solver, ln, scores, paths, plen, poff = _path_buffers(B, n_s, n_t, lengths, locality, direction, dtw, gap,
-                                                          x.device, "the series")
+    plan = _Plan(lengths, B, n_s, n_t, "the series")
+    solver, ln, scores, paths, plen, poff = _path_buffers(B, n_s, n_t, plan, locality, direction, dtw, gap, x.device)
     _alg.check(_lib().pa_solve_series_paths(
         solver.handle, x.data_ptr(), x.stride(0), y.data_ptr(), y.stride(0), B, n_s, n_t, ln.ctypes.data,
         scores.data_ptr(), paths.data_ptr(), poff.ctypes.data, plen.data_ptr()))
     return scores, paths, plen, _to_device(poff, x.device)
 
 
-def _gap_grads(dtw, linear, locality, direction, B, paths, plen, poff, grad):
-    """d score / d (open, extend) summed over pairs (pa_path_gradients without dS)."""
-    if dtw:
-        return None, None
+def _gap_grads(linear, locality, direction, B, paths, plen, poff, grad, device):
+    """d score / d (open, extend) summed over pairs (pa_path_gradients without dS), on the gap
+    costs' device (in one copy)."""
     A = _alg
     dgap = torch.empty((B, 4), dtype=torch.float32, device=grad.device)  # every pair writes its 4
     _alg.check(_lib().pa_path_gradients(
@@ -312,7 +322,7 @@ def _gap_grads(dtw, linear, locality, direction, B, paths, plen, poff, grad):
     # one reduction: (open_s + open_t, extend_s + extend_t) summed over pairs
     if linear:
         return dgap.sum(), None
-    tot = dgap.view(B, 2, 2).sum(dim=(0, 1))
+    tot = dgap.view(B, 2, 2).sum(dim=(0, 1)).to(device)
     return tot[0], tot[1]
 
 
@@ -324,13 +334,13 @@ class AlignmentScore(torch.autograd.Function):
         gap = None if dtw else ((float(gap_open), None) if linear else (float(gap_open), float(gap_extend)))
         scores, paths, plen, poff, transposed = _forward_paths(S, lengths, gap, locality, direction, dtw)
         ctx.save_for_backward(paths, plen, poff)
-        ctx.meta = (S.shape, locality, direction, dtw, linear, transposed)
+        ctx.meta = (S.shape, locality, direction, dtw, linear, transposed, gap_open.device)
         return scores
 
     @staticmethod
     def backward(ctx, grad):
         paths, plen, poff = ctx.saved_tensors
-        (B, n_s, n_t), locality, direction, dtw, linear, transposed = ctx.meta
+        (B, n_s, n_t), locality, direction, dtw, linear, transposed, gap_device = ctx.meta
         A = _alg
         grad = grad.contiguous().float()
         # dS in the layout S came in: a transposed view when S was one
@@ -338,17 +348,17 @@ class AlignmentScore(torch.autograd.Function):
             dS = torch.zeros((B, n_t, n_s), dtype=torch.float32, device=grad.device).transpose(1, 2)
         else:
             dS = torch.zeros((B, n_s, n_t), dtype=torch.float32, device=grad.device)
-        dgap = torch.zeros((B, 4), dtype=torch.float32, device=grad.device)
+        dgap = torch.empty((B, 4), dtype=torch.float32, device=grad.device)  # every pair writes its 4
         offsets = torch.arange(B, dtype=torch.int64, device=grad.device) * (n_s * n_t)
         _alg.check(_lib().pa_path_gradients(
             int(A.Type.DTW if dtw else A.Type.ALIGNMENT), int(A.Locality.__members__[locality.upper()]),
             int(A.Direction.__members__[direction.upper()]), B, paths.data_ptr(), poff.data_ptr(),
             plen.data_ptr(), grad.data_ptr(), dS.data_ptr(), offsets.data_ptr(), dS.stride(1), dS.stride(2),
             dgap.data_ptr(), torch.cuda.current_stream().cuda_stream))
-        tot = dgap.sum(dim=0)
-        if dtw:
-            d_open = d_ext = None
-        elif linear:
+        if dtw or not any(ctx.needs_input_grad[2:4]):
+            return dS, None, None, None, None, None, None, None
+        tot = dgap.sum(dim=0).to(gap_device)  # in one copy
+        if linear:
             d_open, d_ext = tot[0] + tot[1] + tot[2] + tot[3], None
         else:
             d_open, d_ext = tot[0] + tot[2], tot[1] + tot[3]
@@ -477,22 +487,24 @@ class EmbeddingAlignmentScore(torch.autograd.Function):
         # words (rows no pair reaches) for the DP's loads
         B, n_s, n_t = Es.shape[0], Es.shape[1], Et.shape[1]
         St = torch.empty((B, n_t, (n_s + 3) // 4 * 4), dtype=torch.float32, device=Es.device)
+        plan = None
         if rows:
-            inv_s, inv_t = _similarity_rows(Es, Et, lengths, normalize, St)
+            plan = _Plan(lengths, B, n_s, n_t, "the embeddings", ROWS_TILE)
+            inv_s, inv_t = _similarity_rows(Es, Et, lengths, normalize, St, plan)
         else:
             similarity_bf16(Esb, Etb, lengths, out=St[:, :, :n_s])
         S = St.transpose(1, 2)
         gap = (float(gap_open), None) if linear else (float(gap_open), float(gap_extend))
-        scores, paths, plen, poff, _ = _forward_paths(S, lengths, gap, locality, direction, False)
+        scores, paths, plen, poff, _ = _forward_paths(S, lengths, gap, locality, direction, False, plan)
         ctx.save_for_backward(Es, Et, Esb, Etb, inv_s, inv_t, paths, plen, poff)
-        ctx.meta = (locality, direction, linear, normalize)
+        ctx.meta = (locality, direction, linear, normalize, gap_open.device)
         ctx.dim_in = dim_in
         return scores
 
     @staticmethod
     def backward(ctx, grad):
         Es, Et, Esb, Etb, inv_s, inv_t, paths, plen, poff = ctx.saved_tensors
-        locality, direction, linear, normalize = ctx.meta
+        locality, direction, linear, normalize, gap_device = ctx.meta
         grad = grad.contiguous().float()
         B, n_s, dim = Es.shape
         n_t = Et.shape[1]
@@ -507,7 +519,9 @@ class EmbeddingAlignmentScore(torch.autograd.Function):
             _alg.check(_lib().pa_path_embedding_gradients_rows(*walk, *out))
         else:
             _alg.check(_lib().pa_path_embedding_gradients_full(*walk, Esb.data_ptr(), Etb.data_ptr(), *out))
-        d_open, d_ext = _gap_grads(False, linear, locality, direction, B, paths, plen, poff, grad)
+        d_open = d_ext = None
+        if any(ctx.needs_input_grad[3:5]):
+            d_open, d_ext = _gap_grads(linear, locality, direction, B, paths, plen, poff, grad, gap_device)
         return dEs[..., :d_in], dEt[..., :d_in], None, d_open, d_ext, None, None, None, None
 
 

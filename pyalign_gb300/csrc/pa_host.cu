@@ -722,20 +722,24 @@ int choose_G(const std::vector<int32_t> &ls, const std::vector<int32_t> &lt, int
 		if (g == 1 || g == 2 || g == 4 || g == 8 || g == 16 || g == 32) return g;
 	}
 	static const int cand[6] = {32, 16, 8, 4, 2, 1};  // 1: a lane per pair
+	const size_t B = ls.size();
+	const int32_t *a = ls.data(), *b = lt.data();
 	int64_t pairs = 0;
-	for (size_t k = 0; k < ls.size(); k++) pairs += (ls[k] > 0 && lt[k] > 0);
+	for (size_t k = 0; k < B; k++) pairs += int64_t(a[k] > 0) & int64_t(b[k] > 0);
 	double best = 0;
 	int bestG = 32;
 	for (int c = 0; c < 6; c++) {
 		const int G = cand[c];
-		const int64_t rpp = int64_t(G) * R;
-		double cells = 0;
-		for (size_t k = 0; k < ls.size(); k++) {
-			if (ls[k] == 0 || lt[k] == 0) continue;
-			const int64_t npass = (ls[k] + rpp - 1) / rpp;
-			cells += double(npass * rpp) * double(lt[k] + G - 1);
+		const uint32_t rpp = uint32_t(G) * R;  // a power of two
+		// in whole numbers, without a branch or a division a pair (this loop of 6 passes was most of
+		// a solve's host time: 4,096 pairs, all of it, 150 us with divisions)
+		int64_t sum = 0;
+		for (size_t k = 0; k < B; k++) {
+			const uint32_t rows = (uint32_t(a[k]) + rpp - 1) & ~(rpp - 1);
+			const uint32_t cols = b[k] > 0 ? uint32_t(b[k]) + uint32_t(G) - 1 : 0;
+			sum += int64_t(uint64_t(rows) * cols);
 		}
-		cells *= 1.0 + 0.06 * c;
+		const double cells = double(sum) * (1.0 + 0.06 * c);
 		// keep at least 4 warps per SM busy: narrower groups pack more pairs per warp (below
 		// that the launch is latency-bound; at 4096 pairs of 64 x 64 one 64-row stripe per
 		// pair, G = 8 with 7 warps per SM, beats G = 32 with 27 per SM, 3 of 4 lanes idle, 3x)
@@ -762,16 +766,22 @@ bool choose_units(const std::vector<int32_t> &ls, const std::vector<int32_t> &lt
 	}
 	if (std::getenv("PA_GROUP_WIDTH")) return false;  // a forced group width means group mode
 	const double slots = double(sm_count) * 16.0;
-	const int64_t rg = int64_t(G) * R, ru = 32 * R;
-	double work_g = 0, work_u = 0, chain_g = 0, chain_u = 0;
+	int lg = 0;  // rows of a stripe: 2^lg in a group of G (a power of two), 2^lu in one of 32
+	while ((1 << lg) < G * R) lg++;
+	constexpr int lu = 8;
+	static_assert(32 * R == 1 << lu, "stripe rows");
+	int64_t sum_g = 0, sum_u = 0, most_g = 0, most_u = 0;
 	for (size_t k = 0; k < ls.size(); k++) {
-		if (ls[k] == 0 || lt[k] == 0) continue;
-		const int64_t ng = (ls[k] + rg - 1) / rg, nu = (ls[k] + ru - 1) / ru;
-		work_g += double(ng) * double(lt[k] + G - 1) * double(G) / 32.0;
-		work_u += double(nu) * double(lt[k] + 31);
-		chain_g = std::max(chain_g, double(ng) * double(lt[k] + G - 1));
-		chain_u = std::max(chain_u, double(lt[k] + 31) + double(nu) * double(PUB_CHUNK + 32));
+		const int64_t a = ls[k], b = lt[k];
+		if (a == 0 || b == 0) continue;
+		const int64_t ng = (a + (int64_t(1) << lg) - 1) >> lg, nu = (a + (1 << lu) - 1) >> lu;
+		sum_g += ng * (b + G - 1);
+		sum_u += nu * (b + 31);
+		most_g = std::max(most_g, ng * (b + G - 1));
+		most_u = std::max(most_u, b + 31 + nu * (PUB_CHUNK + 32));
 	}
+	const double work_g = double(sum_g) * double(G) / 32.0, work_u = double(sum_u);
+	const double chain_g = double(most_g), chain_u = double(most_u);
 	const double tg = std::max(work_g / slots, chain_g), tu = std::max(work_u / slots, chain_u);
 	return tu < 0.8 * tg;
 }
@@ -2012,12 +2022,14 @@ pa_status solve_impl(pa_solver *s, const Input &in, int method, float *scores_ou
 		pair_g.assign(size_t(B), int8_t(plan.G));
 		if (!plan.seg) {
 			{
-				const int64_t rpp = int64_t(plan.G) * plan_rows(plan);
+				const int64_t rpp = int64_t(plan.G) * plan_rows(plan);  // a power of two
+				int lr = 0;
+				while ((int64_t(1) << lr) < rpp) lr++;
 				const int64_t kt = max_lt + 1;
 				const int64_t nkeys = ((max_ls + rpp - 1) / rpp + 1) * kt;
 				std::vector<int32_t> count(size_t(nkeys) + 1);
 				auto key = [&](int64_t k) {
-					const int64_t np = (ls[size_t(k)] + rpp - 1) / rpp;
+					const int64_t np = (ls[size_t(k)] + rpp - 1) >> lr;
 					return nkeys - 1 - (np * kt + lt[size_t(k)]);  // descending
 				};
 				for (int c = 0; c < plan.nchunks; c++) {
@@ -2108,11 +2120,16 @@ pa_status solve_impl(pa_solver *s, const Input &in, int method, float *scores_ou
 		dense_off.assign(size_t(B), 0);
 		copy_off.assign(plan.copy_pitch ? size_t(B) : 0, 0);
 		int64_t copied = 0;
+		int lc = 0, log_of[33] = {};  // plan.C and the rows of a stripe are powers of two
+		while ((1 << lc) < plan.C) lc++;
+		for (int g = 1; g <= 32; g *= 2)
+			while ((1 << log_of[g]) < g * plan_rows(plan)) log_of[g]++;
 		for (int64_t k = 0; k < B; k++) {
 			const int64_t a = ls[size_t(k)], b = lt[size_t(k)];
-			const int64_t gk = pair_g[size_t(k)], rpp = gk * plan_rows(plan);
-			const int64_t npass = (a == 0 || b == 0) ? 0 : (a + rpp - 1) / rpp;
-			const int64_t steps = (b + plan.C - 1) / plan.C + gk - 1;
+			const int64_t gk = pair_g[size_t(k)];
+			const int lr = log_of[gk];
+			const int64_t npass = (a == 0 || b == 0) ? 0 : (a + (int64_t(1) << lr) - 1) >> lr;
+			const int64_t steps = ((b + plan.C - 1) >> lc) + gk - 1;
 			mask_off[size_t(k) + 1] = mask_off[size_t(k)] + npass * steps * gk * plan_words(plan);
 			map_off[size_t(k) + 1] = map_off[size_t(k)] + std::min(a, b);
 			path_off[size_t(k) + 1] = path_off[size_t(k)] + 2 * (a + b + 2);
@@ -3052,6 +3069,55 @@ pa_status pa_solve_batch_result(pa_solver *s, const pa_batch *b, int32_t *maps, 
 	r->d->maps_external = true;
 	*out = r;
 	return PA_OK;
+}
+
+pa_status pa_pair_plan(const void *lengths, int32_t wide, int64_t batch, int64_t n_s, int64_t n_t, int32_t tile_s,
+                       int32_t tile_t, int32_t *len, int32_t *tile_start, int64_t *path_offsets, int64_t *totals) {
+	if (batch < 0 || tile_s <= 0 || tile_t <= 0 || (batch > 0 && !lengths) || !len || !tile_start || !path_offsets || !totals)
+		return fail(PA_ERR_INVALID_ARGUMENT, "pa_pair_plan: bad argument");
+	const int32_t *l32 = static_cast<const int32_t *>(lengths);
+	const int64_t *l64 = static_cast<const int64_t *>(lengths);
+	int ss = -1, st = -1;  // the tiles' logarithms where they are powers of two
+	for (int x = 0; x < 31; x++) {
+		if (tile_s == 1 << x) ss = x;
+		if (tile_t == 1 << x) st = x;
+	}
+	const uint32_t ts = uint32_t(tile_s), tt = uint32_t(tile_t);
+	int64_t tiles = 0, entries = 0;
+	tile_start[0] = 0;
+	for (int64_t k = 0; k < batch; k++) {
+		const int32_t ls = wide ? int32_t(l64[2 * k]) : l32[2 * k], lt = wide ? int32_t(l64[2 * k + 1]) : l32[2 * k + 1];
+		if (ls < 0 || lt < 0 || ls > n_s || lt > n_t) return fail(PA_ERR_LENGTH, "a length exceeds its array");
+		len[k] = ls;
+		len[batch + k] = lt;
+		const uint32_t cs = uint32_t(ls) + ts - 1, ct = uint32_t(lt) + tt - 1;
+		tiles += ss >= 0 && st >= 0 ? int64_t(cs >> ss) * int64_t(ct >> st) : int64_t(cs / ts) * int64_t(ct / tt);
+		tile_start[k + 1] = int32_t(tiles);
+		path_offsets[k] = entries;
+		entries += 2 * (int64_t(ls) + lt + 2);
+	}
+	totals[0] = tiles;
+	totals[1] = entries;
+	return PA_OK;
+}
+
+uint64_t pa_content_hash(const void *data, int64_t bytes) {
+	// four independent multiply chains over 8-byte words (a table key, compared in full on a hit)
+	constexpr uint64_t M = 0x9e3779b97f4a7c15ull;
+	uint64_t h[4] = {uint64_t(bytes), 1, 2, 3};
+	const char *p = static_cast<const char *>(data);
+	int64_t x = 0;
+	for (; x + 32 <= bytes; x += 32)
+		for (int c = 0; c < 4; c++) {
+			uint64_t w;
+			std::memcpy(&w, p + x + 8 * c, 8);
+			h[c] = (h[c] ^ w) * M;
+			h[c] ^= h[c] >> 29;
+		}
+	for (int c = 0; x < bytes; x++, c = (c + 1) & 3) h[c] = (h[c] ^ uint64_t(static_cast<unsigned char>(p[x]))) * M;
+	uint64_t r = 0;
+	for (int c = 0; c < 4; c++) r = (r ^ h[c] ^ (h[c] >> 31)) * M;
+	return r ^ (r >> 32);
 }
 
 pa_status pa_solve_dense_paths(pa_solver *s, const float *sim, const int64_t *offsets, int64_t stride_s,
