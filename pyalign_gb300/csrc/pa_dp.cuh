@@ -1044,6 +1044,6 @@ struct WalkParams {
 	int32_t *path_len;
 };
 
-__global__ void walk_kernel(WalkParams p);
+void launch_walk(const WalkParams &w, cudaStream_t st);
 
 }  // namespace pa

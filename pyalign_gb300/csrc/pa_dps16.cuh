@@ -1,4 +1,4 @@
-// Packed 16-bit DP kernel for scores alone (sm_103a).
+// Packed 16-bit DP kernel for scores alone, and with one traceback (sm_103a).
 //
 // Same recurrences and scores as dp_kernel (pa_dp.cuh; solver.h:2825-2855, 2970-3036, 1980-2327)
 // for integer scoring whose values provably fit in 16 bits.  As in dp16_kernel (pa_dp16.cuh)
@@ -43,6 +43,19 @@
 
 namespace pa {
 
+// With one traceback (TB): value * 4 + tag, the tag's order zero 3 > diagonal 2 > P 1 > Q 0 as in the
+// int32 kernels.  P = max(extend, open) is formed with tag 0 for its extension and 1 for its
+// opening, Q with 0 and 2 -- among equals the opening wins -- and then P takes its tag 1 and Q its
+// tag 0 for the choice of D.  The nibble of a cell, 4 (key - D) + (the opening bits), is dp16_kernel's
+// (code in bits 2-3, P-open bit 0, Q-open bit 1), worked out on the FMA pipe: differences of packed
+// values and the shift by a nibble are integer multiply-adds, exact in the end although a half may
+// borrow on the way.  Four tag values leave a quarter of the range (600 residues at 11 each still
+// fit, scores of -32 .. 31), eight ALU operations a twin cell of affine gaps.  Seeds as dp2_kernel's:
+// a local optimum's position is looked for only in steps whose maximum reaches the lane's best.
+// DNA that fits dp16_kernel's bounds stays there.  4,096 protein pairs of 50..600, global Gotoh, DP
+// alone: int32 0.73 -> 0.55 ms (too few pairs to fill the GPU with twins); whole calls, 6,400 of
+// 79..479 x 64..645 global linear 0.86 -> 0.61 ms.
+
 enum { SUBS_PROFILE = 0, SUBS_COLPROF = 1 };
 constexpr int CHAIN_CHUNK = PUB_CHUNK;  // boundary columns read at a time
 
@@ -67,6 +80,40 @@ __device__ __forceinline__ void cell_s16(const DpParams<int32_t> &p, uint32_t S,
 	D = LOC == LOC_LOCAL ? __vimax3_s16x2_relu(t, P, Q) : __vimax3_s16x2(t, P, Q);
 }
 
+// The same with a traceback: the tagged key, D and P clean but for P's tag 1, Q clean; `open`
+// receives a word whose difference to the clean Q is the opening bits.
+template <int GAP, int LOC>
+__device__ __forceinline__ uint32_t cell_t16(const DpParams<int32_t> &p, uint32_t S, uint32_t dsave, uint32_t old,
+                                             uint32_t &Q, uint32_t uD, uint32_t uP, uint32_t &D, uint32_t &P,
+                                             uint32_t &open) {
+	constexpr uint32_t CLEAN = 0xFFFCFFFCu, ONE = 0x00010001u, ZERO = 0x00030003u;
+	if (GAP == GAP_AFFINE) {
+		const uint32_t rP = __viaddmax_s16x2(uP, p.h_ext_s, s_add(uD, p.k_open_s));
+		const uint32_t rQ = __viaddmax_s16x2(Q, p.h_ext_t, s_add(old, p.k_open_t));
+		open = (rP & ONE) | (rQ & ~ONE);
+		P = (rP & CLEAN) | ONE;
+		Q = rQ & CLEAN;
+	} else {
+		P = s_add(uD, p.k_up);
+		Q = s_add(old, p.k_left);
+	}
+	const uint32_t key = LOC == LOC_LOCAL ? __viaddmax_s16x2(dsave, S, __vimax3_s16x2(P, Q, ZERO))
+	                                      : __vimax3_s16x2(s_add(dsave, S), P, Q);
+	D = key & CLEAN;
+	return key;
+}
+
+// The cell's nibbles behind those of the rows above it, in each half of w.
+template <int GAP>
+__device__ __forceinline__ void put_nib_t16(const DpParams<int32_t> &p, uint32_t &w, uint32_t key, uint32_t D, uint32_t Q,
+                                            uint32_t open) {
+	const int32_t below = imad(int32_t(key), p.minus_one, int32_t(D));  // -(the code)
+	if (GAP == GAP_AFFINE)
+		w = uint32_t(imad(below, p.minus_four, imad(int32_t(Q), p.minus_one, imad(int32_t(w), p.sixteen, int32_t(open)))));
+	else
+		w = uint32_t(imad(imad(int32_t(w), p.minus_four, below), p.minus_four, 0));
+}
+
 // Warps of a block: in stripe-chained mode one, so that the stripes in flight spread evenly over
 // the SMs (a stripe cannot outrun the one above it, so the fullest SM sets the pace of all: 2,560
 // stripes lie 16 or 17 to an SM; in blocks of four, 16 or 20).
@@ -81,8 +128,8 @@ __host__ __device__ constexpr int s16_smem(int G, bool colprof, bool chain) {
 	return s16_warps(chain) * ((32 / G) * (s16_ring(G) + 2 * G) * (colprof ? 2 : 4) + (chain ? 2 * CHAIN_CHUNK * 8 : 0));
 }
 
-template <int GAP, int LOC, int SUB, bool CHAIN>
-__global__ void __launch_bounds__(32 * s16_warps(CHAIN), CHAIN ? 17 : 4) dps16_kernel(DpParams<int32_t> p) {
+template <int GAP, int LOC, int SUB, bool CHAIN, bool TB>
+__global__ void __launch_bounds__(32 * s16_warps(CHAIN), CHAIN ? (TB ? 16 : 17) : 4) dps16_kernel(DpParams<int32_t> p) {
 	constexpr bool LOCAL = LOC == LOC_LOCAL;
 	constexpr int32_t NONE = INT32_MIN;
 	constexpr int NW = s16_warps(CHAIN), NT = 32 * NW;  // warps and threads of a block
@@ -115,7 +162,7 @@ __global__ void __launch_bounds__(32 * s16_warps(CHAIN), CHAIN ? 17 : 4) dps16_k
 	const int ntwins = (p.npairs + 1) >> 1;
 	const int rpp = G * R;
 	const int32_t off = p.h_off;
-	auto pack = [&](int32_t v) { return uint32_t((v + off) & 0xffff) * 0x10001u; };  // a value in both halves
+	auto pack = [&](int32_t v) { return uint32_t(((TB ? 4 * v : v) + off) & 0xffff) * 0x10001u; };  // a value in both halves
 	const uint32_t NEG = p.h_neg, LOW = p.h_low;
 	int cursor = -2;
 
@@ -167,6 +214,9 @@ __global__ void __launch_bounds__(32 * s16_warps(CHAIN), CHAIN ? 17 : 4) dps16_k
 
 		uint32_t l_best = 0;                 // local: the lane's best per half (at least 0)
 		int32_t resA = NONE, resB = NONE;    // global: the result; semiglobal: the lane's best seed value
+		// with a traceback: where the best lies (semiglobal: in the last column; rowA: the last row's)
+		int32_t iA = -1, jA = -1, iB = -1, jB = -1, rowA = NONE, rowB = NONE;
+		uint32_t reach = 0x00030003u;  // local: a maximum above this reaches the lane's best (and 0)
 
 		const int q_hi = CHAIN ? min(q_lo + 1, npass) : wpass;
 		for (int q = q_lo; q < q_hi; q++) {
@@ -223,11 +273,17 @@ __global__ void __launch_bounds__(32 * s16_warps(CHAIN), CHAIN ? 17 : 4) dps16_k
 			const bool lastB = pass_active && q == npB - 1 && nvB >= 1 && nvB <= R;
 			const int endA = ctA ? ((ctA - 1) >> 1) + sub : -1, endB = ctB ? ((ctB - 1) >> 1) + sub : -1;
 
+			uint32_t *mA = nullptr, *mB = nullptr;  // this lane's traceback words of step 0
+			if (TB) {
+				uint32_t *m = reinterpret_cast<uint32_t *>(p.masks);
+				if (pass_active && q < npA) mA = m + p.mask_off[pa] + (int64_t(q) * (((ltA + 1) >> 1) + G - 1) * G + sub) * 2;
+				if (pass_active && q < npB) mB = m + p.mask_off[pb] + (int64_t(q) * (((ltB + 1) >> 1) + G - 1) * G + sub) * 2;
+			}
 			// semiglobal: a lane of the warp holds a last row in this pass (warp-uniform)
 			const bool has_last = LOC == LOC_SEMI && __any_sync(0xffffffffu, lastA || lastB);
-			uint32_t rmax[LOC == LOC_SEMI ? R : 1];
+			uint32_t rmax[LOC == LOC_SEMI && !TB ? R : 1];
 #pragma unroll
-			for (int r = 0; r < (LOC == LOC_SEMI ? R : 1); r++) rmax[r] = 0x80008000u;
+			for (int r = 0; r < (LOC == LOC_SEMI && !TB ? R : 1); r++) rmax[r] = 0x80008000u;
 
 			// group mode: (D, P) above the next step's columns, for the group's first lane: the top
 			// border, or what this warp's last lane wrote in the previous pass, a step ahead
@@ -361,6 +417,7 @@ __global__ void __launch_bounds__(32 * s16_warps(CHAIN), CHAIN ? 17 : 4) dps16_k
 					uint32_t dsave0 = prev_up, dsave1 = upD0;
 					uint32_t uD0 = upD0, uP0 = upP0, uD1 = upD1, uP1 = upP1;
 					uint32_t c0[R];  // column j0 (Dl: column j1 after the step)
+					uint32_t mlo0 = 0, mhi0 = 0, mlo1 = 0, mhi1 = 0;
 					auto sub_of = [&](int r, uint32_t sel, uint2 a, uint2 b) {
 						if (SUB == SUBS_PROFILE) return uint32_t(prmt(prA[r], prB[r], sel));
 						return uint32_t(r < 4 ? prmt(a.x, b.x, uint32_t(r) * 0x1111u + 0xC480u)
@@ -370,8 +427,16 @@ __global__ void __launch_bounds__(32 * s16_warps(CHAIN), CHAIN ? 17 : 4) dps16_k
 					for (int r = 0; r < R; r++) {
 						const uint32_t old = Dl[r];
 						uint32_t Q = Ql[r], D0, P0, D1, P1;
-						cell_s16<GAP, LOC>(p, sub_of(r, sel0, xA0, xB0), dsave0, old, Q, uD0, uP0, D0, P0);
-						cell_s16<GAP, LOC>(p, sub_of(r, sel1, xA1, xB1), dsave1, D0, Q, uD1, uP1, D1, P1);
+						if constexpr (TB) {
+							uint32_t open = 0;
+							uint32_t key = cell_t16<GAP, LOC>(p, sub_of(r, sel0, xA0, xB0), dsave0, old, Q, uD0, uP0, D0, P0, open);
+							put_nib_t16<GAP>(p, r < 4 ? mlo0 : mhi0, key, D0, Q, open);
+							key = cell_t16<GAP, LOC>(p, sub_of(r, sel1, xA1, xB1), dsave1, D0, Q, uD1, uP1, D1, P1, open);
+							put_nib_t16<GAP>(p, r < 4 ? mlo1 : mhi1, key, D1, Q, open);
+						} else {
+							cell_s16<GAP, LOC>(p, sub_of(r, sel0, xA0, xB0), dsave0, old, Q, uD0, uP0, D0, P0);
+							cell_s16<GAP, LOC>(p, sub_of(r, sel1, xA1, xB1), dsave1, D0, Q, uD1, uP1, D1, P1);
+						}
 						dsave0 = old;
 						dsave1 = D0;
 						c0[r] = D0;
@@ -391,6 +456,15 @@ __global__ void __launch_bounds__(32 * s16_warps(CHAIN), CHAIN ? 17 : 4) dps16_k
 						if (CHAIN) *reinterpret_cast<uint4 *>(outrow + (j0 & (CHAIN_CHUNK - 1))) = o;
 						else bout[s - sub] = o;
 					}
+					if (TB) {
+						// rows 0-3 of each half in mlo, 4-7 in mhi, row r at bits 4 (R - 1 - r) of the word
+						if (mA && j0 < ctA)
+							reinterpret_cast<uint2 *>(mA)[int64_t(s) * G] =
+							    make_uint2(__byte_perm(mhi0, mlo0, 0x5410), __byte_perm(mhi1, mlo1, 0x5410));
+						if (mB && j0 < ctB)
+							reinterpret_cast<uint2 *>(mB)[int64_t(s) * G] =
+							    make_uint2(__byte_perm(mhi0, mlo0, 0x7632), __byte_perm(mhi1, mlo1, 0x7632));
+					}
 					if (LOCAL) {
 						uint32_t m0 = __vimax3_s16x2(c0[0], c0[1], c0[2]), m1 = __vimax3_s16x2(Dl[0], Dl[1], Dl[2]);
 						m0 = __vimax3_s16x2(m0, c0[3], c0[4]);
@@ -403,34 +477,87 @@ __global__ void __launch_bounds__(32 * s16_warps(CHAIN), CHAIN ? 17 : 4) dps16_k
 							m0 &= colmask16(j0, ctA, ctB);
 							m1 &= colmask16(j1, ctA, ctB);
 						}
-						l_best = __vimax3_s16x2(l_best, m0, m1);
+						if (!TB) {
+							l_best = __vimax3_s16x2(l_best, m0, m1);
+						} else if (__vimax3_s16x2(m0, m1, reach) != reach) {
+							// the step's best of a half reaches the lane's: its largest row, then column
+							const uint32_t m = __vmaxs2(m0, m1);
+							auto look = [&](int sh, int ct, int32_t &best, int32_t &bi, int32_t &bj) {
+								const int32_t v = int32_t((m >> sh) & 0xffffu);
+								if (v == 0 || v < best) return;
+								int at = 0, aj = j0;
+#pragma unroll
+								for (int r = 0; r < R; r++) {
+									const bool x0 = int32_t((c0[r] >> sh) & 0xffffu) == v, x1 = j1 < ct && int32_t((Dl[r] >> sh) & 0xffffu) == v;
+									if (x0 || x1) {
+										at = r;
+										aj = x1 ? j1 : j0;
+									}
+								}
+								if (v > best || row0 + at >= bi) {
+									bi = row0 + at;
+									bj = aj;
+								}
+								best = v;
+							};
+							look(0, ctA, resA, iA, jA);
+							look(16, ctB, resB, iB, jB);
+							reach = uint32_t(max(resA, 4) - 1) | uint32_t(max(resB, 4) - 1) << 16;
+						}
 					} else {
 						auto lo16 = [](uint32_t x) { return int32_t(int16_t(x & 0xffffu)); };
 						auto hi16 = [](uint32_t x) { return int32_t(x) >> 16; };
-						if (LOC == LOC_SEMI && has_last) {
+						if (TB && LOC == LOC_SEMI && has_last) {
+							// the first of the largest in the pair's last row, by the lane that holds it
+							auto row_of = [&](const uint32_t (&x)[R], int nv) {
+								uint32_t v = x[0];
+#pragma unroll
+								for (int r = 1; r < R; r++)
+									if (r == nv - 1) v = x[r];
+								return v;
+							};
+							if (lastA && j0 < ltA) {
+								const int32_t x = lo16(row_of(c0, nvA)) - off, y = lo16(row_of(Dl, nvA)) - off;
+								if (x > rowA) { rowA = x; jA = j0; }
+								if (j1 < ltA && y > rowA) { rowA = y; jA = j1; }
+							}
+							if (lastB && j0 < ltB) {
+								const int32_t x = hi16(row_of(c0, nvB)) - off, y = hi16(row_of(Dl, nvB)) - off;
+								if (x > rowB) { rowB = x; jB = j0; }
+								if (j1 < ltB && y > rowB) { rowB = y; jB = j1; }
+							}
+						} else if (!TB && LOC == LOC_SEMI && has_last) {
 							// the running maximum of every row over the columns inside each pair's |t|; the last
 							// row's is taken after the pass
 							if (j1 < ctmin) {
 #pragma unroll
-								for (int r = 0; r < R; r++) rmax[r] = __vimax3_s16x2(rmax[r], c0[r], Dl[r]);
+								for (int r = 0; r < R; r++) rmax[TB ? 0 : r] = __vimax3_s16x2(rmax[TB ? 0 : r], c0[r], Dl[r]);
 							} else {
 								const uint32_t m0 = colmask16(j0, ctA, ctB), m1 = colmask16(j1, ctA, ctB);
 #pragma unroll
 								for (int r = 0; r < R; r++)
-									rmax[r] = __vimax3_s16x2(rmax[r], (c0[r] & m0) | (0x80008000u & ~m0), (Dl[r] & m1) | (0x80008000u & ~m1));
+									rmax[TB ? 0 : r] = __vimax3_s16x2(rmax[TB ? 0 : r], (c0[r] & m0) | (0x80008000u & ~m0), (Dl[r] & m1) | (0x80008000u & ~m1));
 							}
 						}
 						if (s == endA) {  // the pair's last column
 							const bool odd = j0 == ltA - 1;
 #pragma unroll
 							for (int r = 0; r < R; r++)
-								if (LOC == LOC_SEMI ? r < nvA : (lastA && r == nvA - 1)) resA = max(resA, lo16(odd ? c0[r] : Dl[r]) - off);
+								if (LOC == LOC_SEMI ? r < nvA : (lastA && r == nvA - 1)) {
+									const int32_t x = lo16(odd ? c0[r] : Dl[r]) - off;
+									if (TB && x > resA) iA = row0 + r;
+									resA = max(resA, x);
+								}
 						}
 						if (s == endB) {
 							const bool odd = j0 == ltB - 1;
 #pragma unroll
 							for (int r = 0; r < R; r++)
-								if (LOC == LOC_SEMI ? r < nvB : (lastB && r == nvB - 1)) resB = max(resB, hi16(odd ? c0[r] : Dl[r]) - off);
+								if (LOC == LOC_SEMI ? r < nvB : (lastB && r == nvB - 1)) {
+									const int32_t x = hi16(odd ? c0[r] : Dl[r]) - off;
+									if (TB && x > resB) iB = row0 + r;
+									resB = max(resB, x);
+								}
 						}
 					}
 				}
@@ -444,24 +571,48 @@ __global__ void __launch_bounds__(32 * s16_warps(CHAIN), CHAIN ? 17 : 4) dps16_k
 					}
 				}
 			}
-			if (LOC == LOC_SEMI && has_last) {
+			if (!TB && LOC == LOC_SEMI && has_last) {
 #pragma unroll
 				for (int r = 0; r < R; r++) {
-					if (lastA && r == nvA - 1) resA = max(resA, int32_t(int16_t(rmax[r] & 0xffffu)) - off);
-					if (lastB && r == nvB - 1) resB = max(resB, (int32_t(rmax[r]) >> 16) - off);
+					if (lastA && r == nvA - 1) resA = max(resA, int32_t(int16_t(rmax[TB ? 0 : r] & 0xffffu)) - off);
+					if (lastB && r == nvB - 1) resB = max(resB, (int32_t(rmax[TB ? 0 : r]) >> 16) - off);
 				}
 			}
 			__syncwarp();
 		}
 
 		// ---- the twin's results: maxima over the group (global: the one lane that has it)
-		if (LOCAL) {
+		if (LOCAL && !TB) {
 			resA = emptyA ? NONE : int32_t(l_best & 0xffffu);
 			resB = emptyB ? NONE : int32_t(l_best >> 16);
 		}
+		// with positions: local, the largest row, then column, of the largest; semiglobal, the
+		// smallest row of the last column's largest (the last row's is one lane's)
+		auto fold = [&](int32_t &v, int32_t &i, int32_t &j, int32_t ov, int32_t oi, int32_t oj) {
+			const bool take = LOCAL ? ov > v || (ov == v && (oi > i || (oi == i && oj > j)))
+			                        : oi >= 0 && (i < 0 || ov > v || (ov == v && oi < i));
+			if (take) {
+				v = ov;
+				i = oi;
+				if (LOCAL) j = oj;
+			}
+		};
 		for (int o = 1; o < G; o <<= 1) {
-			resA = max(resA, __shfl_xor_sync(0xffffffffu, resA, o, G));
-			resB = max(resB, __shfl_xor_sync(0xffffffffu, resB, o, G));
+			const int32_t oA = __shfl_xor_sync(0xffffffffu, resA, o, G), oB = __shfl_xor_sync(0xffffffffu, resB, o, G);
+			if (TB && LOC != LOC_GLOBAL) {
+				const int32_t oiA = __shfl_xor_sync(0xffffffffu, iA, o, G), ojA = __shfl_xor_sync(0xffffffffu, jA, o, G);
+				const int32_t oiB = __shfl_xor_sync(0xffffffffu, iB, o, G), ojB = __shfl_xor_sync(0xffffffffu, jB, o, G);
+				fold(resA, iA, jA, oA, oiA, ojA);
+				fold(resB, iB, jB, oB, oiB, ojB);
+				if (LOC == LOC_SEMI) {
+					const int32_t orA = __shfl_xor_sync(0xffffffffu, rowA, o, G), orB = __shfl_xor_sync(0xffffffffu, rowB, o, G);
+					if (orA > rowA) { rowA = orA; jA = ojA; }
+					if (orB > rowB) { rowB = orB; jB = ojB; }
+				}
+			} else {
+				resA = max(resA, oA);
+				resB = max(resB, oB);
+			}
 		}
 		bool last_unit = true;
 		if (CHAIN) {
@@ -470,11 +621,24 @@ __global__ void __launch_bounds__(32 * s16_warps(CHAIN), CHAIN ? 17 : 4) dps16_k
 			if (q_lo > 0) {
 				if (ld_acquire(p.progress + prod) < lt) wait_progress(p.progress + prod, lt, p.status);
 				const int4 rc = __ldcg(p.chain + prod);
-				resA = max(resA, rc.x);
-				resB = max(resB, rc.y);
+				if (TB && LOCAL) {  // positions in 16 bits each (the host's bound)
+					fold(resA, iA, jA, rc.x, rc.z < 0 ? -1 : rc.z >> 16, rc.z < 0 ? -1 : rc.z & 0xffff);
+					fold(resB, iB, jB, rc.y, rc.w < 0 ? -1 : rc.w >> 16, rc.w < 0 ? -1 : rc.w & 0xffff);
+				} else if (TB && LOC == LOC_SEMI) {
+					fold(resA, iA, jA, rc.x, rc.z, -1);
+					fold(resB, iB, jB, rc.y, rc.w, -1);
+				} else {
+					resA = max(resA, rc.x);
+					resB = max(resB, rc.y);
+				}
 			}
 			if (!last_unit && lane == 0) {
-				p.chain[base] = make_int4(resA, resB, 0, 0);
+				int32_t zA = iA, zB = iB;
+				if (LOCAL) {
+					zA = iA < 0 ? -1 : iA << 16 | jA;
+					zB = iB < 0 ? -1 : iB << 16 | jB;
+				}
+				p.chain[base] = make_int4(resA, resB, zA, zB);
 				st_release(p.progress + base, lt);  // every column (put_row, before a __syncwarp), and the record
 			}
 		}
@@ -494,8 +658,43 @@ __global__ void __launch_bounds__(32 * s16_warps(CHAIN), CHAIN ? 17 : 4) dps16_k
 						for (int i = 0; i < n; i++) v = max(v, p.left_D[i + 1]);
 					}
 				}
+				int32_t si = -1, sj = -1;  // scores alone: no seed
+				if (TB && n > 0 && m > 0) {
+					const int32_t bi = h ? iB : iA, bj = h ? jB : jA, row = h ? rowB : rowA;
+					si = n - 1;
+					sj = m - 1;
+					if (LOCAL) {
+						if (v == NONE) v = 0;  // every cell is 0: the last one
+						if (v > 0) {
+							si = bi;
+							sj = bj;
+						}
+					}
+					if (LOC == LOC_SEMI) {
+						if (bj >= 0 && (bi < 0 || !(v > row))) {
+							v = row;
+							sj = bj;
+						} else {
+							si = bi;
+						}
+					}
+					v >>= 2;
+				} else if (TB) {
+					if (LOC == LOC_GLOBAL) {
+						si = n - 1;
+						sj = m - 1;
+					}
+					if (LOC == LOC_SEMI) {
+						int32_t b = NONE;
+						for (int j = 0; j < m; j++)
+							if (p.top_D[j + 1] > b) { b = p.top_D[j + 1]; si = n - 1; sj = j; }
+						for (int i = 0; i < n; i++)
+							if (p.left_D[i + 1] > b) { b = p.left_D[i + 1]; si = i; sj = m - 1; }
+					}
+				}
 				p.score[pair] = v == NONE ? -INFINITY * p.out_sign : float(v) * p.out_sign;
-				p.seed[2 * pair] = p.seed[2 * pair + 1] = -1;  // scores alone
+				p.seed[2 * pair] = si;
+				p.seed[2 * pair + 1] = sj;
 				p.has_seed[pair] = v != NONE;
 			}
 		}

@@ -518,7 +518,7 @@ struct Plan {
 	SegInfo segs[PA_MAX_CHUNKS];
 	int32_t h_neg = 0;
 	bool uneven = false;       // the pairs' costs differ: group mode spreads the first tasks (run_dp)
-	bool s16 = false;          // scores alone in packed 16-bit twins (dps16_kernel), before h16
+	bool s16 = false;          // packed 16-bit twins of dps16_kernel: scores alone, or one traceback where h16 is not
 	int32_t s_neg = 0, h_off = 0, h_low = 0;
 	int sub2 = -1;             // float: what dpf2_kernel reads (C = 2), or -1
 	int64_t copy_pitch = 0;    // float, dense: > 0, the similarity is copied first, with this pitch
@@ -602,26 +602,35 @@ bool h16_plan(const pa_solver *s, const Input &in, const float *host_table, cons
 // border, then down and across; local: 0).  P and Q lie at most one opening and one extension
 // lower, a padding row's diagonal 128.  It also needs an indexed form of at most 32 letters of t,
 // int8 similarities, and gap costs of at least 0 (rows past |s| must not exceed the optimum).
+// One traceback in the same twins holds value * 4 + tag: a quarter of the range, similarities of
+// -32 .. 31, for local alignment gap costs of at least 1 (a row past |s| must not even tie) and
+// positions of 15 bits; it takes the launches that dp16_kernel cannot -- more than 4 letters,
+// semiglobal alignment, values past a sixteenth of the range.
 // PA_DP16=0 turns it off, as do the switches that pick a variant of dp16_kernel.
-bool s16_plan(const pa_solver *s, const Input &in, const float *host_table, int64_t mls, int64_t mlt, Plan &plan) {
+bool s16_plan(const pa_solver *s, const Input &in, const float *host_table, int64_t mls, int64_t mlt, bool want_values,
+              Plan &plan) {
 	for (const char *e : {"PA_DP_BLOCK", "PA_BUCKET_WIDTHS"})
 		if (std::getenv(e)) return false;
 	if (const char *e = std::getenv("PA_DP16"))
 		if (std::strcmp(e, "0") == 0) return false;
 	if (const char *e = std::getenv("PA_DP_COLS"))
 		if (std::atoi(e) == 1) return false;
-	if (!plan.use_int || plan.tb != TB_NONE || in.form != F_INDEXED) return false;
+	if (!plan.use_int || plan.tb == TB_ALL || want_values || in.form != F_INDEXED) return false;
+	const bool tagged = plan.tb == TB_ONE;
+	const double unit = tagged ? 4 : 1;
+	if (tagged && s->loc == LOC_LOCAL && (mls > 32767 || mlt > 32767)) return false;
 	if (in.table_cols > MAX_COLPROF || in.table_rows > MAX_SMEM_TABLE || in.table_cols < 1) return false;
 	if (s->gap != GAP_LINEAR && s->gap != GAP_AFFINE) return false;
 	const pa_options &o = s->opt;
 	const bool affine = s->gap == GAP_AFFINE;
 	const double us = affine ? o.affine_u_s : o.linear_s, ut = affine ? o.affine_u_t : o.linear_t;
 	const double ws = affine ? double(o.affine_u_s) + o.affine_v_s : us, wt = affine ? double(o.affine_u_t) + o.affine_v_t : ut;
-	if (!(us >= 0 && ut >= 0 && ws >= 0 && wt >= 0)) return false;
+	const double least = tagged && s->loc == LOC_LOCAL ? 1 : 0;
+	if (!(us >= least && ut >= least && ws >= least && wt >= least)) return false;
 	double smax = 0;
 	for (int64_t k = 0; k < in.table_rows * in.table_cols; k++) {
 		const double v = double(host_table[k]) * s->sign;
-		if (v < -128 || v > 127) return false;
+		if (v * unit + (tagged ? 2 : 0) < -128 || v * unit + (tagged ? 2 : 0) > 127) return false;
 		smax = std::max(smax, v);
 	}
 	double bmin = 0, bmax = 0;
@@ -635,16 +644,17 @@ bool s16_plan(const pa_solver *s, const Input &in, const float *host_table, int6
 		bmin = std::min(bmin, double(s->top_D[size_t(k)]));
 		bmax = std::max(bmax, double(s->top_D[size_t(k)]));
 	}
-	const double hi = smax * double(std::min(mls, mlt)) + bmax;
+	const double hi = (smax * double(std::min(mls, mlt)) + bmax) * unit + (unit - 1);
 	const double down = ws + us * double(mls + 256), across = wt + ut * double(mlt);
 	const double lo = s->loc == LOC_LOCAL ? 0.0 : s->loc == LOC_SEMI ? -std::min(down, across) : bmin - down - across;
-	const double step = std::max(ws, wt) + std::max(us, ut) + 128.0;
-	const double neg = -32767.0 + std::max({us, ut, ws, wt, 128.0});  // a gap below it stays in range
-	const double off = s->loc == LOC_LOCAL ? 0.0 : neg + step + 1.0 - lo;
-	if (lo + off - step < neg || hi + off > 32767.0) return false;
+	// in the units of the packed values; the sentinel and the offset are values without a tag
+	const double step = (std::max(ws, wt) + std::max(us, ut)) * unit + 128.0 + 2 * (unit - 1);
+	const double neg = std::ceil((-32767.0 + std::max(std::max({us, ut, ws, wt}) * unit, 128.0) + 2 * (unit - 1)) / unit) * unit;
+	const double off = s->loc == LOC_LOCAL ? 0.0 : std::ceil((neg + step + 1.0 - lo * unit) / unit) * unit;
+	if (lo * unit + off - step < neg || hi + off > 32767.0) return false;
 	plan.s_neg = int32_t(neg);
 	plan.h_off = int32_t(off);
-	plan.h_low = int32_t((s->loc == LOC_GLOBAL ? lo : 0.0) + off);
+	plan.h_low = int32_t((s->loc == LOC_GLOBAL ? lo * unit : 0.0) + off);
 	return true;
 }
 
@@ -959,15 +969,18 @@ pa_status run_dp(pa_solver *s, const Input &in, const Plan &plan, int tb, const 
 		p.h_neg = h16_value(plan.h_neg);
 	}
 	if (s16) {
-		auto both = [](float x) { return h16_pack(int32_t(std::nearbyint(x))); };
+		// with a traceback value * 4 + tag: P extends from tag 1 to 0 and opens to 1, Q from 0 to 0
+		// and to 2
+		const bool t = tb == TB_ONE;
+		auto both = [&](float x, int tag) { return h16_pack(t ? int32_t(std::nearbyint(x)) * 4 + tag : int32_t(std::nearbyint(x))); };
 		if (gk == GAP_LINEAR) {
-			p.k_up = both(-o.linear_s);
-			p.k_left = both(-o.linear_t);
+			p.k_up = both(-o.linear_s, 1);
+			p.k_left = both(-o.linear_t, 0);
 		} else {
-			p.k_open_s = both(-(o.affine_u_s + o.affine_v_s));
-			p.h_ext_s = both(-o.affine_u_s);
-			p.k_open_t = both(-(o.affine_u_t + o.affine_v_t));
-			p.h_ext_t = both(-o.affine_u_t);
+			p.k_open_s = both(-(o.affine_u_s + o.affine_v_s), 1);
+			p.h_ext_s = both(-o.affine_u_s, -1);
+			p.k_open_t = both(-(o.affine_u_t + o.affine_v_t), 2);
+			p.h_ext_t = both(-o.affine_u_t, 0);
 		}
 		p.h_off = plan.h_off;
 		p.h_neg = h16_pack(plan.s_neg);
@@ -1023,6 +1036,7 @@ pa_status run_dp(pa_solver *s, const Input &in, const Plan &plan, int tb, const 
 			bool fits_int8 = ISINT && tag && in.table_cols <= 8 && in.table_rows <= MAX_SMEM_TABLE;
 			for (size_t k = 0; k < nt_; k++) {
 				tabv[k] = h16 ? V(int32_t(std::nearbyint(host_table[k] * s->sign)) * 16 + 8)
+				          : s16 && tb == TB_ONE ? V(int32_t(std::nearbyint(host_table[k] * s->sign)) * 4 + 2)
 				              : cvt<V>(host_table[k] * s->sign, ISINT, scale, diag_tag);
 				if (ISINT && (int64_t(tabv[k]) < -128 || int64_t(tabv[k]) > 127)) fits_int8 = false;
 			}
@@ -1094,6 +1108,8 @@ pa_status run_dp(pa_solver *s, const Input &in, const Plan &plan, int tb, const 
 		                              : occupancy_dp16b_affine(loc, tb, smem, &bps);
 		else if (h16) e = gk == GAP_LINEAR ? occupancy_dp16_linear(loc, tb, cols, smem, &bps)
 		                                   : occupancy_dp16_affine(loc, tb, cols, smem, &bps);
+		else if (s16 && tb == TB_ONE) e = gk == GAP_LINEAR ? occupancy_dps16t_linear(loc, subs, ch, smem, &bps)
+		                                                   : occupancy_dps16t_affine(loc, subs, ch, smem, &bps);
 		else if (s16) e = gk == GAP_LINEAR ? occupancy_dps16_linear(loc, subs, ch, smem, &bps)
 		                                   : occupancy_dps16_affine(loc, subs, ch, smem, &bps);
 		else if (sub2 >= 0) e = gk == GAP_LINEAR   ? occupancy_dpf2_linear(loc, tb, sub2, smem, &bps)
@@ -1156,6 +1172,8 @@ pa_status run_dp(pa_solver *s, const Input &in, const Plan &plan, int tb, const 
 		                              : launch_dp16b_affine(loc, tb, p, int(grid), smem, st);
 		else if (h16) e = gk == GAP_LINEAR ? launch_dp16_linear(loc, tb, cols, p, int(grid), smem, st)
 		                                   : launch_dp16_affine(loc, tb, cols, p, int(grid), smem, st);
+		else if (s16 && tb == TB_ONE) e = gk == GAP_LINEAR ? launch_dps16t_linear(loc, subs, ch, p, int(grid), smem, st)
+		                                                   : launch_dps16t_affine(loc, subs, ch, p, int(grid), smem, st);
 		else if (s16) e = gk == GAP_LINEAR ? launch_dps16_linear(loc, subs, ch, p, int(grid), smem, st)
 		                                   : launch_dps16_affine(loc, subs, ch, p, int(grid), smem, st);
 		else e = dp_launch<V>(gk, ch, loc, tb, want_values, p, int(grid), smem, st, cols);
@@ -1546,7 +1564,12 @@ constexpr double TUNE_MIN_CELLS = 4e6;  // smaller launches keep the analytic ch
 // two pairs' profiles at the head of a stripe, so the tuner times both, and below TUNE_MIN_CELLS
 // the int32 kernel runs (266 pairs of 13..27 x 51..102: 98 us a call in int32, 107 in 16 bits; 1,203
 // of 39..196 x 20..80 89 and 101; 2,647 of 35..350 x 36..144 211 and 171).
+// With one traceback the same holds (protein pairs of 50..600, chained, us a call in int32 and in
+// 16 bits: 256 pairs 338 and 355, 512 387 and 363, 1,024 470 and 425, 4,096 871 and 672; in groups
+// 65,536 8,118 and 4,907; local alignment gains less, 8,636 and 5,826), but for fewer than
+// S16_SURE_PAIRS however long: twins halve the stripes in flight.
 constexpr double S16_SURE_CELLS = 2e8;
+constexpr size_t S16_SURE_PAIRS = 2048;
 constexpr int64_t SPREAD_MIN_CELLS = 50000000;  // smaller launches take their tasks from one counter
 
 uint64_t tune_key(const pa_solver *s, const Input &in, const Plan &plan, const std::vector<int32_t> &ls,
@@ -1616,7 +1639,7 @@ pa_status tune_plan(pa_solver *s, const std::vector<int32_t> &ls, const std::vec
 		bool s16;
 	};
 	std::vector<Cand> cand;
-	const bool both = plan.s16 && cells < S16_SURE_CELLS;
+	const bool both = plan.s16 && (cells < S16_SURE_CELLS || (plan.tb == TB_ONE && ls.size() < S16_SURE_PAIRS));
 	for (int G : {32, 16, 8, 4, 2, 1})
 		if (G == 4 || (int64_t(G) * R <= 2 * plan.max_ls && (G >= 4 || plan.max_ls <= 256))) {
 			cand.push_back({G, false, false, C0, false, plan.s16});
@@ -1630,7 +1653,10 @@ pa_status tune_plan(pa_solver *s, const std::vector<int32_t> &ls, const std::vec
 	if (plan.h16 && !plan.s16 && C0 == 2)
 		for (int G : {32, 16, 8})
 			if (int64_t(G) * 4 <= 2 * plan.max_ls) cand.push_back({G, false, true, 4, true, false});
-	if (plan.max_ls > 2 * 32 * R) cand.push_back({32, true, false, cols_of(plan, true), false, plan.s16});
+	if (plan.max_ls > 2 * 32 * R) {
+		cand.push_back({32, true, false, cols_of(plan, true), false, plan.s16});
+		if (both) cand.push_back({32, true, false, cols_of(plan, true), false, false});
+	}
 	if (cand.size() < 2) return PA_OK;
 	cudaStream_t st = s->stream;
 	float best = INFINITY;
@@ -1942,6 +1968,7 @@ pa_status solve_impl(pa_solver *s, const Input &in, int method, float *scores_ou
 	plan.max_ls = max_ls;
 	plan.max_lt = max_lt;
 	plan.tb = tb;
+	int64_t cells_sum = 0;
 	if (!hit) {
 		plan.G = choose_G(ls, lt, s->sm_count);
 		int64_t most = 0, sum = 0, n = 0;
@@ -1951,6 +1978,7 @@ pa_status solve_impl(pa_solver *s, const Input &in, int method, float *scores_ou
 			sum += c;
 			n += c > 0;
 		}
+		cells_sum = sum;
 		plan.uneven = 2 * most * n > 3 * sum && sum >= SPREAD_MIN_CELLS;  // the largest over 1.5 times the mean
 	}
 	if (!hit && s->gap != GAP_GENERAL) {
@@ -1985,9 +2013,12 @@ pa_status solve_impl(pa_solver *s, const Input &in, int method, float *scores_ou
 			if (std::atoi(e) == 1) plan.C32 = 1;
 		plan.C = cols_of(plan, plan.units);
 		int32_t hneg = 0;
-		plan.s16 = s16_plan(s, in, host_table.data(), max_ls, max_lt, plan);
 		plan.h16 = !plan.units && h16_plan(s, in, host_table.data(), ls, lt, tb, want_values, use_int, &hneg);
 		plan.h_neg = hneg;
+		// (one traceback: small launches in int32, see S16_SURE_CELLS; PA_DP16=all for tests)
+		const char *all16 = std::getenv("PA_DP16");
+		const bool large = double(cells_sum) >= TUNE_MIN_CELLS || (all16 && std::strcmp(all16, "all") == 0);
+		plan.s16 = !(tb == TB_ONE && (plan.h16 || !large)) && s16_plan(s, in, host_table.data(), max_ls, max_lt, want_values, plan);
 		if (plan.h16) plan.C = plan.C32;  // two columns per step unless PA_DP_COLS=1
 		if (const char *e = std::getenv("PA_DP_BLOCK"))  // experiments and tests: the 4 x 4 block kernel
 			if (plan.h16 && std::strcmp(e, "1") == 0) {
@@ -2251,7 +2282,7 @@ pa_status solve_impl(pa_solver *s, const Input &in, int method, float *scores_ou
 		w.mask_off = s->m.mask_off;
 		w.G = plan.G;
 		w.cols = plan.C;
-		w.fmt16 = plan.h16 ? 1 : 0;
+		w.fmt16 = plan.h16 || plan.s16 ? 1 : 0;
 		w.rows4 = plan.blk ? 1 : 0;
 		w.pair_G = plan.seg ? s->m.pair_G : nullptr;
 		w.status = s->d_status.as<int32_t>();
@@ -2307,7 +2338,7 @@ pa_status solve_impl(pa_solver *s, const Input &in, int method, float *scores_ou
 		if (need_walk) {
 		PA_CUDA(ensure_walk_buffers());
 		WalkParams w = walk_params();
-		walk_kernel<<<int((B + 3) / 4), 128, 0, sw>>>(w);  // a warp per pair
+		launch_walk(w, sw);
 		PA_CUDA(cudaGetLastError());
 		launches++;
 		}
@@ -2413,7 +2444,7 @@ pa_status solve_impl(pa_solver *s, const Input &in, int method, float *scores_ou
 				WalkParams w = walk_params();
 				w.pair0 = int32_t(k0);
 				w.npairs = int32_t(k1 - k0);
-				walk_kernel<<<int((k1 - k0 + 3) / 4), 128, 0, sc>>>(w);
+				launch_walk(w, sc);
 				PA_CUDA(cudaGetLastError());
 				launches++;
 				if (!defer_maps) {

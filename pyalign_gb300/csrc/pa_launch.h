@@ -56,6 +56,15 @@ PA_DECLS16(linear)
 PA_DECLS16(affine)
 #undef PA_DECLS16
 
+// the same with one traceback
+#define PA_DECLS16(GAP)                                                                              \
+	cudaError_t launch_dps16t_##GAP(int loc, int sub, bool chain, const DpParams<int32_t> &p, int grid, \
+	                                size_t smem, cudaStream_t st);                                \
+	cudaError_t occupancy_dps16t_##GAP(int loc, int sub, bool chain, size_t smem, int *blocks_per_sm);
+PA_DECLS16(linear)
+PA_DECLS16(affine)
+#undef PA_DECLS16
+
 #define PA_DECL16B(GAP)                                                                                 \
 	cudaError_t launch_dp16b_##GAP(int loc, int tb, const DpParams<int32_t> &p, int grid, size_t smem,  \
 	                               cudaStream_t st);                                                 \
