@@ -26,13 +26,14 @@
 // entry a point pushes is the next one popped, so it stays in registers and only the others
 // are written to the stack.  Most cells of a path have the diagonal as their only entry: from
 // every cell the lanes test the 32 cells up its diagonal at once (one ballot), and a run of such
-// cells is appended to the path in one step; only the cells that branch go through the search.
+// cells is appended to the path in one step; only the cells that branch go through the search, and
+// the openings of a gap are looked for 32 cells at a time as well.
 // What bounds it then is round trips: one per window and, per yielded path, those of reading the
 // path back, 256 points in flight together.  A yield differs from the one before it only past
 // the point where the search turned, mostly near the path's end: with the pair's current map in
 // shared memory (pairs of up to ENUM_SMEM_MAP) only that part of map and hash is worked out.  The
 // stack's lower 256 entries lie there too.  16 pairs of 2000..3000 x 3000..5000, the first 101
-// alignments of each: 9.66 -> 2.83 ms.  Local seeds come from enum_seed_kernel (every cell with the
+// alignments of each: 9.66 -> 2.14 ms.  Local seeds come from enum_seed_kernel (every cell with the
 // seed bit, one block per pair), sorted on the host in the order the reference's stack
 // pops them: increasing row, then increasing column.
 //
@@ -90,35 +91,46 @@ struct Window {
 	int gb0, j0;  // row blocks [gb0, gb0 + WIN_B), columns [j0, j0 + WIN_C)
 };
 
-// cell (i, j) of the pair's masks through the warp's shared window (warp-uniform call)
-__device__ __forceinline__ uint32_t enum_cell(const EnumParams &p, uint4 (*win)[WIN_C], Window &w, const uint4 *m,
-                                              int64_t S, int ls, int lt, int i, int j, int lane) {
-	const int gb = i >> 3;
-	if (gb < w.gb0 || gb >= w.gb0 + WIN_B || j < w.j0 || j >= w.j0 + WIN_C) {
-		w.gb0 = max(0, gb - (WIN_B - 1));
-		w.j0 = max(0, j - (WIN_C - 1));
-		__syncwarp();  // every lane is done with the old window
-		uint4 x[WIN_B][2];  // every load in flight together
+// the warp's shared window loaded from row block w.gb0 and column w.j0 on.  Not inlined: the search
+// of a single warp waits for instructions as for everything else, so its code is kept small.
+__device__ __noinline__ void enum_load(uint4 (*win)[WIN_C], Window w, const uint4 *m, int64_t S, int lg, int ls, int lt,
+                                       int lane) {
+	__syncwarp();  // every lane is done with the old window
+	uint4 x[WIN_B][2];  // every load in flight together
 #pragma unroll
-		for (int r = 0; r < WIN_B; r++) {
-			const int g = w.gb0 + r, q = g / p.G, sb = g - q * p.G;
+	for (int r = 0; r < WIN_B; r++) {
+		const int g = w.gb0 + r, q = g >> lg, sb = g & ((1 << lg) - 1);  // G = 2^lg
 #pragma unroll
-			for (int h = 0; h < 2; h++) {
-				const int jj = w.j0 + lane + 32 * h;
-				if (jj < lt && g * R < ls) x[r][h] = m[(int64_t(q) * S + jj + sb) * p.G + sb];
-			}
+		for (int h = 0; h < 2; h++) {
+			const int jj = w.j0 + lane + 32 * h;
+			if (jj < lt && g * R < ls) x[r][h] = m[((int64_t(q) * S + jj + sb) << lg) + sb];
 		}
-#pragma unroll
-		for (int r = 0; r < WIN_B; r++)
-#pragma unroll
-			for (int h = 0; h < 2; h++)
-				if (w.j0 + lane + 32 * h < lt && (w.gb0 + r) * R < ls) win[r][lane + 32 * h] = x[r][h];
-		__syncwarp();
 	}
-	const uint4 e = win[gb - w.gb0][j - w.j0];
-	const int r = i & 7, h = r >> 1;
-	const uint32_t word = h == 0 ? e.x : h == 1 ? e.y : h == 2 ? e.z : e.w;
-	return (word >> (16 * (r & 1))) & 0xffffu;
+#pragma unroll
+	for (int r = 0; r < WIN_B; r++)
+#pragma unroll
+		for (int h = 0; h < 2; h++)
+			if (w.j0 + lane + 32 * h < lt && (w.gb0 + r) * R < ls) win[r][lane + 32 * h] = x[r][h];
+	__syncwarp();
+}
+
+// the window moved so that it holds cell (i, j) (warp-uniform)
+__device__ __forceinline__ void enum_place(uint4 (*win)[WIN_C], Window &w, const uint4 *m, int64_t S, int lg, int ls,
+                                           int lt, int i, int j, int lane) {
+	const int gb = i >> 3;
+	if (gb >= w.gb0 && gb < w.gb0 + WIN_B && j >= w.j0 && j < w.j0 + WIN_C) return;
+	w.gb0 = max(0, gb - (WIN_B - 1));
+	w.j0 = max(0, j - (WIN_C - 1));
+	enum_load(win, w, m, S, lg, ls, lt, lane);
+}
+
+// this lane's cell (i, j) where the window holds it -- it lies up and left of a cell that the
+// window holds -- and `in` says so
+__device__ __forceinline__ uint32_t enum_look(uint4 (*win)[WIN_C], const Window &w, int i, int j, bool &in) {
+	in = i >= 0 && j >= 0 && (i >> 3) >= w.gb0 && j >= w.j0;
+	if (!in) return 0u;
+	const uint32_t *e = reinterpret_cast<const uint32_t *>(&win[(i >> 3) - w.gb0][j - w.j0]);
+	return (e[(i & 7) >> 1] >> (16 * (i & 1))) & 0xffffu;
 }
 
 __device__ __forceinline__ unsigned long long enum_mix(int u, int v) {
@@ -152,6 +164,7 @@ __global__ void __launch_bounds__(32) enum_kernel(EnumParams p) {
 	int32_t *npts = p.npts + int64_t(L) * p.k;
 	const int plen_cap = ls + lt + 2;
 	Window w{-WIN_B, -WIN_C};
+	const int lg = __ffs(p.G) - 1;
 
 	int count = 0, sp = 0, si = 0, status = 0;
 	const int nseed = p.local ? p.seed_n[L] : 0;
@@ -201,15 +214,13 @@ __global__ void __launch_bounds__(32) enum_kernel(EnumParams p) {
 		bool cont = eu >= 0 && ev >= 0;
 		uint32_t c = 0;
 		if (cont) {
-			c = enum_cell(p, win, w, mk, S, ls, lt, eu, ev, lane);  // the window holds (eu, ev)
+			enum_place(win, w, mk, S, lg, ls, lt, eu, ev, lane);
 			// lane k: cell (eu - k, ev - k), while it lies in the window and its list is the diagonal
 			const int i = eu - lane, j = ev - lane;
-			bool simple = i >= 0 && j >= 0 && (i >> 3) >= w.gb0 && j >= w.j0;
-			if (simple) {
-				const uint32_t *e = reinterpret_cast<const uint32_t *>(&win[(i >> 3) - w.gb0][j - w.j0]);
-				simple = ((e[(i & 7) >> 1] >> (16 * (i & 1))) & 15u) == 2u;
-			}
-			const uint32_t b = __ballot_sync(0xffffffffu, simple);
+			bool in;
+			c = enum_look(win, w, i, j, in);
+			const uint32_t b = __ballot_sync(0xffffffffu, in && (c & 15u) == 2u);
+			c = __shfl_sync(0xffffffffu, c, 0);
 			const int run = min(b == 0xffffffffu ? 32 : __ffs(int(~b)) - 1, plen_cap - plen);
 			if (run > 0) {
 				__syncwarp();  // and may overwrite points of an earlier path
@@ -243,28 +254,62 @@ __global__ void __launch_bounds__(32) enum_kernel(EnumParams p) {
 				nv = v;
 				pend = true;
 			};
+			// the cells up the column (left along the row) where a gap that ends here may have been
+			// opened: from (eu, ev) on while the cell's extend bit is set, 32 cells a look
+			auto gap_list = [&](bool up, uint32_t open_bit, uint32_t extend_bit, int k) {
+				const int u0 = eu, v0 = ev;
+				for (;;) {
+					enum_place(win, w, mk, S, lg, ls, lt, up ? k : u0, up ? v0 : k, lane);
+					bool in;
+					const uint32_t x = enum_look(win, w, up ? k - lane : u0, up ? v0 : k - lane, in);
+					const uint32_t go = __ballot_sync(0xffffffffu, in && (x & extend_bit) && k - lane > 0);
+					const uint32_t seen = __ballot_sync(0xffffffffu, in);
+					const int n = go == 0xffffffffu ? 32 : __ffs(int(~go)) - 1;  // cells the gap goes on from
+					const bool ends = n < 32 && ((seen >> n) & 1u);              // it ends at cell n, in the window
+					const uint32_t upto = n + ends >= 32 ? 0xffffffffu : (1u << (n + ends)) - 1u;
+					uint32_t opens = __ballot_sync(0xffffffffu, (x & open_bit) != 0) & upto;
+					for (; opens; opens &= opens - 1) {
+						const int m = k - (__ffs(int(opens)) - 1) - 1;
+						add(up ? m : u0, up ? v0 : m);
+					}
+					if (ends) break;
+					k -= n;
+				}
+			};
+			// both gaps' first 16 cells in one look: lanes 0-15 up the column, 16-31 left along the row
+			uint32_t go2 = 0, open2 = 0, seen2 = 0;
+			if (p.affine && (c & 12u)) {
+				const int k = lane & 15;
+				const bool up = lane < 16;
+				bool in;
+				const uint32_t x = enum_look(win, w, up ? eu - k : eu, up ? ev : ev - k, in);
+				go2 = __ballot_sync(0xffffffffu, in && (x & (up ? 32u : 128u)) && (up ? eu : ev) - k > 0);
+				open2 = __ballot_sync(0xffffffffu, (x & (up ? 16u : 64u)) != 0);
+				seen2 = __ballot_sync(0xffffffffu, in);
+			}
+			auto near_list = [&](bool up) {
+				const uint32_t go = (up ? go2 : go2 >> 16) & 0xffffu, seen = up ? seen2 : seen2 >> 16;
+				const int n = __ffs(int(~go)) - 1;  // at most 16
+				const bool ends = n < 16 && ((seen >> n) & 1u);
+				uint32_t opens = (up ? open2 : open2 >> 16) & ((1u << (n + ends)) - 1u);
+				for (; opens; opens &= opens - 1) {
+					const int m = __ffs(int(opens));
+					add(up ? eu - m : eu, up ? ev : ev - m);
+				}
+				if (!ends) gap_list(up, up ? 16u : 64u, up ? 32u : 128u, (up ? eu : ev) - n);
+			};
 			if (c & 1u) add(ENUM_NO_TB, ENUM_NO_TB);
 			if (c & 2u) add(eu - 1, ev - 1);
 			if (c & 4u) {
 				if (p.affine) {
-					for (int k = eu;; k--) {
-						const uint32_t ck = k == eu ? c : enum_cell(p, win, w, mk, S, ls, lt, k, ev, lane);
-						if (ck & 16u) add(k - 1, ev);
-						if ((ck & 32u) && k > 0) continue;
-						break;
-					}
+					near_list(true);
 				} else {
 					add(eu - 1, ev);
 				}
 			}
 			if (c & 8u) {
 				if (p.affine) {
-					for (int k = ev;; k--) {
-						const uint32_t ck = k == ev ? c : enum_cell(p, win, w, mk, S, ls, lt, eu, k, lane);
-						if (ck & 64u) add(eu, k - 1);
-						if ((ck & 128u) && k > 0) continue;
-						break;
-					}
+					near_list(false);
 				} else {
 					add(eu, ev - 1);
 				}
@@ -362,8 +407,10 @@ __global__ void __launch_bounds__(32) enum_kernel(EnumParams p) {
 			}
 		}
 		if (dup) continue;
-		if (SM)
+		if (SM) {
+#pragma unroll 8
 			for (int x = lane; x < m; x += 32) mp[x] = smap[x];
+		}
 		if (lane == 0) {
 			hash[count] = h;
 			npts[count] = n;
