@@ -24,8 +24,8 @@
 // memory, and (N, Qc) of each row stay in registers along the row.  Counts are uint64,
 // exact below 2^64 and saturating at 2^64 - 1.
 //
-// Few long pairs (masks written with G = 32): path_count_chain_kernel gives every 256-row
-// stripe of every pair to its own warp, like the DP's stripe-chained mode -- tickets numbered
+// Few long pairs (masks written with G = 32 or 16): path_count_chain_kernel gives every 256-row
+// (128-row) stripe of every pair to its own warp, like the DP's stripe-chained mode -- tickets numbered
 // stripe-major (stripe q of the pair at rank w is ticket level_start[q] + w), the warp of
 // stripe q reading the boundary row of stripe q - 1 while that stripe's warp still writes
 // it, behind a progress counter published every 32 columns (bounded waits: past the limit
@@ -225,8 +225,10 @@ __global__ void __launch_bounds__(BLOCK) path_count_kernel(CountParams p) {
 	}
 }
 
+// G: the width of the masks' groups, 32 or (stripes of 128 rows) 16, then half of the lanes idle
+template <int G>
 __global__ void __launch_bounds__(BLOCK) path_count_chain_kernel(CountParams p) {
-	constexpr int G = 32, rpp = G * R;
+	constexpr int rpp = G * R;
 	const int lane = threadIdx.x & 31;
 	const int sub = lane;
 	for (;;) {
@@ -263,7 +265,7 @@ __global__ void __launch_bounds__(BLOCK) path_count_chain_kernel(CountParams p) 
 		const uint4 zero4 = make_uint4(0u, 0u, 0u, 0u);
 		auto load = [&](int st) -> uint4 {
 			const int jj = st - sub;
-			return (pass_active && jj >= 0 && jj < lt) ? __ldg(M + (int64_t(q) * S + st) * G + sub) : zero4;
+			return (pass_active && sub < G && jj >= 0 && jj < lt) ? __ldg(M + (int64_t(q) * S + st) * G + sub) : zero4;
 		};
 		// lane 0: the boundary row of column col, once the stripe above has published it
 		auto load_row = [&](int col) -> ulonglong2 {
@@ -287,7 +289,7 @@ __global__ void __launch_bounds__(BLOCK) path_count_chain_kernel(CountParams p) 
 			const int j = s - sub;
 			unsigned long long upN = shfl_up64(outN, G);
 			unsigned long long upP = shfl_up64(outP, G);
-			if (j >= 0 && j < lt) {
+			if (sub < G && j >= 0 && j < lt) {
 				if (sub == 0) {
 					upN = bcur.x;
 					upP = bcur.y;
@@ -549,7 +551,8 @@ __global__ void __launch_bounds__(32 * NW) path_count_band_kernel(BandParams p) 
 }
 
 cudaError_t launch_path_count(const CountParams &p, int grid, cudaStream_t st) {
-	if (p.ntickets > 0) path_count_chain_kernel<<<grid, BLOCK, 0, st>>>(p);
+	if (p.ntickets > 0 && p.G == 16) path_count_chain_kernel<16><<<grid, BLOCK, 0, st>>>(p);
+	else if (p.ntickets > 0) path_count_chain_kernel<32><<<grid, BLOCK, 0, st>>>(p);
 	else path_count_kernel<<<grid, BLOCK, 0, st>>>(p);
 	return cudaGetLastError();
 }

@@ -442,7 +442,12 @@ __device__ __forceinline__ void finish_pair(const DpParams<V> &p, int G, int sub
 	}
 }
 
-template <typename V, int GAP, int LOC, int TB, bool VALS, bool CHAIN>
+// RR: rows per lane.  4 instead of 8 (CHAIN, all-optimal int32 masks in the layout of G = 16, where
+// two lanes write the halves of a word): a stripe of 128 rows on its warp, half the dependent cells
+// a step at the cost of twice the stripes, each 64 columns and a hand-over behind the one above.
+// Where the 256-row stripes would leave schedulers empty a step's chain is the time: 16 pairs of
+// 2000..3000 x 3000..5000 2.93 -> 2.49 ms.
+template <typename V, int GAP, int LOC, int TB, bool VALS, bool CHAIN, int RR>
 __global__ void __launch_bounds__(BLOCK, 4) dp_kernel(DpParams<V> p) {
 	constexpr bool ISINT = std::is_same<V, int32_t>::value;
 	constexpr bool TAG = ISINT && TB != TB_ALL;  // int32 tagged values
@@ -467,7 +472,8 @@ __global__ void __launch_bounds__(BLOCK, 4) dp_kernel(DpParams<V> p) {
 	__shared__ V2 chunk_all[CHAIN ? WARPS : 1][CHAIN ? PUB_CHUNK : 1];
 	V2 *const chunk = chunk_all[CHAIN ? threadIdx.x >> 5 : 0];
 
-	const int G = p.G;
+	const int G = RR == R ? p.G : 32;
+	static_assert(RR == R || (RR == 4 && CHAIN && TB == TB_ALL), "8 rows per lane, or 4 of all-optimal stripes");
 	const int lane = threadIdx.x & 31;
 	const int sub = lane % G;          // lane within the group
 	const int grp = lane / G;          // group within the warp
@@ -476,7 +482,7 @@ __global__ void __launch_bounds__(BLOCK, 4) dp_kernel(DpParams<V> p) {
 	const int slot = warp_global * gpw + grp;
 	const int64_t half = p.scratch_stride / 2;
 	const V NEG = p.neg_inf;
-	const int rpp = G * R;  // rows per pass
+	const int rpp = G * RR;  // rows per pass
 	const int sub_kind = p.sub_kind;
 	constexpr bool units = CHAIN;  // stripe-chained mode (G == 32)
 	int cursor = -2;
@@ -560,8 +566,8 @@ __global__ void __launch_bounds__(BLOCK, 4) dp_kernel(DpParams<V> p) {
 		const int q_hi = units ? min(q_lo + 1, npass) : wpass;
 		for (int q = q_lo; q < q_hi; q++) {
 			const bool pass_active = q < npass;
-			const int row0 = q * rpp + sub * R;
-			const int nvalid = ls - row0;  // rows of this lane that are < ls (may be <= 0 or >= R)
+			const int row0 = q * rpp + sub * RR;
+			const int nvalid = ls - row0;  // rows of this lane that are < ls (may be <= 0 or >= RR)
 			const V2 *bin = scr + (q & 1) * half;
 			V2 *bout = scr + ((q + 1) & 1) * half;
 			const bool write_boundary = sub == G - 1 && q + 1 < npass;
@@ -607,10 +613,10 @@ __global__ void __launch_bounds__(BLOCK, 4) dp_kernel(DpParams<V> p) {
 			bool ahead = false;  // `above` holds the next chunk
 
 			// query codes, and the int8 substitution profile of each row (SUB_PROFILE)
-			uint32_t qa[R];
-			uint32_t plo[R], phi[R];
+			uint32_t qa[RR];
+			uint32_t plo[RR], phi[RR];
 #pragma unroll
-			for (int r = 0; r < R; r++) {
+			for (int r = 0; r < RR; r++) {
 				const int i = row0 + r;
 				qa[r] = (pass_active && i < ls && arow) ? arow[i] : 0u;
 				plo[r] = phi[r] = 0u;
@@ -620,7 +626,7 @@ __global__ void __launch_bounds__(BLOCK, 4) dp_kernel(DpParams<V> p) {
 				for (int c = 0; c < cols; c++) {
 					uint32_t lo = 0, hi = 0;
 #pragma unroll
-					for (int r = 0; r < R; r++) {
+					for (int r = 0; r < RR; r++) {
 						const uint32_t byte = uint32_t(int32_t(tab[qa[r] * cols + c])) & 0xffu;
 						if (r < 4) lo |= byte << (8 * r);
 						else hi |= byte << (8 * (r - 4));
@@ -630,7 +636,7 @@ __global__ void __launch_bounds__(BLOCK, 4) dp_kernel(DpParams<V> p) {
 			} else if (sub_kind == SUB_PROFILE) {
 				const int cols = p.table_cols;
 #pragma unroll
-				for (int r = 0; r < R; r++) {
+				for (int r = 0; r < RR; r++) {
 					uint32_t lo = 0, hi = 0;
 					for (int c = 0; c < cols; c++) {
 						const uint32_t byte = uint32_t(int32_t(tab[qa[r] * cols + c])) & 0xffu;
@@ -642,32 +648,32 @@ __global__ void __launch_bounds__(BLOCK, 4) dp_kernel(DpParams<V> p) {
 				}
 			}
 
-			V Dl[R], Ql[R];
+			V Dl[RR], Ql[RR];
 #pragma unroll
-			for (int r = 0; r < R; r++) {
+			for (int r = 0; r < RR; r++) {
 				const int i = row0 + r;
 				Dl[r] = (pass_active && i < ls) ? p.left_D[i + 1] : NEG;
 				Ql[r] = NEG;
 			}
 			// (D, P) of this lane's last row as seen by the next lane; column -1 initially
-			V outD = Dl[R - 1], outP = NEG;
+			V outD = Dl[RR - 1], outP = NEG;
 			V prev_up = (pass_active && row0 <= ls) ? p.left_D[row0] : NEG;  // D(row0-1, -1)
 
 			// best cell per row for local one-optimal seeds (solver.h:2048-2056)
-			constexpr int NB = (TB == TB_ONE && LOC == LOC_LOCAL) ? R : 1;
+			constexpr int NB = (TB == TB_ONE && LOC == LOC_LOCAL) ? RR : 1;
 			V bv[NB];
 			int bj[NB];
 #pragma unroll
 			for (int r = 0; r < NB; r++) { bv[r] = KEYSEED ? V(-1) : NEG; bj[r] = -1; }
 			const int kshift = p.key_shift;
 			const int kmul = 1 << kshift;
-			const bool last_row_lane = pass_active && nvalid >= 1 && nvalid <= R;
+			const bool last_row_lane = pass_active && nvalid >= 1 && nvalid <= RR;
 			const int r_last = nvalid - 1;
 
 			uint32_t tnext = (pass_active && brow) ? brow[0] : 0u;  // code of column 0 (lt >= 1 here)
 			// dense S with stride 1 along s: a lane whose 8 rows all lie in the pair reads them as
 			// two 16-byte loads, one column ahead of its use (drow + row0 + j * sj)
-			const bool dvec = sub_kind == SUB_DENSE && pass_active && nvalid >= R && p.dense_si == 1 &&
+			const bool dvec = RR == R && sub_kind == SUB_DENSE && pass_active && nvalid >= RR && p.dense_si == 1 &&
 			                  (p.dense_sj & 3) == 0 && ((reinterpret_cast<uintptr_t>(drow) & 15) == 0);
 			const float *dcol = dvec ? drow + row0 : nullptr;
 			// column jj's 8 rows into ring slot jj % DENSE_RING, one commit group per column (an
@@ -687,9 +693,13 @@ __global__ void __launch_bounds__(BLOCK, 4) dp_kernel(DpParams<V> p) {
 			// this lane's traceback word of step s is mrow[s * G] (hoisted out of the step loop)
 			uint32_t *mrow1 = nullptr;
 			uint4 *mrow4 = nullptr;
+			uint2 *mrow2 = nullptr;  // RR = 4: of column 0
 			if (TB == TB_ONE && pass_active)
 				mrow1 = reinterpret_cast<uint32_t *>(p.masks) + p.mask_off[pair] + int64_t(q) * nsteps_pair * G + sub;
-			if (TB == TB_ALL && pass_active)
+			if (RR == 4 && pass_active)
+				mrow2 = reinterpret_cast<uint2 *>(p.masks) +
+				        2 * (p.mask_off[pair] + (int64_t(q) * (lt + 15) + (sub >> 1)) * 16 + (sub >> 1)) + (sub & 1);
+			else if (TB == TB_ALL && pass_active)
 				mrow4 = reinterpret_cast<uint4 *>(p.masks) + p.mask_off[pair] + int64_t(q) * nsteps_pair * G + sub;
 			for (int s = 0; s < wsteps; s++) {
 				const int j = s - sub;
@@ -721,26 +731,26 @@ __global__ void __launch_bounds__(BLOCK, 4) dp_kernel(DpParams<V> p) {
 					}
 				}
 				if (act) {
-					// substitution values of the R rows at column j
-					V S[R];
+					// substitution values of the RR rows at column j
+					V S[RR];
 					if (sub_kind == SUB_COLPROF) {
 						const uint2 pr = colprof[tcode * BLOCK + threadIdx.x];
 #pragma unroll
-						for (int r = 0; r < R; r++) S[r] = V(prmt(pr.x, pr.y, sext_selector(uint32_t(r))));
+						for (int r = 0; r < RR; r++) S[r] = V(prmt(pr.x, pr.y, sext_selector(uint32_t(r))));
 					} else if (sub_kind == SUB_PROFILE) {
 						const uint32_t sel = sext_selector(tcode);
 #pragma unroll
-						for (int r = 0; r < R; r++) S[r] = V(prmt(plo[r], phi[r], sel));
+						for (int r = 0; r < RR; r++) S[r] = V(prmt(plo[r], phi[r], sel));
 					} else if (sub_kind == SUB_BINARY) {
 #pragma unroll
-						for (int r = 0; r < R; r++) S[r] = (qa[r] == tcode) ? p.eq : p.ne;
+						for (int r = 0; r < RR; r++) S[r] = (qa[r] == tcode) ? p.eq : p.ne;
 					} else if (sub_kind == SUB_TABLE) {
 #pragma unroll
-						for (int r = 0; r < R; r++) S[r] = tab[qa[r] * p.table_cols + tcode];
+						for (int r = 0; r < RR; r++) S[r] = tab[qa[r] * p.table_cols + tcode];
 					} else if (sub_kind == SUB_SERIES) {
 						const float yj = __int_as_float(int(tcode));
 #pragma unroll
-						for (int r = 0; r < R; r++) S[r] = V(fabsf(__int_as_float(int(qa[r])) - yj) * p.dense_sign);
+						for (int r = 0; r < RR; r++) S[r] = V(fabsf(__int_as_float(int(qa[r])) - yj) * p.dense_sign);
 					} else if (dvec) {
 						// column j's group is complete once at most DENSE_RING - 2 newer ones remain;
 						// the refill goes to the slot read in the previous step
@@ -751,24 +761,24 @@ __global__ void __launch_bounds__(BLOCK, 4) dp_kernel(DpParams<V> p) {
 						S[1] = V(dn0.y * p.dense_sign);
 						S[2] = V(dn0.z * p.dense_sign);
 						S[3] = V(dn0.w * p.dense_sign);
-						S[4] = V(dn1.x * p.dense_sign);
-						S[5] = V(dn1.y * p.dense_sign);
-						S[6] = V(dn1.z * p.dense_sign);
-						S[7] = V(dn1.w * p.dense_sign);
+						S[4 % RR] = V(dn1.x * p.dense_sign);
+						S[5 % RR] = V(dn1.y * p.dense_sign);
+						S[6 % RR] = V(dn1.z * p.dense_sign);
+						S[7 % RR] = V(dn1.w * p.dense_sign);
 					} else {
 #pragma unroll
-						for (int r = 0; r < R; r++) {
+						for (int r = 0; r < RR; r++) {
 							const int i = min(row0 + r, ls - 1);
 							S[r] = V(drow[int64_t(i) * p.dense_si + int64_t(j) * p.dense_sj] * p.dense_sign);
 						}
 					}
 
-					uint32_t mword = 0;  // one-optimal traceback nibbles of the R rows
+					uint32_t mword = 0;  // one-optimal traceback nibbles of the RR rows
 					uint32_t mall[4] = {0, 0, 0, 0};
 					V dsave = prev_up;  // D(i-1, j-1) for the first row
 					V uD = upD, uP = upP;
 #pragma unroll
-					for (int r = 0; r < R; r++) {
+					for (int r = 0; r < RR; r++) {
 						const V old = Dl[r];
 						V D, P = NEG, Q = NEG;
 						if (TAG) {
@@ -785,7 +795,7 @@ __global__ void __launch_bounds__(BLOCK, 4) dp_kernel(DpParams<V> p) {
 								const int32_t code = key & 3;
 								D = imad(code, p.minus_one, key);
 								if (TB == TB_ONE) {
-									// nibble code | P-extend << 2 | Q-extend << 3, row r at bits 4(R-1-r)
+									// nibble code | P-extend << 2 | Q-extend << 3, row r at bits 4(RR-1-r)
 									int32_t nb = imad(int32_t(gt_mask(P, oP)), p.minus_four, code);
 									nb = imad(int32_t(gt_mask(Q, oQ)), p.minus_eight, nb);
 									mword = uint32_t(imad(int32_t(mword), p.sixteen, nb));
@@ -946,6 +956,8 @@ __global__ void __launch_bounds__(BLOCK, 4) dp_kernel(DpParams<V> p) {
 
 					if (TB == TB_ONE) {
 						mrow1[s * G] = mword;
+					} else if (RR == 4) {
+						mrow2[int64_t(j) * 32] = make_uint2(mall[0], mall[1]);
 					} else if (TB == TB_ALL) {
 						mrow4[s * G] = make_uint4(mall[0], mall[1], mall[2], mall[3]);
 					}
@@ -954,7 +966,7 @@ __global__ void __launch_bounds__(BLOCK, 4) dp_kernel(DpParams<V> p) {
 						if (last_row_lane && q == npass - 1) {
 							V x = Dl[0];
 #pragma unroll
-							for (int r = 1; r < R; r++)
+							for (int r = 1; r < RR; r++)
 								if (r == r_last) x = Dl[r];
 							if (LOC == LOC_SEMI) {
 								if (x > row_best) { row_best = x; row_bj = j; }
@@ -965,7 +977,7 @@ __global__ void __launch_bounds__(BLOCK, 4) dp_kernel(DpParams<V> p) {
 						}
 						if (LOC == LOC_SEMI && j == lt - 1) {
 #pragma unroll
-							for (int r = 0; r < R; r++)
+							for (int r = 0; r < RR; r++)
 								if (r < nvalid && Dl[r] > col_best) { col_best = Dl[r]; col_bi = row0 + r; }
 						}
 					}

@@ -150,6 +150,7 @@ struct ResultData {
 	int method = 0;
 	float sign = 1.0f;
 	int G = 32;
+	bool units = false;  // the masks were written stripe by stripe
 	float worst = -INFINITY;
 	std::vector<float> scores;
 	std::vector<int32_t> has;     // has_alignment per lane
@@ -2542,6 +2543,14 @@ pa_status solve_impl(pa_solver *s, const Input &in, int method, float *scores_ou
 		// host buffers and many pairs: the repeats of this solve run as a pipeline of chunks
 		// (3 chunks from 32K pairs, 2 from 8K; PA_CHUNKS overrides, up to 12); host maps use
 		// the packed offsets (checked above)
+		if (tb == TB_ALL && plan.units && plan.use_int && !want_values && s->loc != LOC_LOCAL) {
+			// all-optimal stripes of 128 rows (dp_kernel, RR = 4) while 256-row stripes would not give
+			// every scheduler a warp.  PA_DP_ROWS=8 turns it off (tests)
+			int64_t stripes = 0;
+			for (int32_t a : ls) stripes += (a + 32 * R - 1) / (32 * R);
+			const char *e = std::getenv("PA_DP_ROWS");
+			if (stripes <= int64_t(s->sm_count) * 4 && !(e && std::atoi(e) == 8)) plan.G = 16;
+		}
 		plan.nchunks = 1;
 		if (repeatable && in.location == PA_HOST && in.form != F_DENSE && !plan.units && !want_paths) {
 			int K = B >= 32768 ? 3 : B >= 8192 ? 2 : 1;
@@ -2553,6 +2562,7 @@ pa_status solve_impl(pa_solver *s, const Input &in, int method, float *scores_ou
 		if (pa_status e = device_work(st, true)) return e;
 	}
 	res.G = plan.G;
+	res.units = plan.units;
 	s->last_plan[0] = s->gap == GAP_GENERAL ? 4
 	                  : plan.s16 && !plan.units ? 5
 	                  : plan.h16  ? (plan.blk ? 6 : plan.C == 2 ? 5 : 3)
@@ -3551,19 +3561,20 @@ pa_status pa_result_path_counts(const pa_result *r, uint64_t *counts) {
 		PA_CUDA(cudaMemcpy(dm.p, d.mask_off.data(), size_t(B) * 8, cudaMemcpyHostToDevice));
 		PA_CUDA(cudaMemcpy(dseed.p, seed.data(), size_t(2 * B) * 4, cudaMemcpyHostToDevice));
 		PA_CUDA(cudaMemset(dctr.p, 0, 4));
-		// few long pairs written with G = 32: a warp per 256-row stripe, stripes chained
-		const int64_t rpp32 = 32 * R;
+		// few long pairs written with G = 32 or 16: a warp per stripe, stripes chained
+		const bool wide = d.G == 32 || (d.G == 16 && d.units);
+		const int64_t rpp32 = int64_t(d.G) * R;
 		int64_t max_np = 0;
 		for (int64_t k = 0; k < B; k++)
 			if (d.ls[size_t(k)] > 0 && d.lt[size_t(k)] > 0)
 				max_np = std::max<int64_t>(max_np, (d.ls[size_t(k)] + rpp32 - 1) / rpp32);
-		bool chain = d.G == 32 && max_np >= 3;
+		bool chain = wide && max_np * rpp32 >= 3 * 256;
 		// one seed per pair (not local alignment): along the band of its co-optimal paths, which is
 		// the faster at every size measured, 64 x 64 to 4000 x 4000, one pair to 4000 (pa_count.cu)
 		std::vector<int32_t> ls_left(d.ls.begin(), d.ls.end()), lt_left(d.lt.begin(), d.lt.end());
 		bool band = !local;
-		if (const char *e = std::getenv("PA_COUNT_MODE")) {  // tests: "group" or "chain" (G = 32 only)
-			chain = std::strcmp(e, "chain") == 0 ? d.G == 32 : std::strcmp(e, "group") == 0 ? false : chain;
+		if (const char *e = std::getenv("PA_COUNT_MODE")) {  // tests: "group" or "chain" (G = 32 or 16)
+			chain = std::strcmp(e, "chain") == 0 ? wide : std::strcmp(e, "group") == 0 ? false : chain;
 			band = false;
 		}
 		std::vector<uint64_t> c(static_cast<size_t>(B), 0);
@@ -3636,7 +3647,7 @@ pa_status pa_result_path_counts(const pa_result *r, uint64_t *counts) {
 			PA_CUDA(cudaMemset(dprog.p, 0, size_t(nt) * 4));
 			PA_CUDA(cudaMemset(dstat.p, 0, 4));
 			const int64_t grid = std::max<int64_t>(1, std::min<int64_t>(int64_t(sms) * 4, (nt + WARPS - 1) / WARPS));
-			PA_CUDA(pa::path_count_solve(int32_t(B), 32, local ? 1 : 0, d.gap == GAP_AFFINE ? 1 : 0, dl.as<int32_t>(),
+			PA_CUDA(pa::path_count_solve(int32_t(B), d.G, local ? 1 : 0, d.gap == GAP_AFFINE ? 1 : 0, dl.as<int32_t>(),
 			                             dl.as<int32_t>() + B, dm.as<int64_t>(), d.dev_masks_all, dseed.as<int32_t>(),
 			                             dcnt.as<unsigned long long>(), dscr.as<unsigned long long>(), stride,
 			                             dctr.as<int32_t>(), int(grid), nullptr, int32_t(nt), int32_t(nlev),

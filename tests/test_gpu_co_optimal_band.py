@@ -49,17 +49,18 @@ def _long_pairs(rng, letters):
 @pytest.mark.parametrize("letters", [2, 4])
 @pytest.mark.parametrize("locality", ["global", "semiglobal"])
 @pytest.mark.parametrize("gap", ["linear", "affine", "free"])
-@pytest.mark.parametrize("mode", ["G8", "chained"])
+@pytest.mark.parametrize("mode", ["G8", "chained", "chained8"])  # stripes of 128 and of 256 rows
 def test_band_counts_equal_whole_matrix_counts(monkeypatch, gpu_alg, letters, locality, gap, mode):  # noqa: F811
-    if mode == "chained":
+    if mode.startswith("chained"):
         monkeypatch.setenv("PA_DP_MODE", "units")
+        monkeypatch.setenv("PA_DP_ROWS", mode[7:] or "4")
     else:
         monkeypatch.setenv("PA_GROUP_WIDTH", mode[1:])
     pairs = _long_pairs(np.random.default_rng(77 + letters), letters)
     table = (3.0 * np.eye(letters) - 1.0).astype(np.float32)
     g = {"linear": Gap("linear", 1.0), "affine": Gap("affine", 2.0, 1.0), "free": Gap("affine", 0.0, 0.0)}[gap]
     got = {}
-    for how in ("group", None):
+    for how in ("group", "chain", None):
         if how:
             monkeypatch.setenv("PA_COUNT_MODE", how)
         else:
@@ -67,6 +68,7 @@ def test_band_counts_equal_whole_matrix_counts(monkeypatch, gpu_alg, letters, lo
         _, its, _, _, _, _ = _solve(gpu_alg, pairs, locality, g, "maximize", False, table)
         got[how] = [it.path_count() for it in its]
     assert got[None] == got["group"]
+    assert got["chain"] == got["group"]
 
 
 @pytest.mark.parametrize("locality", ["global", "semiglobal", "local"])
