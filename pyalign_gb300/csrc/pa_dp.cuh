@@ -1021,7 +1021,7 @@ __global__ void dense_copy_kernel(const float *src, const int64_t *src_off, int6
 
 // Largest code in a batch of sequences (host validation of the indexed form,
 // factory.h:602-614, done on the device for device-resident inputs).
-__global__ void codes_max_kernel(const uint32_t *x, int64_t n, uint32_t *out);
+__global__ void codes_max_kernel(const uint32_t *a, int64_t na, const uint32_t *b, int64_t nb, uint32_t *out);
 
 // ---------------------------------------------------------------------------------------
 // Traceback walk for one optimal path (TracebackIterators<false>::Iterator::next,

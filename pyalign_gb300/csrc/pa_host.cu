@@ -71,6 +71,13 @@ struct DevBuf {
 	T *as() const { return reinterpret_cast<T *>(p); }
 };
 
+// A part of a DevBuf.
+struct DevView {
+	void *p = nullptr;
+	template <typename T>
+	T *as() const { return reinterpret_cast<T *>(p); }
+};
+
 struct PinBuf {
 	void *p = nullptr;
 	size_t cap = 0;
@@ -382,10 +389,21 @@ struct pa_solver {
 	int32_t last_widths[4] = {0, 0, 0, 0};  // group width per length bucket (0: one width)
 	int64_t bytes_h2d = 0, bytes_d2h = 0;
 
-	DevBuf d_a, d_b, d_tab, d_dense, d_dense_off, d_ls, d_lt, d_order, d_mask_off, d_score, d_seed, d_has,
-	    d_masks, d_scratch, d_counter, d_status, d_border, d_maps, d_map_off, d_paths, d_path_off,
+	DevBuf d_a, d_b, d_tab, d_dense, d_dense_off, d_ls, d_lt, d_order, d_mask_off, d_out,
+	    d_masks, d_scratch, d_counter, d_border, d_maps, d_map_off, d_paths, d_path_off,
 	    d_path_len, d_vals, d_val_off, d_best, d_gen, d_wsb_off, d_wsb_tb, d_wsb_vals, d_wsb_vals_t, d_wsb_sub,
 	    d_wsb_sub_off, d_codes_max, d_progress, d_chain;
+	// what a solve hands back to the host, in d_out: the status word, scores, has-seed flags, seeds
+	DevView d_status, d_score, d_has, d_seed;
+	cudaError_t ensure_out(int64_t B) {
+		if (cudaError_t e = d_out.ensure(16 + size_t(B) * 16)) return e;
+		unsigned char *b = d_out.as<unsigned char>();
+		d_status.p = b + 12;
+		d_score.p = b + 16;
+		d_has.p = b + 16 + size_t(B) * 4;
+		d_seed.p = b + 16 + size_t(B) * 8;
+		return cudaSuccess;
+	}
 	PinBuf h_stage, h_out;
 	// per-call pair metadata, staged in one pinned buffer and sent with one copy
 	DevBuf d_meta;
@@ -739,6 +757,22 @@ int choose_G(const std::vector<int32_t> &ls, const std::vector<int32_t> &lt, int
 	for (size_t k = 0; k < B; k++) pairs += int64_t(a[k] > 0) & int64_t(b[k] > 0);
 	double best = 0;
 	int bestG = 32;
+	if (pairs < int64_t(sm_count) * 4) {
+		// fewer pairs than schedulers: what counts is the longest pair, stripes times columns and the
+		// skew of the group's lanes (8 pairs of 8..40 letters, float: G = 32 19 us, G = 8 12 us)
+		int64_t least = INT64_MAX;
+		for (int c = 0; c < 6; c++) {
+			const int64_t G = cand[c];
+			int64_t chain = 0;
+			for (size_t k = 0; k < B; k++)
+				if (a[k] > 0 && b[k] > 0) chain = std::max<int64_t>(chain, (a[k] + G * R - 1) / (G * R) * (b[k] + G - 1));
+			if (chain < least) {
+				least = chain;
+				bestG = int(G);
+			}
+		}
+		return bestG;
+	}
 	for (int c = 0; c < 6; c++) {
 		const int G = cand[c];
 		const uint32_t rpp = uint32_t(G) * R;  // a power of two
@@ -1954,10 +1988,10 @@ pa_status solve_impl(pa_solver *s, const Input &in, int method, float *scores_ou
 		const uint32_t *da = in.location == PA_DEVICE ? in.a : s->d_a.as<uint32_t>();
 		const uint32_t *db = in.location == PA_DEVICE ? in.b : s->d_b.as<uint32_t>();
 		const int grid = std::max(1, std::min(s->sm_count * 4, int((B * std::max(in.n_s, in.n_t) + 255) / 256)));
-		if (B * in.n_s > 0) codes_max_kernel<<<grid, 256, 0, st>>>(da, B * in.n_s, s->d_codes_max.as<uint32_t>());
-		if (B * in.n_t > 0) codes_max_kernel<<<grid, 256, 0, st>>>(db, B * in.n_t, s->d_codes_max.as<uint32_t>() + 1);
+		if (B * in.n_s > 0 || B * in.n_t > 0)
+			codes_max_kernel<<<dim3(grid, 2), 256, 0, st>>>(da, B * in.n_s, db, B * in.n_t, s->d_codes_max.as<uint32_t>());
 		PA_CUDA(cudaGetLastError());
-		launches += int(B * in.n_s > 0) + int(B * in.n_t > 0);
+		launches += B * in.n_s > 0 || B * in.n_t > 0;
 		// no wait here: the DP kernels read the maxima at launch and do nothing (ST_BAD_CODE)
 		// when a code is out of bounds; the error is raised after the solve's one sync
 	}
@@ -2014,11 +2048,12 @@ pa_status solve_impl(pa_solver *s, const Input &in, int method, float *scores_ou
 			if (std::atoi(e) == 1) plan.C32 = 1;
 		plan.C = cols_of(plan, plan.units);
 		int32_t hneg = 0;
-		plan.h16 = !plan.units && h16_plan(s, in, host_table.data(), ls, lt, tb, want_values, use_int, &hneg);
-		plan.h_neg = hneg;
-		// (one traceback: small launches in int32, see S16_SURE_CELLS; PA_DP16=all for tests)
 		const char *all16 = std::getenv("PA_DP16");
-		const bool large = double(cells_sum) >= TUNE_MIN_CELLS || (all16 && std::strcmp(all16, "all") == 0);
+		const bool all = all16 && std::strcmp(all16, "all") == 0;
+		plan.h16 = !plan.units && !(all && tb == TB_ONE) && h16_plan(s, in, host_table.data(), ls, lt, tb, want_values, use_int, &hneg);
+		plan.h_neg = hneg;
+		// (one traceback: small launches in int32, see S16_SURE_CELLS; PA_DP16=all for tests, DNA included)
+		const bool large = double(cells_sum) >= TUNE_MIN_CELLS || all;
 		plan.s16 = !(tb == TB_ONE && (plan.h16 || !large)) && s16_plan(s, in, host_table.data(), max_ls, max_lt, want_values, plan);
 		if (plan.h16) plan.C = plan.C32;  // two columns per step unless PA_DP_COLS=1
 		if (const char *e = std::getenv("PA_DP_BLOCK"))  // experiments and tests: the 4 x 4 block kernel
@@ -2214,10 +2249,7 @@ pa_status solve_impl(pa_solver *s, const Input &in, int method, float *scores_ou
 			PA_CUDA(cudaEventRecord(s->meta_ev, st));
 			s->meta_pending = true;
 		}
-		PA_CUDA(s->d_score.ensure(size_t(B) * 4));
-		PA_CUDA(s->d_seed.ensure(size_t(B) * 8));
-		PA_CUDA(s->d_has.ensure(size_t(B) * 4));
-		PA_CUDA(s->d_status.ensure(4));
+		PA_CUDA(s->ensure_out(B));
 		PA_CUDA(cudaMemsetAsync(s->d_status.p, 0, 4, st));
 		const size_t mask_elem = tb == TB_ALL ? 16 : 4;
 		if (tb != TB_NONE) PA_CUDA(s->d_masks.ensure(size_t(mask_off[size_t(B)]) * mask_elem));
@@ -2421,8 +2453,9 @@ pa_status solve_impl(pa_solver *s, const Input &in, int method, float *scores_ou
 				PA_CUDA(cudaMemsetAsync(mx, 0, 8, sc));
 				const int64_t na = (k1 - k0) * in.n_s, nb = (k1 - k0) * in.n_t;
 				const int grid = std::max(1, std::min(s->sm_count * 4, int((std::max(na, nb) + 255) / 256)));
-				if (na > 0) codes_max_kernel<<<grid, 256, 0, sc>>>(s->d_a.as<uint32_t>() + k0 * in.n_s, na, mx);
-				if (nb > 0) codes_max_kernel<<<grid, 256, 0, sc>>>(s->d_b.as<uint32_t>() + k0 * in.n_t, nb, mx + 1);
+				if (na > 0 || nb > 0)
+					codes_max_kernel<<<dim3(grid, 2), 256, 0, sc>>>(s->d_a.as<uint32_t>() + k0 * in.n_s, na,
+					                                                s->d_b.as<uint32_t>() + k0 * in.n_t, nb, mx);
 				PA_CUDA(cudaGetLastError());
 				launches += int(na > 0) + int(nb > 0);
 			}
@@ -2651,15 +2684,11 @@ pa_status solve_impl(pa_solver *s, const Input &in, int method, float *scores_ou
 	// ---- download: the status word, and the per-pair scores and seeds where the host needs
 	// them (a result object, or host scores), through the solver's pinned block
 	const bool host_scores = out != nullptr || scores_out != nullptr || (goal == GOAL_ALL && method == M_SCORE);
+	// (they lie behind one another, in one copy: four cost 8 word pairs 9 us of 84)
 	const size_t hb = 16 + (host_scores ? size_t(B) * 4 : 0) + (out ? size_t(B) * 12 : 0);
 	PA_CUDA(s->h_out.ensure(hb));
 	unsigned char *hp = s->h_out.as<unsigned char>();
-	PA_CUDA(pa_copy(s, hp, s->d_status.p, 4, cudaMemcpyDeviceToHost, st));
-	if (host_scores) PA_CUDA(pa_copy(s, hp + 16, s->d_score.p, size_t(B) * 4, cudaMemcpyDeviceToHost, st));
-	if (out) {
-		PA_CUDA(pa_copy(s, hp + 16 + size_t(B) * 4, s->d_has.p, size_t(B) * 4, cudaMemcpyDeviceToHost, st));
-		PA_CUDA(pa_copy(s, hp + 16 + size_t(B) * 8, s->d_seed.p, size_t(B) * 8, cudaMemcpyDeviceToHost, st));
-	}
+	PA_CUDA(pa_copy(s, hp + 12, s->d_status.p, hb - 12, cudaMemcpyDeviceToHost, st));
 	if (out) {
 		res.map_off = map_off;
 		res.mask_off = mask_off;
@@ -2709,7 +2738,7 @@ pa_status solve_impl(pa_solver *s, const Input &in, int method, float *scores_ou
 	s->dp_timing_pending = false;
 	s->last_launches = launches;
 	int32_t status = 0;
-	std::memcpy(&status, hp, 4);
+	std::memcpy(&status, hp + 12, 4);
 	if (host_scores) {
 		res.scores.resize(size_t(B));
 		std::memcpy(res.scores.data(), hp + 16, size_t(B) * 4);

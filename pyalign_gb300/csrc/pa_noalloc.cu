@@ -194,8 +194,8 @@ extern "C" pa_status pa_solve_indexed_for_score_noalloc(const pa_options *o, con
 	// codes must index the table (factory.h:602-614)
 	if (cudaMemsetAsync(codes_max, 0, 8, st) != cudaSuccess) return reject(PA_ERR_CUDA, "cudaMemsetAsync failed");
 	const int cgrid = std::max(1, std::min(sms * 4, int((batch * std::max(n_s, n_t) + 255) / 256)));
-	if (batch * n_s > 0) codes_max_kernel<<<cgrid, 256, 0, st>>>(a, batch * n_s, codes_max);
-	if (batch * n_t > 0) codes_max_kernel<<<cgrid, 256, 0, st>>>(b, batch * n_t, codes_max + 1);
+	if (batch * n_s > 0 || batch * n_t > 0)
+		codes_max_kernel<<<dim3(cgrid, 2), 256, 0, st>>>(a, batch * n_s, b, batch * n_t, codes_max);
 	uint32_t mx[2] = {0, 0};
 	if (cudaMemcpyAsync(mx, codes_max, 8, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
 	    cudaStreamSynchronize(st) != cudaSuccess)

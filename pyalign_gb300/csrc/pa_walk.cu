@@ -265,7 +265,12 @@ __global__ void __launch_bounds__(256) dense_copy_kernel(const float *src, const
 // Largest code of an array, folded into *out with atomicMax.  Streams 16-byte words with
 // four loads in flight per thread (the reads are the whole cost: 4 bytes per code), after a
 // scalar head up to the first 16-byte boundary and before a scalar tail.
-__global__ void codes_max_kernel(const uint32_t *x, int64_t n, uint32_t *out) {
+// (blocks of y 0: the largest code of a into out[0], y 1: of b into out[1]; an empty array adds
+// nothing.  One launch: beside a small solve a second one is 5 us.)
+__global__ void codes_max_kernel(const uint32_t *a, int64_t na, const uint32_t *b, int64_t nb, uint32_t *out) {
+	const uint32_t *const x = blockIdx.y ? b : a;
+	const int64_t n = blockIdx.y ? nb : na;
+	out += blockIdx.y;
 	const int64_t tid = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
 	const int64_t nth = int64_t(gridDim.x) * blockDim.x;
 	const int64_t head = min(n, int64_t(((16 - (reinterpret_cast<uintptr_t>(x) & 15)) & 15) >> 2));
