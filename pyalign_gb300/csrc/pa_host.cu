@@ -1674,18 +1674,20 @@ pa_status tune_plan(pa_solver *s, const std::vector<int32_t> &ls, const std::vec
 		bool s16;
 	};
 	std::vector<Cand> cand;
+	// (1,033 DNA pairs of 20..62 x 52..419, scores: int32 79 us, dp16_kernel's 4 x 4 blocks 48)
 	const bool both = plan.s16 && (cells < S16_SURE_CELLS || (plan.tb == TB_ONE && ls.size() < S16_SURE_PAIRS));
+	const bool h16 = plan.h16 && (!plan.s16 || both);
 	for (int G : {32, 16, 8, 4, 2, 1})
 		if (G == 4 || (int64_t(G) * R <= 2 * plan.max_ls && (G >= 4 || plan.max_ls <= 256))) {
 			cand.push_back({G, false, false, C0, false, plan.s16});
 			if (both) cand.push_back({G, false, false, C0, false, false});
-			if (plan.h16 && !plan.s16) {
+			if (h16) {
 				cand.push_back({G, false, true, 1, false, false});
 				if (C0 == 2) cand.push_back({G, false, true, 2, false, false});
 			}
 		}
 	// the 16-bit 4 x 4 block kernel (stripes of 4 G rows: the tile height 4 instead of 8)
-	if (plan.h16 && !plan.s16 && C0 == 2)
+	if (h16 && C0 == 2)
 		for (int G : {32, 16, 8})
 			if (int64_t(G) * 4 <= 2 * plan.max_ls) cand.push_back({G, false, true, 4, true, false});
 	if (plan.max_ls > 2 * 32 * R) {

@@ -116,3 +116,26 @@ def test_values_around_the_edge_of_the_range(monkeypatch, gpu_alg, locality, top
     s, got = _solve(gpu_alg, pairs, locality, Gap("affine", 11.0, 1.0), table)
     monkeypatch.setenv("PA_DP16", "0")
     _same(got, _solve(gpu_alg, pairs, locality, Gap("affine", 11.0, 1.0), table)[1], (locality, top))
+
+
+@pytest.mark.parametrize("locality", ["local", "global", "semiglobal"])
+def test_repeated_host_calls_run_as_a_pipeline(monkeypatch, gpu_alg, locality):
+    """8,401 short pairs: the second call on one solver runs in chunks on two streams."""
+    monkeypatch.setenv("PA_TUNE", "0")
+    rng = np.random.default_rng(12)
+    n = 8401
+    a, b = (rng.integers(0, 20, (n, 40)).astype(np.uint32) for _ in range(2))
+    b[::2] = a[::2]
+    b[:, 7::9] = rng.integers(0, 20, b[:, 7::9].shape)
+    ln = rng.integers(1, 41, (2, n)).astype(np.uint16)
+    table = _table(rng, 20, "scores")
+    got = {}
+    for dp16 in ("0", "all"):
+        monkeypatch.setenv("PA_DP16", dp16)
+        o = dict(options(gpu_alg, locality=locality, gap=Gap("affine", 5.0, 1.0)), batch_size=n, batch=True)
+        s = gpu_alg.m16.create_solver(40, 40, gpu_alg.m16.create_options(o))
+        got[dp16] = [[(x.score, np.asarray(x.s_to_t).tobytes(), np.asarray(x.t_to_s).tobytes())
+                      for x in s.solve_indexed_for_alignment(a, b, table, ln)] for _ in range(3)]
+        assert s.last_plan()["arithmetic"] == ("int32" if dp16 == "0" else "int16x2")
+    for calls in got["all"] + got["0"][1:]:
+        assert calls == got["0"][0]
