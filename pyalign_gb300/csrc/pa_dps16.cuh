@@ -312,6 +312,7 @@ __global__ void __launch_bounds__(32 * s16_warps(CHAIN), CHAIN ? (TB ? 16 : 17) 
 						if (v < need && wait) v = wait_progress(prog_in, need, p.status);
 					}
 					avail = __shfl_sync(0xffffffffu, v, 0);
+					__syncwarp();  // the other lanes read after lane 0's acquire
 					if (avail < need) return false;
 				}
 				if (j < lt) above = __ldcg(reinterpret_cast<const uint2 *>(bin) + j);
