@@ -469,6 +469,8 @@ class EmbeddingAlignmentScore(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, Es, Et, lengths, gap_open, gap_extend, locality, direction, linear, normalize):
+        if Es.dim() != 3 or Et.dim() != 3 or not Es.is_cuda or Et.device != Es.device:
+            raise ValueError("Es, Et must be (batch, len, d) CUDA tensors on one device")
         dim_in = Es.shape[-1]
         Es, Et = Es.contiguous().float(), Et.contiguous().float()
         # the product straight from the float rows where their width allows it; else through stored
