@@ -615,10 +615,8 @@ __global__ void __launch_bounds__(32 * s16_warps(CHAIN), CHAIN ? (TB ? 16 : 17) 
 				resB = max(resB, oB);
 			}
 		}
-		bool last_unit = true;
 		if (CHAIN) {
 			// fold in the stripes above, pass the twin's best on (a record per ticket)
-			last_unit = q_lo >= npass - 1;
 			if (q_lo > 0) {
 				if (ld_acquire(p.progress + prod) < lt) wait_progress(p.progress + prod, lt, p.status);
 				const int4 rc = __ldcg(p.chain + prod);
@@ -633,7 +631,7 @@ __global__ void __launch_bounds__(32 * s16_warps(CHAIN), CHAIN ? (TB ? 16 : 17) 
 					resB = max(resB, rc.y);
 				}
 			}
-			if (!last_unit && lane == 0) {
+			if (q_lo < npass - 1 && lane == 0) {
 				int32_t zA = iA, zB = iB;
 				if (LOCAL) {
 					zA = iA < 0 ? -1 : iA << 16 | jA;
@@ -643,11 +641,15 @@ __global__ void __launch_bounds__(32 * s16_warps(CHAIN), CHAIN ? (TB ? 16 : 17) 
 				st_release(p.progress + base, lt);  // every column (put_row, before a __syncwarp), and the record
 			}
 		}
-		if (sub == 0 && last_unit) {
+		if (sub == 0) {
 #pragma unroll
 			for (int h = 0; h < 2; h++) {
 				const int pair = h ? pb : pa;
 				if (pair < 0) continue;
+				// chained: written by the ticket of the pair's own last stripe (its first, if it has no
+				// cells), which holds its last row's best; the record passed down does not carry that, and
+				// the twin's later stripes hold nothing of this pair
+				if (CHAIN && q_lo != max((h ? npB : npA) - 1, 0)) continue;
 				const int n = h ? lsB : lsA, m = h ? ltB : ltA;
 				int32_t v = h ? resB : resA;
 				if (n == 0 || m == 0) {
