@@ -57,6 +57,11 @@ constexpr int ST_TIMEOUT = 2;   // a chained stripe waited too long for the stri
 
 // Stripe-chained mode: columns a stripe publishes at a time, and the bound of one wait.
 constexpr int PUB_CHUNK = 32;
+// dp_kernel, dp2_kernel and the dp16 kernels ask for a table and column profiles at most, beside a
+// chunk of the boundary row per warp: the 48 KB every kernel may use without an attribute
+static_assert(MAX_SMEM_TABLE * MAX_SMEM_TABLE * 4 + WARPS * PUB_CHUNK * 8 <= 48 * 1024 &&
+                  MAX_SMEM_TABLE * MAX_COLPROF * 4 + MAX_COLPROF * BLOCK * 8 + WARPS * PUB_CHUNK * 8 <= 48 * 1024,
+              "shared memory of a launch");
 constexpr int WAIT_LIMIT = 1 << 23;
 
 constexpr int PA_MAX_SEG = 4;  // length buckets of one launch (|s| <= 128, 256, 512, more)

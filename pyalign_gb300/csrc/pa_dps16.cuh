@@ -128,6 +128,10 @@ __host__ __device__ constexpr int s16_smem(int G, bool colprof, bool chain) {
 	return s16_warps(chain) * ((32 / G) * (s16_ring(G) + 2 * G) * (colprof ? 2 : 4) + (chain ? 2 * CHAIN_CHUNK * 8 : 0));
 }
 
+// The most dynamic shared memory a launch asks for: the table, the rings, 32 column profiles
+constexpr int S16_SMEM_MOST = MAX_SMEM_TABLE * MAX_COLPROF + s16_smem(1, true, false) + MAX_COLPROF * 32 * WARPS * 16;
+static_assert(s16_smem(1, false, false) <= S16_SMEM_MOST && s16_smem(32, true, true) <= S16_SMEM_MOST, "rings");
+
 template <int GAP, int LOC, int SUB, bool CHAIN, bool TB>
 __global__ void __launch_bounds__(32 * s16_warps(CHAIN), CHAIN ? (TB ? 16 : 17) : 4) dps16_kernel(DpParams<int32_t> p) {
 	constexpr bool LOCAL = LOC == LOC_LOCAL;
