@@ -1101,7 +1101,7 @@ pa_status run_dp(pa_solver *s, const Input &in, const Plan &plan, int tb, const 
 	p.best_in = best_in_dev;
 	p.values = want_values ? s->d_vals.as<float>() : nullptr;
 	p.val_off = s->m.val_off;
-	constexpr size_t counter_bytes = size_t(1 + SPREAD_CLASSES + SPREAD_SMS) * 4;
+	constexpr size_t counter_bytes = size_t(1 + SPREAD_CLASSES + 4 * SPREAD_SMS) * 4;
 	PA_CUDA(counter.ensure(counter_bytes));
 	p.work_counter = counter.as<int32_t>();
 	p.status = s->d_status.as<int32_t>();
@@ -1176,7 +1176,11 @@ pa_status run_dp(pa_solver *s, const Input &in, const Plan &plan, int tb, const 
 	// 64 x 64: 28 against 21 us), as on launches below SPREAD_MIN_CELLS, too short to gain them back.  4,096 protein pairs of
 	// 50..600 (int32) 0.80 -> 0.73 ms, 8,192 dense pairs of 32..512 (float) 1.72 -> 1.53 ms, 4,096
 	// series pairs of 128..1024 1.75 -> 1.63 ms.
-	if (!plan.units && !h16 && !exact && plan.uneven && groups_needed > WARPS &&
+	// Up to one task a scheduler there is nothing to balance, a block per SM and a warp per scheduler
+	// come without it (590 pairs of 250..500, affine, int32: 0.27 ms, by classes 0.35), and next_task
+	// counts on at least four classes.
+	static_assert(WARPS == 4, "a block's warps, one to a scheduler");
+	if (!plan.units && !h16 && !exact && plan.uneven && groups_needed > int64_t(s->sm_count) * WARPS &&
 	    groups_needed <= 3 * int64_t(s->sm_count) * bps * WARPS) {
 		grid = int64_t(s->sm_count) * bps;
 		p.spread = p.work_counter + 1;
