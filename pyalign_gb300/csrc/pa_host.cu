@@ -2463,7 +2463,7 @@ pa_status solve_impl(pa_solver *s, const Input &in, int method, float *scores_ou
 					codes_max_kernel<<<dim3(grid, 2), 256, 0, sc>>>(s->d_a.as<uint32_t>() + k0 * in.n_s, na,
 					                                                s->d_b.as<uint32_t>() + k0 * in.n_t, nb, mx);
 				PA_CUDA(cudaGetLastError());
-				launches += int(na > 0) + int(nb > 0);
+				launches += na > 0 || nb > 0;
 			}
 			if (c == 1) PA_CUDA(cudaStreamWaitEvent(sc, ev_table, 0));  // the table chunk 0 uploaded
 			if (k1 > k0) {
