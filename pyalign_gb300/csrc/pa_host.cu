@@ -1632,7 +1632,11 @@ uint64_t tune_key(const pa_solver *s, const Input &in, const Plan &plan, const s
 	       (oct(double(mlt)) << 24) | (uint64_t(s->gap & 3) << 30) | (uint64_t(s->loc & 3) << 32) |
 	       (uint64_t(plan.tb & 3) << 34) | (uint64_t(plan.use_int) << 36) | (uint64_t(in.form & 3) << 37) |
 	       (tabk << 39) | (uint64_t(s->sm_count & 1023) << 41) | (uint64_t(s->device & 63) << 51) |
-	       (uint64_t(plan.s16) << 57);
+	       (uint64_t(plan.s16) << 57) |
+	       // what else decides which kernels a launch chooses between, and their cost: dp16_kernel's
+	       // bounds, the float kernels' layout, a copied similarity, profiles in registers or not
+	       (uint64_t(plan.h16) << 58) | (uint64_t(plan.sub2 + 1) << 59) | (uint64_t(plan.copy_pitch > 0) << 61) |
+	       (uint64_t(in.form == F_INDEXED && in.table_cols <= 4) << 62);
 }
 
 template <typename Stage, typename Dp>
