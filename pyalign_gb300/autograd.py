@@ -67,6 +67,10 @@ def _lib():
         vp, i64, i32 = ctypes.c_void_p, ctypes.c_int64, ctypes.c_int32
         L.pa_solve_dense_paths.restype = i32
         L.pa_solve_dense_paths.argtypes = [vp, vp, vp, i64, i64, i64, i64, i64, vp, vp, vp, vp, vp]
+        L.pa_dense_paths_work.restype = i64
+        L.pa_dense_paths_work.argtypes = [vp, vp, i64, i64, i64, i64, i64, vp]
+        L.pa_solve_dense_paths_work.restype = i32
+        L.pa_solve_dense_paths_work.argtypes = L.pa_solve_dense_paths.argtypes + [vp, i64]
         L.pa_solve_series_paths.restype = i32
         L.pa_solve_series_paths.argtypes = [vp, vp, i64, vp, i64, i64, i64, i64, vp, vp, vp, vp, vp]
         L.pa_path_gradients.restype = i32
@@ -262,24 +266,53 @@ def _pair_offsets(B, first, stride):
     return off
 
 
+DENSE_ROOM_ASKED = 1 << 26  # bytes from which the room of a copy is worked out from the lengths
+
+
+def _dense_work(S, args):
+    """Room for a copy of S in the layout the DP reads fastest, from torch's allocator (which has it
+    back for dS, of the same size): None where there is no room.  args: of pa_solve_dense_paths."""
+    B, n_s, n_t = args[5:8]
+    room = B * n_t * (n_s + 3 & ~3)
+    if room > DENSE_ROOM_ASKED // 4:
+        room = _lib().pa_dense_paths_work(*args[1:9]) // 4
+    try:
+        return S.new_empty(room) if room else None
+    except torch.cuda.OutOfMemoryError:
+        return None
+
+
 def _forward_paths(S, lengths, gap, locality, direction, dtw, plan=None):
     """Scores and optimal paths of the pairs of S (device); returns (scores, paths, path
     lengths, device path offsets, layout flag).  plan: the _Plan of the lengths if there is one."""
     if not S.is_cuda or S.dtype != torch.float32 or S.dim() != 3:
         raise ValueError("S must be a (batch, len_s, len_t) float32 CUDA tensor")
-    # any layout with unit stride along s or t is read in place; a transposed view
-    # (stride 1 along s) is the fastest: each lane reads its 8 rows as one 32-byte sector
+    # any layout with unit stride along s or t is taken; a transposed view (stride 1 along s, rows
+    # of whole 16-byte words) is the fastest, being read in place: others are copied to it first
     if S.stride(1) != 1 and S.stride(2) != 1:
         S = S.contiguous()
     B, n_s, n_t = S.shape
     ss, st_ = S.stride(1), S.stride(2)
     plan = plan or _Plan(lengths, B, n_s, n_t, "the similarity tensor")
     solver, ln, scores, paths, plen, poff = _path_buffers(B, n_s, n_t, plan, locality, direction, dtw, gap, S.device)
-    offsets = _pair_offsets(B, S.storage_offset(), S.stride(0))
-    base = S.data_ptr() - S.storage_offset() * S.element_size()
-    _alg.check(_lib().pa_solve_dense_paths(
-        solver.handle, base, offsets.ctypes.data, ss, st_, B, n_s, n_t, ln.ctypes.data,
-        scores.data_ptr(), paths.data_ptr(), poff.ctypes.data, plen.data_ptr()))
+    pair, first, ptr = S.stride(0), S.storage_offset(), S.data_ptr()
+    offsets = _pair_offsets(B, first, pair)
+    args = (solver.handle, ptr - 4 * first, offsets.ctypes.data, ss, st_, B, n_s, n_t, ln.ctypes.data,
+            scores.data_ptr(), paths.data_ptr(), poff.ctypes.data, plen.data_ptr())
+    L = _lib()
+    # (pa_solve_dense_paths reads these layouts in place, and ignores room for a copy)
+    in_place = ss == 1 and not (pair | st_ | n_s) & 3 and not ptr & 15
+    work = None if in_place else _dense_work(S, args)
+    if work is None:
+        status = L.pa_solve_dense_paths(*args)
+    else:
+        status = L.pa_solve_dense_paths_work(*args, work.data_ptr(), 4 * work.numel())
+        if status and "out of memory" in L.pa_last_error().decode():
+            # the copy's room was the solver's last: without the copy
+            del work
+            torch.cuda.empty_cache()
+            status = L.pa_solve_dense_paths(*args)
+    _alg.check(status)
     return scores, paths, plen, _to_device(poff, S.device), ss == 1
 
 

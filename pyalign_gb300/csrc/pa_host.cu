@@ -65,6 +65,7 @@ struct DevBuf {
 		const size_t want = std::max<size_t>(n + n / 4, 256);
 		cudaError_t e = cudaMalloc(&p, want);
 		if (e == cudaSuccess) cap = want;
+		else cudaGetLastError();  // reported by the caller; the next launch's check must not find it
 		return e;
 	}
 	template <typename T>
@@ -117,6 +118,9 @@ struct Input {
 	// dense form with explicit layout: S(k, i, j) = sim[dense_off[k] + i * dense_si + j * dense_sj]
 	const int64_t *dense_off_host = nullptr;
 	int64_t dense_si = 0, dense_sj = 0;
+	// room for a copy of the dense similarity in the float kernels' layout (device; may be null)
+	float *work = nullptr;
+	int64_t work_bytes = 0;
 	// series form: S(k, i, j) = |x[k * x_stride + i] - y[k * y_stride + j]| (device)
 	const float *sx = nullptr, *sy = nullptr;
 	int64_t sx_stride = 0, sy_stride = 0;
@@ -432,6 +436,8 @@ struct pa_solver {
 		int64_t B = 0, n_s = 0, n_t = 0, trows = 0, tcols = 0, dsi = 0, dsj = 0;
 		const void *a = nullptr, *b = nullptr, *sim = nullptr, *table = nullptr, *sx = nullptr, *sy = nullptr;
 		int64_t sxs = 0, sys = 0;
+		const void *work = nullptr;
+		int64_t work_bytes = 0;
 		float eq = 0, ne = 0;
 		int32_t *maps_out = nullptr, *paths = nullptr, *path_len = nullptr;
 		float *scores = nullptr;
@@ -725,18 +731,23 @@ int dpf2_sub(const Input &in, int tb, bool want_values) {
 	return SUBF_DENSE;
 }
 
-// Whether a dense similarity that kernel cannot read in place is copied to its layout first
-// (dense_copy_kernel): unit stride along s or t, and a copy of at most 4 GiB.  The copy moves 8
-// bytes a cell at the speed of HBM, and the DP then reads 32-byte rows instead of single floats of
-// eight rows: 1,024
-// pairs of 100..400 with stride 1 along t 0.98 ms in place (dp_kernel), 0.11 + 0.38 ms copied.
+// Bytes of the copy that a dense similarity is brought to that kernel's layout by
+// (dense_copy_kernel) when it cannot be read in place, or 0: unit stride along s or t, and at most
+// 4 GiB.  The copy moves 8 bytes a cell at the speed of HBM, and the DP then reads 32-byte rows
+// instead of single floats of eight rows.  With stride 1 along t, whole calls in place (dp_kernel) and
+// copied, both ms: 1,024 pairs of 400 1.25 and 0.82, 256 of 60 0.21 and 0.16, 1 of 100 0.23 and 0.17;
+// few long pairs, which run chained in dp_kernel either way, 16 of 2000 3.4 and 2.2, 1 of 5000 7.2 and
+// 5.1 (6.6 when 8 blocks a pair copied it).  No size was found where reading in place is the faster.
+// The room is the caller's (from its own allocator, which has the use of it between calls, as for
+// the gradient of the same size); without it the similarity is read in place.
 constexpr int64_t DENSE_COPY_BYTES = int64_t(4) << 30;
-bool dense_copy_ok(const Input &in, int tb, bool want_values, const std::vector<int32_t> &lt, int64_t pitch) {
-	if (in.form != F_DENSE || in.location != PA_DEVICE || tb != TB_ONE || want_values || !in.dense_off_host) return false;
-	if (in.dense_si != 1 && in.dense_sj != 1) return false;
-	int64_t cells = 0;
-	for (int32_t t : lt) cells += t * pitch;
-	return cells * 4 <= DENSE_COPY_BYTES;
+int64_t dense_copy_pitch(int64_t max_ls) { return (max_ls + 3) & ~int64_t(3); }
+int64_t dense_copy_bytes(const Input &in, int tb, bool want_values, int64_t max_ls, int64_t columns) {
+	if (in.form != F_DENSE || in.location != PA_DEVICE || tb != TB_ONE || want_values || !in.dense_off_host) return 0;
+	if (in.dense_si != 1 && in.dense_sj != 1) return 0;
+	if (dpf2_sub(in, tb, want_values) >= 0) return 0;
+	const int64_t bytes = dense_copy_pitch(max_ls) * columns * 4;
+	return bytes <= DENSE_COPY_BYTES ? bytes : 0;
 }
 
 // Group width G (lanes per pair, R = 8 rows each; G = 1 is a lane per pair) that minimises the cells a launch
@@ -971,7 +982,7 @@ pa_status run_dp(pa_solver *s, const Input &in, const Plan &plan, int tb, const 
 		p.dense_sj = in.dense_si ? in.dense_sj : in.batch;
 		p.dense_sign = s->sign;
 		if (plan.copy_pitch) {
-			p.dense = s->d_dense.as<float>();
+			p.dense = in.work;
 			p.dense_si = 1;
 			p.dense_sj = plan.copy_pitch;
 		}
@@ -1950,6 +1961,7 @@ pa_status solve_impl(pa_solver *s, const Input &in, int method, float *scores_ou
 		if (!r.valid || r.method != method || r.form != in.form || r.B != B || r.n_s != in.n_s || r.n_t != in.n_t)
 			return false;
 		if (r.sx != in.sx || r.sy != in.sy || r.sxs != in.sx_stride || r.sys != in.sy_stride) return false;
+		if (r.work != in.work || r.work_bytes != in.work_bytes) return false;
 		if (r.a != in.a || r.b != in.b || r.sim != in.sim || r.table != in.table || r.trows != in.table_rows ||
 		    r.tcols != in.table_cols || r.dsi != in.dense_si || r.dsj != in.dense_sj || r.stream != st)
 			return false;
@@ -2040,17 +2052,13 @@ pa_status solve_impl(pa_solver *s, const Input &in, int method, float *scores_ou
 		}
 		plan.use_int = use_int;
 		if (!use_int) plan.sub2 = dpf2_sub(in, tb, want_values);
-		if (!use_int && plan.sub2 < 0) {
-			const int64_t pitch = (max_ls + 3) & ~int64_t(3);
-			int64_t cells = 0;
-			for (int32_t t : lt) cells += t * pitch;
-			if (cells > 0 && dense_copy_ok(in, tb, want_values, lt, pitch)) {
-				if (s->d_dense.ensure(size_t(cells) * 4) == cudaSuccess) {
-					plan.copy_pitch = pitch;
-					plan.sub2 = SUBF_DENSE;
-				} else {
-					cudaGetLastError();  // no room for the copy: the similarity is read in place
-				}
+		if (!use_int && plan.sub2 < 0 && in.work && (reinterpret_cast<uintptr_t>(in.work) & 15) == 0) {
+			int64_t columns = 0;
+			for (int32_t t : lt) columns += t;
+			const int64_t need = dense_copy_bytes(in, tb, want_values, max_ls, columns);
+			if (need > 0 && need <= in.work_bytes) {
+				plan.copy_pitch = dense_copy_pitch(max_ls);
+				plan.sub2 = SUBF_DENSE;
 			}
 		}
 		plan.C32 = cols2_ok(plan, want_values) || plan.sub2 >= 0 ? 2 : 1;
@@ -2269,9 +2277,13 @@ pa_status solve_impl(pa_solver *s, const Input &in, int method, float *scores_ou
 	// a dense similarity into the layout the float kernels read (the staged offsets are in place)
 	auto dense_copy = [&](cudaStream_t sw) -> cudaError_t {
 		if (!plan.copy_pitch) return cudaSuccess;
-		dense_copy_kernel<<<dim3(unsigned(B), unsigned(std::min<int64_t>(8, (max_lt + 31) / 32))), 256, 0, sw>>>(in.sim, s->m.dense_src, in.dense_si, in.dense_sj,
-		                                                     s->d_dense.as<float>(), s->m.dense_off, plan.copy_pitch,
-		                                                     s->m.ls, s->m.lt);
+		// a block per strip of columns of a pair, at most 8 of them with many pairs; with few pairs
+		// every strip, and its rows in parts of at least 64, until there are 8 blocks an SM
+		const int64_t strips = (max_lt + 31) / 32, parts = (max_ls + 63) / 64, fill = int64_t(s->sm_count) * 8;
+		const int64_t gy = std::min(strips, std::min<int64_t>(std::max<int64_t>(8, (fill + B - 1) / B), 65535));
+		const int64_t gz = std::min(parts, std::max<int64_t>(1, fill / (B * gy)));
+		dense_copy_kernel<<<dim3(unsigned(B), unsigned(gy), unsigned(gz)), 256, 0, sw>>>(
+		    in.sim, s->m.dense_src, in.dense_si, in.dense_sj, in.work, s->m.dense_off, plan.copy_pitch, s->m.ls, s->m.lt);
 		launches++;
 		return cudaGetLastError();
 	};
@@ -2637,6 +2649,8 @@ pa_status solve_impl(pa_solver *s, const Input &in, int method, float *scores_ou
 		r.sy = in.sy;
 		r.sxs = in.sx_stride;
 		r.sys = in.sy_stride;
+		r.work = in.work;
+		r.work_bytes = in.work_bytes;
 		r.table = in.table;
 		r.eq = in.eq;
 		r.ne = in.ne;
@@ -3200,9 +3214,38 @@ uint64_t pa_content_hash(const void *data, int64_t bytes) {
 	return r ^ (r >> 32);
 }
 
+int64_t pa_dense_paths_work(const float *sim, const int64_t *offsets, int64_t stride_s, int64_t stride_t,
+                            int64_t batch, int64_t n_s, int64_t n_t, const int32_t *length) {
+	if (!sim || !offsets || !length || batch <= 0) return 0;
+	Input in{};
+	in.form = F_DENSE;
+	in.location = PA_DEVICE;
+	in.batch = batch;
+	in.n_s = n_s;
+	in.n_t = n_t;
+	in.sim = sim;
+	in.dense_off_host = offsets;
+	in.dense_si = stride_s;
+	in.dense_sj = stride_t;
+	int64_t max_ls = 0, columns = 0;  // clamped as the solve clamps them
+	for (int64_t k = 0; k < batch; k++) {
+		max_ls = std::max<int64_t>(max_ls, std::min<int64_t>(std::max(length[k], 0), n_s));
+		columns += std::min<int64_t>(std::max(length[batch + k], 0), n_t);
+	}
+	return dense_copy_bytes(in, TB_ONE, false, max_ls, columns);
+}
+
 pa_status pa_solve_dense_paths(pa_solver *s, const float *sim, const int64_t *offsets, int64_t stride_s,
                                int64_t stride_t, int64_t batch, int64_t n_s, int64_t n_t, const int32_t *length,
                                float *scores, int32_t *paths, const int64_t *path_offsets, int32_t *path_len) {
+	return pa_solve_dense_paths_work(s, sim, offsets, stride_s, stride_t, batch, n_s, n_t, length, scores, paths,
+	                                 path_offsets, path_len, nullptr, 0);
+}
+
+pa_status pa_solve_dense_paths_work(pa_solver *s, const float *sim, const int64_t *offsets, int64_t stride_s,
+                                    int64_t stride_t, int64_t batch, int64_t n_s, int64_t n_t, const int32_t *length,
+                                    float *scores, int32_t *paths, const int64_t *path_offsets, int32_t *path_len,
+                                    void *work, int64_t work_bytes) {
 	if (!s || !sim || !offsets || !length || !paths || !path_offsets || !path_len)
 		return fail(PA_ERR_INVALID_ARGUMENT, "null argument");
 	Input in{};
@@ -3216,6 +3259,8 @@ pa_status pa_solve_dense_paths(pa_solver *s, const float *sim, const int64_t *of
 	in.dense_off_host = offsets;
 	in.dense_si = stride_s;
 	in.dense_sj = stride_t;
+	in.work = static_cast<float *>(work);
+	in.work_bytes = work_bytes;
 	UserPaths up_{};
 	up_.paths = paths;
 	up_.path_off = path_offsets;

@@ -214,8 +214,8 @@ void launch_walk(const WalkParams &w, cudaStream_t st) {
 	else walk_kernel<false><<<grid, WALK_WARPS * 32, 0, st>>>(w);
 }
 
-// See pa_dp.cuh.  A block takes every gridDim.y-th strip of 32 columns of one pair, 64 x 32 cells
-// at a time through shared memory, so that both the reads (along the source's unit stride) and the
+// See pa_dp.cuh.  A block takes every gridDim.y-th strip of 32 columns of one pair, and of it every
+// gridDim.z-th part of 64 rows, 64 x 32 cells at a time through shared memory, so that both the reads (along the source's unit stride) and the
 // writes (along s) are whole 128-byte lines.  HBM-bound, 8 bytes moved per cell, with eight loads
 // of a thread in flight: 1,024 pairs of 100..400 (64 M
 // cells) in 109 us (137 us with 32 x 32 tiles and four loads).
@@ -230,7 +230,7 @@ __global__ void __launch_bounds__(256) dense_copy_kernel(const float *src, const
 	float *D = dst + dst_off[pair];
 	const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
 	for (int j0 = 32 * blockIdx.y; j0 < lt; j0 += 32 * gridDim.y)
-		for (int i0 = 0; i0 < ls; i0 += TI) {
+		for (int i0 = TI * blockIdx.z; i0 < ls; i0 += TI * gridDim.z) {
 			float v[8];
 			if (si == 1) {  // only the pitch or the alignment differs
 #pragma unroll
