@@ -68,6 +68,11 @@ struct DevBuf {
 		else cudaGetLastError();  // reported by the caller; the next launch's check must not find it
 		return e;
 	}
+	void release() {
+		if (p) cudaFree(p);
+		p = nullptr;
+		cap = 0;
+	}
 	template <typename T>
 	T *as() const { return reinterpret_cast<T *>(p); }
 };
@@ -1495,8 +1500,6 @@ pa_status run_wsb_tiles(pa_solver *s, const Input &in, const std::vector<int32_t
 	PA_CUDA(pa_copy(s, d, h, o, cudaMemcpyHostToDevice, st));
 	if (in.form == F_INDEXED && in.location == PA_DEVICE)
 		PA_CUDA(pa_copy(s, d + o_tab, in.table, size_t(in.table_rows * in.table_cols) * 4, cudaMemcpyDeviceToDevice, st));
-	PA_CUDA(s->d_wsb_vals.ensure(size_t(voff[size_t(B)]) * 4));
-	PA_CUDA(s->d_wsb_vals_t.ensure(size_t(voff[size_t(B)]) * 4));
 	// zeroed per call: the optimum keys, the tile counters, the work counter
 	const size_t zb = size_t(B) * 8 + size_t(poff[size_t(B)]) * 4 + 4;
 	PA_CUDA(s->d_progress.ensure(zb));
@@ -1560,6 +1563,19 @@ bool wsb_tiles_ok(const std::vector<int32_t> &ls, const std::vector<int32_t> &lt
 	for (size_t k = 0; k < ls.size(); k++)
 		if (int64_t(ls[k]) * lt[k] >= (int64_t(1) << 32) || std::max(ls[k], lt[k]) >= (1 << 20)) return false;
 	return true;
+}
+
+// The sweep's two matrices of whole tiles: up to 32 times the cells' memory where the pairs are
+// narrow.  False, with nothing kept, when there is no room for them (wsb_kernel then takes the solve).
+bool wsb_tiles_room(pa_solver *s, const std::vector<int32_t> &ls, const std::vector<int32_t> &lt) {
+	constexpr int64_t T = WSB_TILE;
+	int64_t cells = 0;
+	for (size_t k = 0; k < ls.size(); k++) cells += (ls[k] + T - 1) / T * ((lt[k] + T - 1) / T) * T * T;
+	if (s->d_wsb_vals.ensure(size_t(cells) * 4) == cudaSuccess && s->d_wsb_vals_t.ensure(size_t(cells) * 4) == cudaSuccess)
+		return true;
+	s->d_wsb_vals.release();
+	s->d_wsb_vals_t.release();
+	return false;
 }
 
 pa_status download_wsb(pa_solver *s, ResultData &res) {
@@ -2374,7 +2390,7 @@ pa_status solve_impl(pa_solver *s, const Input &in, int method, float *scores_ou
 					wmaps = s->d_maps.as<int32_t>();
 				}
 			}
-			if (!wsb_host && wsb_tiles_ok(ls, lt)) {
+			if (!wsb_host && wsb_tiles_ok(ls, lt) && wsb_tiles_room(s, ls, lt)) {
 				if (pa_status e = run_wsb_tiles(s, in, ls, lt, &launches, wmaps)) return e;
 			} else if (pa_status e = run_wsb(s, in, ls, lt, &launches, res, wmaps)) {
 				return e;
