@@ -254,6 +254,13 @@ pa_status pa_result_path_counts(const pa_result *r, uint64_t *counts);
 pa_status pa_result_first_alignments(const pa_result *r, int32_t k, int32_t *counts, int32_t *maps,
                                      int32_t *paths, int32_t *path_len);
 
+/* The same for about `seconds` at most.  De-duplication can make the search for the next
+ * alignment as long as a pair has co-optimal paths, however few alignments they spell: a lane
+ * whose search was cut off has more[lane] = 1 (host, batch entries; 0 otherwise) and counts[lane]
+ * results, which need not be all; pa_iterator_next goes on from there. */
+pa_status pa_result_first_alignments_within(const pa_result *r, int32_t k, double seconds, int32_t *counts,
+                                            int32_t *more, int32_t *maps, int32_t *paths, int32_t *path_len);
+
 /* ---- batched form: the whole bag in one call (no per-lane objects) ----
  * Score plus one optimal traceback for `batch` pairs of uneven lengths, the throughput
  * path behind ProblemBatch.  Inputs and outputs are host or device memory

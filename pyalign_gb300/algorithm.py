@@ -128,6 +128,8 @@ def lib():
         L.pa_iterator_destroy.argtypes = [_P]
         L.pa_result_path_counts.argtypes = [_P, ctypes.POINTER(ctypes.c_uint64)]
         L.pa_result_first_alignments.argtypes = [_P, _c_i32, _PI, _PI, _PI, _PI]
+        L.pa_result_first_alignments_within.restype = _c_i32
+        L.pa_result_first_alignments_within.argtypes = [_P, _c_i32, ctypes.c_double, _PI, _PI, _PI, _PI, _PI]
         L.pa_solve_batch_result.argtypes = [_P, ctypes.POINTER(Batch), _PI, _PL, ctypes.POINTER(_P)]
         _lib = L
     return _lib
@@ -508,12 +510,15 @@ class Solution:
 
 class FirstAlignments:
     """The first k optimal alignments of every lane of an all-optimal result, enumerated on
-    the GPU in one pass (pa_result_first_alignments): what the first k next() calls of each
-    lane's iterator return.  `counts[lane]` results per lane (fewer than k: the lane has no
-    more); `alignment(lane, j)` -> the j-th map (s_to_t if |s| <= |t|, else t_to_s) and, when
+    the GPU in one pass (pa_result_first_alignments_within): what the first k next() calls of
+    each lane's iterator return.  `counts[lane]` results per lane (fewer than k: the lane has no
+    more, or, where `more[lane]` is set, the search took longer than SECONDS and was cut off);
+    `alignment(lane, j)` -> the j-th map (s_to_t if |s| <= |t|, else t_to_s) and, when
     enumerated with paths, the j-th walk ((n, 2) points)."""
 
-    __slots__ = ("k", "counts", "maps", "mstart", "msize", "paths", "plen", "pstart", "pstride")
+    SECONDS = 10.0
+
+    __slots__ = ("k", "counts", "more", "maps", "mstart", "msize", "paths", "plen", "pstart", "pstride")
 
     def __init__(self, res, k, with_paths=False):
         L = lib()
@@ -526,6 +531,7 @@ class FirstAlignments:
         self.mstart = np.zeros(n, np.int64)
         self.mstart[1:] = np.cumsum(self.msize)[:-1] * self.k
         self.counts = np.zeros(n, np.int32)
+        self.more = np.zeros(n, np.int32)
         self.maps = np.zeros(max(1, int(self.msize.sum()) * self.k), np.int32)
         self.paths = self.plen = self.pstart = self.pstride = None
         if with_paths:
@@ -534,9 +540,9 @@ class FirstAlignments:
             self.pstart[1:] = np.cumsum(self.pstride)[:-1] * self.k
             self.paths = np.zeros((max(1, int(self.pstride.sum()) * self.k), 2), np.int32)
             self.plen = np.zeros(n * self.k, np.int32)
-        st = L.pa_result_first_alignments(res.ptr, self.k, _ip(self.counts), _ip(self.maps),
-                                          _ip(self.paths) if with_paths else None,
-                                          _ip(self.plen) if with_paths else None)
+        st = L.pa_result_first_alignments_within(res.ptr, self.k, self.SECONDS, _ip(self.counts), _ip(self.more),
+                                                 _ip(self.maps), _ip(self.paths) if with_paths else None,
+                                                 _ip(self.plen) if with_paths else None)
         if st == PA_ERR_UNSUPPORTED:
             raise NotImplementedError(L.pa_last_error().decode())
         check(st)
@@ -614,7 +620,7 @@ class _Iter:
                 self._served += 1
                 return float(L.pa_result_score(self._res.ptr, self._lane)), mp.copy(), \
                     (path.copy() if path is not None else np.zeros((0, 2), np.int32))
-            if c < f.k:
+            if c < f.k and not f.more[self._lane]:
                 return None
         if self._it is None:
             # the host search (pa_iterator_next), resumed after the results already served

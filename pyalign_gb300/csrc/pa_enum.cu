@@ -171,11 +171,27 @@ __global__ void __launch_bounds__(32) enum_kernel(EnumParams p) {
 	const int2 *seeds = p.local ? p.seeds + p.seed_off[L] : nullptr;
 	bool have = false;
 	int eu = 0, ev = 0, epl = 0;
-	if (!p.local && p.has[L]) {
+	if (p.resume) {
+		const EnumState from = p.state[L];
+		have = from.have;
+		eu = from.u;
+		ev = from.v;
+		epl = from.path_len;
+		sp = from.sp;
+		si = from.si;
+		count = from.count;
+		for (int x = lane; x < min(sp, SMEM_STACK); x += 32) top[x] = stk[x];
+		__syncwarp();
+	} else if (!p.local && p.has[L]) {
 		eu = p.seed[2 * L];
 		ev = p.seed[2 * L + 1];
 		have = true;
 	}
+	// De-duplication makes the search as long as the pair has paths, however few alignments they
+	// spell (30 letters against 30 others without gap costs: 10^17 paths, one alignment), so a launch
+	// stops after p.cycles and the host launches it again, or not.
+	const long long begun = clock64();
+	bool paused = false;
 	// path points 0 .. low - 1 are those of the last complete path; its hash and point count
 	int low = 0, n = 0;
 	unsigned long long h = 0;
@@ -406,7 +422,11 @@ __global__ void __launch_bounds__(32) enum_kernel(EnumParams p) {
 				}
 			}
 		}
-		if (dup) continue;
+		if (dup) {  // (between two yields lie |s| + |t| + 2 entries at most)
+			paused = __shfl_sync(0xffffffffu, clock64() - begun, 0) > p.cycles;
+			if (paused) break;
+			continue;
+		}
 		if (SM) {
 #pragma unroll 8
 			for (int x = lane; x < m; x += 32) mp[x] = smap[x];
@@ -429,9 +449,14 @@ __global__ void __launch_bounds__(32) enum_kernel(EnumParams p) {
 	for (int64_t x = int64_t(count) * m + lane; x < int64_t(p.k) * m; x += 32) maps[x] = -1;
 	if (p.paths)
 		for (int j = count + lane; j < p.k; j += 32) p.path_len[int64_t(L) * p.k + j] = 0;
+	if (paused) {
+		__syncwarp();  // lane 0's writes
+		for (int x = lane; x < min(sp, SMEM_STACK); x += 32) stk[x] = top[x];
+	}
 	if (lane == 0) {
 		p.count[L] = count;
-		p.status[L] = status;
+		p.status[L] = paused ? ENUM_PAUSED : status;
+		p.state[L] = EnumState{have, eu, ev, epl, sp, si, count};
 	}
 }
 

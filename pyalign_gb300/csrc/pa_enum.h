@@ -9,6 +9,13 @@ namespace pa {
 constexpr int32_t ENUM_NO_TB = INT32_MIN;  // the terminal point of an empty list
 constexpr int32_t ENUM_OVERFLOW = 1;  // the stack was full: enumerate again with a larger one
 constexpr int32_t ENUM_BAD_PATH = 2;  // a path longer than |s| + |t| + 2 points (not reachable)
+constexpr int32_t ENUM_PAUSED = 3;    // the launch's time was up: launch again to go on
+
+// A paused search (its stack and path are in memory).
+struct EnumState {
+	int32_t have, u, v, path_len;  // the entry to go on with, if `have`
+	int32_t sp, si, count;
+};
 
 struct EnumParams {
 	int32_t nwork;
@@ -36,7 +43,10 @@ struct EnumParams {
 	unsigned long long *hash;   // k per pair
 	int32_t *npts;              // k per pair
 	int32_t *count;             // per pair: paths yielded (<= k)
-	int32_t *status;            // per pair: ENUM_OVERFLOW
+	int32_t *status;            // per pair: 0 = done, ENUM_OVERFLOW, ENUM_BAD_PATH, ENUM_PAUSED
+	EnumState *state;           // per pair, written
+	int32_t resume;             // 1: the searches go on from their state
+	int64_t cycles;             // SM cycles after which a search pauses
 	int32_t smem_map;           // the largest map when it is kept in shared memory, else 0
 };
 constexpr int32_t ENUM_SMEM_MAP = 40960;  // at most (160 KB)

@@ -8,6 +8,7 @@
 // device every solve fails with PA_ERR_NO_DEVICE.
 
 #include <algorithm>
+#include <chrono>
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
@@ -3806,7 +3807,13 @@ pa_status pa_result_path_counts(const pa_result *r, uint64_t *counts) {
 // caller's host buffers.
 pa_status pa_result_first_alignments(const pa_result *r, int32_t k, int32_t *counts, int32_t *maps, int32_t *paths,
                                      int32_t *path_len) {
-	if (!r || !counts || k < 1) return fail(PA_ERR_INVALID_ARGUMENT, "pa_result_first_alignments: bad argument");
+	return pa_result_first_alignments_within(r, k, INFINITY, counts, nullptr, maps, paths, path_len);
+}
+
+pa_status pa_result_first_alignments_within(const pa_result *r, int32_t k, double seconds, int32_t *counts, int32_t *more,
+                                            int32_t *maps, int32_t *paths, int32_t *path_len) {
+	if (!r || !counts || k < 1 || (!more && std::isfinite(seconds)))
+		return fail(PA_ERR_INVALID_ARGUMENT, "pa_result_first_alignments: bad argument");
 	if ((paths == nullptr) != (path_len == nullptr))
 		return fail(PA_ERR_INVALID_ARGUMENT, "pa_result_first_alignments: paths and path_len go together");
 	const ResultData &d = *r->d;
@@ -3814,6 +3821,7 @@ pa_status pa_result_first_alignments(const pa_result *r, int32_t k, int32_t *cou
 		return fail(PA_ERR_UNSUPPORTED, "device enumeration needs an all-optimal result with linear or affine gap costs");
 	const int64_t B = d.batch;
 	if (B == 0) return PA_OK;
+	if (more) std::fill(more, more + B, 0);
 	const bool local = d.loc == LOC_LOCAL;
 	const int64_t K = k;
 	// per-lane regions: maps k x min(|s|, |t|), paths k x (|s| + |t| + 2), the search's path
@@ -3935,7 +3943,8 @@ pa_status pa_result_first_alignments(const pa_result *r, int32_t k, int32_t *cou
 	PA_CUDA(dhash.ensure(size_t(B * K) * 8));
 	PA_CUDA(dnpts.ensure(size_t(B * K) * 4));
 	PA_CUDA(dcnt.ensure(size_t(B) * 4));
-	PA_CUDA(dstat.ensure(size_t(B) * 4));
+	PA_CUDA(dstat.ensure(size_t(B) * (sizeof(pa::EnumState) + 4)));  // the states, then the status words
+	int32_t *const status_dev = reinterpret_cast<int32_t *>(dstat.as<pa::EnumState>() + B);
 	DevBuf dmo, dpo, dwo;
 	PA_CUDA(dmo.ensure(size_t(B) * 8));
 	PA_CUDA(dpo.ensure(size_t(B) * 8));
@@ -3951,6 +3960,7 @@ pa_status pa_result_first_alignments(const pa_result *r, int32_t k, int32_t *cou
 	for (int64_t L = 0; L < B; L++)
 		scap[size_t(L)] = int32_t(stack0 > 0 ? stack0 : d.ls[size_t(L)] + d.lt[size_t(L)] + 66);
 	std::vector<int32_t> work = all, status(static_cast<size_t>(B), 0);
+	const auto begun = std::chrono::steady_clock::now();
 	DevBuf dstk, dsto, dscp;
 	PA_CUDA(dsto.ensure(size_t(B) * 8));
 	PA_CUDA(dscp.ensure(size_t(B) * 4));
@@ -3997,23 +4007,41 @@ pa_status pa_result_first_alignments(const pa_result *r, int32_t k, int32_t *cou
 		ep.hash = dhash.as<unsigned long long>();
 		ep.npts = dnpts.as<int32_t>();
 		ep.count = dcnt.as<int32_t>();
-		ep.status = dstat.as<int32_t>();
+		ep.status = status_dev;
+		ep.state = dstat.as<pa::EnumState>();
 		int64_t most = 0;
 		for (int32_t L : work) most = std::max<int64_t>(most, std::min(d.ls[size_t(L)], d.lt[size_t(L)]));
 		int64_t smem_most = pa::ENUM_SMEM_MAP;
 		if (const char *e = std::getenv("PA_ENUM_MAP")) smem_most = std::min<int64_t>(smem_most, std::atoll(e));  // tests
 		ep.smem_map = most <= smem_most ? int32_t(std::max<int64_t>(most, 1)) : 0;
-		PA_CUDA(pa::enum_solve(ep, nullptr));
-		PA_CUDA(cudaMemcpy(status.data(), dstat.p, size_t(B) * 4, cudaMemcpyDeviceToHost));
+		// a launch ends after about 0.13 s of each search, so no input holds the GPU for long; the
+		// searches under way then go on in the next one
+		ep.cycles = int64_t(1) << 28;
+		if (const char *e = std::getenv("PA_ENUM_CYCLES")) ep.cycles = std::max(0ll, std::atoll(e));  // tests
 		std::vector<int32_t> again;
-		for (int32_t L : work) {
-			if (status[size_t(L)] == pa::ENUM_BAD_PATH)
-				return fail(PA_ERR_INTERNAL, "device enumeration: a path outgrew |s| + |t| + 2 points");
-			if (status[size_t(L)] == pa::ENUM_OVERFLOW) {
-				if (scap[size_t(L)] > (1 << 28)) return fail(PA_ERR_INTERNAL, "device enumeration: stack limit");
-				scap[size_t(L)] *= 4;
-				again.push_back(L);
+		for (std::vector<int32_t> run = work; !run.empty();) {
+			ep.nwork = int32_t(run.size());
+			PA_CUDA(pa::enum_solve(ep, nullptr));
+			PA_CUDA(cudaMemcpy(status.data(), status_dev, size_t(B) * 4, cudaMemcpyDeviceToHost));
+			std::vector<int32_t> paused;
+			for (int32_t L : run) {
+				if (status[size_t(L)] == pa::ENUM_BAD_PATH)
+					return fail(PA_ERR_INTERNAL, "device enumeration: a path outgrew |s| + |t| + 2 points");
+				if (status[size_t(L)] == pa::ENUM_OVERFLOW) {
+					if (scap[size_t(L)] > (1 << 28)) return fail(PA_ERR_INTERNAL, "device enumeration: stack limit");
+					scap[size_t(L)] *= 4;
+					again.push_back(L);
+				}
+				if (status[size_t(L)] == pa::ENUM_PAUSED) paused.push_back(L);
 			}
+			if (!paused.empty() && more &&
+			    std::chrono::duration<double>(std::chrono::steady_clock::now() - begun).count() >= seconds) {
+				for (int32_t L : paused) more[L] = 1;
+				paused.clear();
+			}
+			run.swap(paused);
+			ep.resume = 1;
+			if (!run.empty()) PA_CUDA(cudaMemcpy(dwork.p, run.data(), run.size() * 4, cudaMemcpyHostToDevice));
 		}
 		work.swap(again);
 	}
