@@ -308,17 +308,20 @@ pa_status pa_solve_dense_paths(pa_solver *s, const float *sim, const int64_t *of
                                int64_t stride_t, int64_t batch, int64_t n_s, int64_t n_t, const int32_t *length,
                                float *scores, int32_t *paths, const int64_t *path_offsets, int32_t *path_len);
 
-/* The same with room for a copy of S in the layout the kernels read fastest.
- * pa_dense_paths_work: the bytes the copy takes (sim is not read; offsets, length: host, as
- * above), 0 where S is read in place with or without room.  work: that many bytes of device
- * memory, 16-byte aligned, not used otherwise until the stream has done the solve's work; null,
- * misaligned or too small: S is read in place, with the same results. */
+/* The same for S with rows to spare, and with room for a copy of S in the layout the kernels read
+ * fastest.  rows: with stride_s = 1, how many entries of a column may be read (what lies past n_s
+ * does not matter); 0, or less than n_s: n_s.  Columns of whole 16-byte words on 16-byte
+ * boundaries are read in place, so n_s needs no multiple of 4 where rows has it.
+ * pa_dense_paths_work: the bytes the copy takes for rows = 0 (sim is not read; offsets, length:
+ * host, as above), 0 where S is read in place with or without room.  work: that many bytes of
+ * device memory, 16-byte aligned, not used otherwise until the stream has done the solve's work;
+ * null, misaligned or too small: S is read in place, with the same results. */
 int64_t pa_dense_paths_work(const float *sim, const int64_t *offsets, int64_t stride_s, int64_t stride_t,
                             int64_t batch, int64_t n_s, int64_t n_t, const int32_t *length);
 pa_status pa_solve_dense_paths_work(pa_solver *s, const float *sim, const int64_t *offsets, int64_t stride_s,
                                     int64_t stride_t, int64_t batch, int64_t n_s, int64_t n_t, const int32_t *length,
                                     float *scores, int32_t *paths, const int64_t *path_offsets, int32_t *path_len,
-                                    void *work, int64_t work_bytes);
+                                    int64_t rows, void *work, int64_t work_bytes);
 
 /* The same for two float32 series per pair (device memory): S(i, j) = |x[k * x_stride + i] -
  * y[k * y_stride + j]| computed in the DP kernel, never stored -- the cost matrix of DTW on

@@ -70,7 +70,7 @@ def _lib():
         L.pa_dense_paths_work.restype = i64
         L.pa_dense_paths_work.argtypes = [vp, vp, i64, i64, i64, i64, i64, vp]
         L.pa_solve_dense_paths_work.restype = i32
-        L.pa_solve_dense_paths_work.argtypes = L.pa_solve_dense_paths.argtypes + [vp, i64]
+        L.pa_solve_dense_paths_work.argtypes = L.pa_solve_dense_paths.argtypes + [i64, vp, i64]
         L.pa_solve_series_paths.restype = i32
         L.pa_solve_series_paths.argtypes = [vp, vp, i64, vp, i64, i64, i64, i64, vp, vp, vp, vp, vp]
         L.pa_path_gradients.restype = i32
@@ -282,9 +282,10 @@ def _dense_work(S, args):
         return None
 
 
-def _forward_paths(S, lengths, gap, locality, direction, dtw, plan=None):
+def _forward_paths(S, lengths, gap, locality, direction, dtw, plan=None, rows=0):
     """Scores and optimal paths of the pairs of S (device); returns (scores, paths, path
-    lengths, device path offsets, layout flag).  plan: the _Plan of the lengths if there is one."""
+    lengths, device path offsets, layout flag).  plan: the _Plan of the lengths if there is one; rows: entries
+    of a column of S (stride 1 along s) that may be read, if more than its rows."""
     if not S.is_cuda or S.dtype != torch.float32 or S.dim() != 3:
         raise ValueError("S must be a (batch, len_s, len_t) float32 CUDA tensor")
     # any layout with unit stride along s or t is taken; a transposed view (stride 1 along s, rows
@@ -300,18 +301,16 @@ def _forward_paths(S, lengths, gap, locality, direction, dtw, plan=None):
     args = (solver.handle, ptr - 4 * first, offsets.ctypes.data, ss, st_, B, n_s, n_t, ln.ctypes.data,
             scores.data_ptr(), paths.data_ptr(), poff.ctypes.data, plen.data_ptr())
     L = _lib()
-    # (pa_solve_dense_paths reads these layouts in place, and ignores room for a copy)
-    in_place = ss == 1 and not (pair | st_ | n_s) & 3 and not ptr & 15
+    # (these layouts are read in place, and room for a copy is ignored)
+    in_place = ss == 1 and not (pair | st_) & 3 and not ptr & 15 and (n_s + 3 & ~3) <= max(n_s, rows)
     work = None if in_place else _dense_work(S, args)
-    if work is None:
+    status = L.pa_solve_dense_paths_work(*args, rows, work.data_ptr() if work is not None else None,
+                                         4 * work.numel() if work is not None else 0)
+    if status and work is not None and "out of memory" in L.pa_last_error().decode():
+        # the copy's room was the solver's last: without the copy
+        del work
+        torch.cuda.empty_cache()
         status = L.pa_solve_dense_paths(*args)
-    else:
-        status = L.pa_solve_dense_paths_work(*args, work.data_ptr(), 4 * work.numel())
-        if status and "out of memory" in L.pa_last_error().decode():
-            # the copy's room was the solver's last: without the copy
-            del work
-            torch.cuda.empty_cache()
-            status = L.pa_solve_dense_paths(*args)
     _alg.check(status)
     return scores, paths, plen, _to_device(poff, S.device), ss == 1
 
@@ -519,18 +518,20 @@ class EmbeddingAlignmentScore(torch.autograd.Function):
             Etb, inv_t = normalized_bf16(Et, normalize, ln[:, 1], tiled=True)
         # S^T = en_t en_s^T on the tensor cores, only the cells inside the lengths; its
         # transposed view is S with stride 1 along s; its columns are padded to whole 16-byte
-        # words (rows no pair reaches) for the DP's loads
+        # words for the DP's loads (the solver keeps the true number of rows, on which the
+        # rounding of its border costs depends)
         B, n_s, n_t = Es.shape[0], Es.shape[1], Et.shape[1]
-        St = torch.empty((B, n_t, (n_s + 3) // 4 * 4), dtype=torch.float32, device=Es.device)
+        St = torch.empty((B, n_t, n_s + 3 & ~3), dtype=torch.float32, device=Es.device)
         plan = None
         if rows:
             plan = _Plan(lengths, B, n_s, n_t, "the embeddings", ROWS_TILE)
             inv_s, inv_t = _similarity_rows(Es, Et, lengths, normalize, St, plan)
         else:
             similarity_bf16(Esb, Etb, lengths, out=St[:, :, :n_s])
-        S = St.transpose(1, 2)
+        pitch = St.shape[2]
+        S = St.transpose(1, 2) if pitch == n_s else St.transpose(1, 2).narrow(1, 0, n_s)
         gap = (float(gap_open), None) if linear else (float(gap_open), float(gap_extend))
-        scores, paths, plen, poff, _ = _forward_paths(S, lengths, gap, locality, direction, False, plan)
+        scores, paths, plen, poff, _ = _forward_paths(S, lengths, gap, locality, direction, False, plan, pitch)
         ctx.save_for_backward(Es, Et, Esb, Etb, inv_s, inv_t, paths, plen, poff)
         ctx.meta = (locality, direction, linear, normalize, gap_open.device)
         ctx.dim_in = dim_in

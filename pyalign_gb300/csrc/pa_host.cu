@@ -124,6 +124,7 @@ struct Input {
 	// dense form with explicit layout: S(k, i, j) = sim[dense_off[k] + i * dense_si + j * dense_sj]
 	const int64_t *dense_off_host = nullptr;
 	int64_t dense_si = 0, dense_sj = 0;
+	int64_t dense_rows = 0;  // stride 1 along s: rows of each column that may be read (at least n_s)
 	// room for a copy of the dense similarity in the float kernels' layout (device; may be null)
 	float *work = nullptr;
 	int64_t work_bytes = 0;
@@ -443,7 +444,7 @@ struct pa_solver {
 		const void *a = nullptr, *b = nullptr, *sim = nullptr, *table = nullptr, *sx = nullptr, *sy = nullptr;
 		int64_t sxs = 0, sys = 0;
 		const void *work = nullptr;
-		int64_t work_bytes = 0;
+		int64_t work_bytes = 0, dense_rows = 0;
 		float eq = 0, ne = 0;
 		int32_t *maps_out = nullptr, *paths = nullptr, *path_len = nullptr;
 		float *scores = nullptr;
@@ -722,14 +723,15 @@ int cols_of(const Plan &plan, bool units) { return units && !plan.use_int ? 1 : 
 
 // The float form of a launch's similarities the two-column float kernel (pa_dpf2.cuh) reads, or
 // -1: scores or one traceback, without Solution values, of a table, of series, or of a dense
-// similarity whose columns can be read 16 bytes at a time (stride 1 along s, aligned, a multiple
-// of 4 rows).
+// similarity whose columns can be read 16 bytes at a time (stride 1 along s, aligned, rows up to a
+// multiple of 4).
 int dpf2_sub(const Input &in, int tb, bool want_values) {
 	if (tb == TB_ALL || want_values) return -1;
 	if (in.form == F_INDEXED) return SUBF_TABLE;
 	if (tb != TB_ONE) return -1;
 	if (in.form == F_SERIES) return SUBF_SERIES;
-	if (in.form != F_DENSE || in.location != PA_DEVICE || in.dense_si != 1 || (in.dense_sj & 3) || (in.n_s & 3) ||
+	if (in.form != F_DENSE || in.location != PA_DEVICE || in.dense_si != 1 || (in.dense_sj & 3) ||
+	    ((in.n_s + 3) & ~int64_t(3)) > std::max(in.n_s, in.dense_rows) ||
 	    (reinterpret_cast<uintptr_t>(in.sim) & 15) || !in.dense_off_host)
 		return -1;
 	for (int64_t k = 0; k < in.batch; k++)
@@ -1978,7 +1980,7 @@ pa_status solve_impl(pa_solver *s, const Input &in, int method, float *scores_ou
 		if (!r.valid || r.method != method || r.form != in.form || r.B != B || r.n_s != in.n_s || r.n_t != in.n_t)
 			return false;
 		if (r.sx != in.sx || r.sy != in.sy || r.sxs != in.sx_stride || r.sys != in.sy_stride) return false;
-		if (r.work != in.work || r.work_bytes != in.work_bytes) return false;
+		if (r.work != in.work || r.work_bytes != in.work_bytes || r.dense_rows != in.dense_rows) return false;
 		if (r.a != in.a || r.b != in.b || r.sim != in.sim || r.table != in.table || r.trows != in.table_rows ||
 		    r.tcols != in.table_cols || r.dsi != in.dense_si || r.dsj != in.dense_sj || r.stream != st)
 			return false;
@@ -2668,6 +2670,7 @@ pa_status solve_impl(pa_solver *s, const Input &in, int method, float *scores_ou
 		r.sys = in.sy_stride;
 		r.work = in.work;
 		r.work_bytes = in.work_bytes;
+		r.dense_rows = in.dense_rows;
 		r.table = in.table;
 		r.eq = in.eq;
 		r.ne = in.ne;
@@ -3256,13 +3259,13 @@ pa_status pa_solve_dense_paths(pa_solver *s, const float *sim, const int64_t *of
                                int64_t stride_t, int64_t batch, int64_t n_s, int64_t n_t, const int32_t *length,
                                float *scores, int32_t *paths, const int64_t *path_offsets, int32_t *path_len) {
 	return pa_solve_dense_paths_work(s, sim, offsets, stride_s, stride_t, batch, n_s, n_t, length, scores, paths,
-	                                 path_offsets, path_len, nullptr, 0);
+	                                 path_offsets, path_len, 0, nullptr, 0);
 }
 
 pa_status pa_solve_dense_paths_work(pa_solver *s, const float *sim, const int64_t *offsets, int64_t stride_s,
                                     int64_t stride_t, int64_t batch, int64_t n_s, int64_t n_t, const int32_t *length,
                                     float *scores, int32_t *paths, const int64_t *path_offsets, int32_t *path_len,
-                                    void *work, int64_t work_bytes) {
+                                    int64_t rows, void *work, int64_t work_bytes) {
 	if (!s || !sim || !offsets || !length || !paths || !path_offsets || !path_len)
 		return fail(PA_ERR_INVALID_ARGUMENT, "null argument");
 	Input in{};
@@ -3276,6 +3279,7 @@ pa_status pa_solve_dense_paths_work(pa_solver *s, const float *sim, const int64_
 	in.dense_off_host = offsets;
 	in.dense_si = stride_s;
 	in.dense_sj = stride_t;
+	in.dense_rows = rows;
 	in.work = static_cast<float *>(work);
 	in.work_bytes = work_bytes;
 	UserPaths up_{};
