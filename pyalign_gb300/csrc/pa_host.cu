@@ -1628,15 +1628,19 @@ struct TuneEntry {
 std::mutex g_tune_mu;
 std::vector<TuneEntry> g_tune;
 constexpr double TUNE_MIN_CELLS = 4e6;  // smaller launches keep the analytic choice
-// Scores alone in 16 bits against int32 (pa_dps16.cuh): from here on the 16-bit kernel always won.
-// Below, a launch that leaves the GPU half empty gains nothing from two pairs per lane and pays for
-// two pairs' profiles at the head of a stripe, so the tuner times both, and below TUNE_MIN_CELLS
-// the int32 kernel runs (266 pairs of 13..27 x 51..102: 98 us a call in int32, 107 in 16 bits; 1,203
-// of 39..196 x 20..80 89 and 101; 2,647 of 35..350 x 36..144 211 and 171).
-// With one traceback the same holds (protein pairs of 50..600, chained, us a call in int32 and in
-// 16 bits: 256 pairs 338 and 355, 512 387 and 363, 1,024 470 and 425, 4,096 871 and 672; in groups
-// 65,536 8,118 and 4,907; local alignment gains less, 8,636 and 5,826), but for fewer than
-// S16_SURE_PAIRS however long: twins halve the stripes in flight.
+// 16 bits against int32 (pa_dps16.cuh).  Scores alone: from S16_SURE_CELLS on the 16-bit kernel won at
+// every size measured (2,100 to 60,000 pairs of 30..900, 8 to 300 of 1000 to 10000, 4 to 32 letters,
+// every locality: calls 1.02 to 2.07 times as fast).  Below, a launch that leaves the GPU half empty
+// gains nothing from two pairs per lane and pays for two pairs' profiles at the head of a stripe, so
+// the tuner times both, and below TUNE_MIN_CELLS the int32 kernel runs (266 pairs of 13..27 x
+// 51..102: 98 us a call in int32, 107 in 16 bits; 1,203 of 39..196 x 20..80 89 and 101; 2,647 of
+// 35..350 x 36..144 211 and 171).
+// One traceback: the same for global and semiglobal alignment (calls 1.05 to 1.5 times as fast), but
+// for fewer than S16_SURE_PAIRS however long, as twins halve the stripes in flight (protein pairs of
+// 50..600, chained, us a call in int32 and in 16 bits: 256 pairs 338 and 355, 512 387 and 363, 1,024
+// 470 and 425).  Local alignment looks for its seeds on the way and gains least, with linear gaps and
+// up to 8 letters (whose int32 profiles are in registers) it loses: 2,100 pairs of 320..400 with 5
+// letters 473 and 510 us, 30,000 of 80..100 424 and 454.  There the tuner always times both.
 constexpr double S16_SURE_CELLS = 2e8;
 constexpr size_t S16_SURE_PAIRS = 2048;
 constexpr int64_t SPREAD_MIN_CELLS = 50000000;  // smaller launches take their tasks from one counter
@@ -1713,7 +1717,8 @@ pa_status tune_plan(pa_solver *s, const std::vector<int32_t> &ls, const std::vec
 	};
 	std::vector<Cand> cand;
 	// (1,033 DNA pairs of 20..62 x 52..419, scores: int32 79 us, dp16_kernel's 4 x 4 blocks 48)
-	const bool both = plan.s16 && (cells < S16_SURE_CELLS || (plan.tb == TB_ONE && ls.size() < S16_SURE_PAIRS));
+	const bool both = plan.s16 && (cells < S16_SURE_CELLS ||
+	                               (plan.tb == TB_ONE && (ls.size() < S16_SURE_PAIRS || s->loc == LOC_LOCAL)));
 	const bool h16 = plan.h16 && (!plan.s16 || both);
 	for (int G : {32, 16, 8, 4, 2, 1})
 		if (G == 4 || (int64_t(G) * R <= 2 * plan.max_ls && (G >= 4 || plan.max_ls <= 256))) {

@@ -34,6 +34,14 @@ def indexed(letters):
     s.solve_indexed_for_score(a, b, (4.0 * np.eye(letters) - 2.0).astype(np.float32), ln)
     return launches(s)
 
+def aligned(locality):
+    rng = np.random.default_rng(1)
+    a, b = (rng.integers(0, 5, (2100, 380)).astype(np.uint32) for _ in range(2))
+    s = alg.m16.create_solver(380, 380, alg.m16.create_options(
+        options(alg, gap=Gap("linear", 2.0), locality=locality, batch_size=2100)))
+    s.solve_indexed_for_alignment(a, b, (4.0 * np.eye(5) - 2.0).astype(np.float32), np.full((2, 2100), 380, np.uint16))
+    return launches(s)
+
 def dense(transposed):
     import torch
     from pyalign_gb300 import autograd as ag
@@ -44,18 +52,31 @@ def dense(transposed):
 
 if sys.argv[3] == "letters":
     out = [indexed(4), indexed(5), indexed(5), indexed(4)]
+elif sys.argv[3] == "locality":
+    out = [aligned("global"), aligned("local")]
 else:
     out = [dense(False), dense(True), dense(True), dense(False)]
 print("RESULT", json.dumps(out))
 """
 
 
-@pytest.mark.parametrize("kind", ["letters", "layout"])
-def test_each_kind_is_tuned(kind):
+def run(kind):
     env = {k: v for k, v in os.environ.items() if not k.startswith("PA_")}
     r = subprocess.run([sys.executable, "-c", RUN, HERE, os.path.dirname(HERE), kind], env=env, capture_output=True,
                        text=True, timeout=300)
     assert r.returncode == 0, r.stderr[-2000:]
-    first, other, again, back = json.loads(r.stdout.split("RESULT")[1])
+    return json.loads(r.stdout.split("RESULT")[1])
+
+
+@pytest.mark.parametrize("kind", ["letters", "layout"])
+def test_each_kind_is_tuned(kind):
+    first, other, again, back = run(kind)
     assert first > 12 and other > 12, (first, other, again, back)
     assert again <= 6 and back <= 6, (first, other, again, back)
+
+
+def test_local_alignments_are_tried_in_int32():
+    """2,100 pairs of 380: global alignments are sure to gain from 16 bits, local ones are timed in
+    both (four widths each, twice)."""
+    globals_, locals_ = run("locality")
+    assert locals_ >= globals_ + 6, (globals_, locals_)
