@@ -126,7 +126,7 @@ struct DpParams {
 	// group mode: the first tasks spread over the SMs (next_task); null: one counter for all
 	int32_t *spread;         // SPREAD_CLASSES task counters, then 4 warp counters per SM of SPREAD_SMS, zeroed
 	int32_t spread_classes;  // classes of spread_size tasks each, the costliest first
-	int32_t spread_size;     // SMs
+	int32_t spread_size;     // SMs; negative: ranks by arrival (next_task)
 	int32_t *status;
 	// stripe-chained mode (units != 0): a ticket is one stripe of one pair; tickets are
 	// numbered stripe-major, level_start[q] is the first ticket of stripe q (nlevels + 1
@@ -204,20 +204,23 @@ static __device__ __noinline__ int32_t wait_progress(const int32_t *prog, int32_
 // and run on when the others are done (8,192 pairs of 32..512 on G = 16: one SM's ALU pipe 97%
 // busy, the average 41%).  So the first tasks go out by classes of one task per SM, as equal in
 // cost as the order makes them: rank r on an SM takes from class r, and every SM holds one task of
-// each class.  The SM's four schedulers share the classes as well: the k-th warp to start on
-// scheduler c has rank 4 k + c, or 4 k + 3 - c for odd k.  (Ranked by arrival on the SM alone, the
-// costliest tasks may meet on one scheduler.  1,000 pairs of 250..500, affine, int32: one counter
+// each class.  An SM's four schedulers share them as well: the k-th warp to start on scheduler c has
+// rank 4 k + c, or 4 k + 3 - c for odd k; with a negative size ranks go by arrival on the SM, and the
+// costliest tasks may meet on one scheduler.  (1,000 pairs of 250..500, affine, int32: one counter
 // 0.36 ms, by arrival 0.42-0.44, by schedulers 0.29; 1,024 dense pairs of 100..400, local: by arrival
-// 0.45, by schedulers 0.39.)  A warp whose class is used up takes from the next class that has a
-// task left (an SM shared with another kernel may start fewer warps than there are classes), then
-// from the counter, which holds the tasks past the classes.  Where those are all in classes the
-// surplus warps leave at once, so no SM takes more than its share; there are at least four classes,
-// so the first warp of a scheduler is never surplus.
+// 0.45, by schedulers 0.39; 3,000 pairs of 50..600, affine, int32, a fifth of which come from the
+// counter: by arrival 0.69, by schedulers 0.60.)  A warp whose class is used up takes from the
+// next class that has a task left (an SM shared with another kernel may start fewer warps than there
+// are classes), then from the counter, which holds the tasks past the classes.  Where those are
+// all in classes the surplus warps leave at once, so no SM takes more than its share; there are at
+// least four classes, so the first warp of a scheduler is never surplus.
 constexpr int SPREAD_CLASSES = 32;
 constexpr int SPREAD_SMS = 256;
 static __device__ __noinline__ int2 next_task(int32_t *counter, int32_t *spread, int nclass, int size, int ntasks,
                                               int cursor) {
 	const int lane = threadIdx.x & 31;
+	const bool share = size > 0;
+	size = abs(size);
 	int first = 0;
 	if (spread) {
 		first = nclass * size;
@@ -227,9 +230,9 @@ static __device__ __noinline__ int2 next_task(int32_t *counter, int32_t *spread,
 			asm volatile("mov.u32 %0, %%warpid;" : "=r"(warp));
 			int r = 0;
 			if (lane == 0) {
-				const int c = int(warp & 3u);
+				const int c = share ? int(warp & 3u) : 0;
 				r = atomicAdd(spread + SPREAD_CLASSES + int(smid % SPREAD_SMS) * 4 + c, 1);
-				r = 4 * r + ((r & 1) ? 3 - c : c);
+				if (share) r = 4 * r + ((r & 1) ? 3 - c : c);
 			}
 			r = __shfl_sync(0xffffffffu, r, 0);
 			if (r >= nclass && first >= ntasks) return make_int2(-1, -1);
