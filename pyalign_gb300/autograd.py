@@ -14,6 +14,7 @@ the reference's optimal path.
 
 import ctypes
 import functools
+import threading
 import types
 
 import numpy as np
@@ -21,7 +22,10 @@ import torch
 
 from . import algorithm as _alg
 
+# A solver's buffers belong to the work queued on one stream by one thread, and so do the cached
+# index arrays and the pinned buffer below: both are part of the keys.
 _SOLVERS = {}
+_lock = threading.Lock()  # around changes of the tables
 
 
 class _Gap:
@@ -40,8 +44,8 @@ class _Linear:
         return {"linear": self.g}
 
 
-def _solver(batch, n_s, n_t, locality, direction, dtw, gap):
-    key = (batch, n_s, n_t, locality, direction, dtw, gap)
+def _solver(batch, n_s, n_t, locality, direction, dtw, gap, stream):
+    key = (batch, n_s, n_t, locality, direction, dtw, gap, stream, threading.get_ident())
     s = _SOLVERS.get(key)
     if s is None:
         A = _alg
@@ -55,9 +59,10 @@ def _solver(batch, n_s, n_t, locality, direction, dtw, gap):
         }
         mod = A.m32 if max(n_s, n_t) >= 16000 else A.m16
         s = mod.create_solver(n_s, n_t, mod.create_options(d))
-        if len(_SOLVERS) > 32:
-            _SOLVERS.clear()
-        _SOLVERS[key] = s
+        with _lock:
+            if len(_SOLVERS) > 32:
+                _SOLVERS.clear()
+            _SOLVERS[key] = s
     return s
 
 
@@ -125,22 +130,27 @@ def tensor_core_status(device=None):
     return v
 
 
-_small_cache = {}   # (device, dtype, shape, content hash) -> (host copy, device tensor): index arrays seen before
-_staging = {}       # (device, dtype) -> (pinned buffer, event of its last copy)
+_small_cache = {}   # (device, stream, dtype, shape, content hash) -> (host copy, device tensor): index arrays seen before
+_staging = {}       # (thread, device, dtype) -> (pinned buffer, event of its last copy)
 
 
-def _to_device(arr, device):
+def _to_device(arr, device, stream=None):
     """A small host index array (lengths, offsets) on the device without blocking the host: a
     content-keyed cache (a training loop passes the same lengths every step; equal hashes are
-    compared in full) and, for new contents, a non-blocking copy out of a reused pinned buffer."""
+    compared in full) and, for new contents, a non-blocking copy out of a reused pinned buffer.
+    An array of one stream is not another's: its copy may still be queued there.  stream: the
+    handle of the current one, if known."""
     arr = np.ascontiguousarray(arr)
     device = torch.device(device)
-    key = (str(device), arr.dtype.str, arr.shape, _lib().pa_content_hash(arr.ctypes.data, arr.nbytes))
+    if stream is None:
+        stream = torch.cuda.current_stream(device).cuda_stream
+    key = (str(device), stream, arr.dtype.str, arr.shape, _lib().pa_content_hash(arr.ctypes.data, arr.nbytes))
     hit = _small_cache.get(key)
     if hit is not None and np.array_equal(hit[0], arr):
         return hit[1]
     dtype = torch.from_numpy(arr[:0]).dtype
-    buf, ev = _staging.get((str(device), arr.dtype.str), (None, None))
+    mine = (threading.get_ident(), str(device), arr.dtype.str)
+    buf, ev = _staging.get(mine, (None, None))
     if buf is None or buf.numel() < arr.size:
         buf, ev = torch.empty(max(arr.size, 1 << 14), dtype=dtype, pin_memory=True), None
     if ev is not None:
@@ -150,10 +160,13 @@ def _to_device(arr, device):
     out = flat.to(device, non_blocking=True).reshape(arr.shape)
     ev = torch.cuda.Event()
     ev.record(torch.cuda.current_stream(device))
-    _staging[(str(device), arr.dtype.str)] = (buf, ev)
-    if key not in _small_cache and len(_small_cache) >= 32:
-        _small_cache.pop(next(iter(_small_cache)))
-    _small_cache[key] = (arr.copy(), out)
+    with _lock:
+        if mine not in _staging and len(_staging) >= 32:
+            _staging.pop(next(iter(_staging)))
+        _staging[mine] = (buf, ev)
+        if key not in _small_cache and len(_small_cache) >= 32:
+            _small_cache.pop(next(iter(_small_cache)))
+        _small_cache[key] = (arr.copy(), out)
     return out
 
 
@@ -184,13 +197,14 @@ def _similarity_rows(Es, Et, lengths, normalize, out, plan=None):
     B, n_s, dim = Es.shape
     n_t = Et.shape[1]
     plan = plan or _Plan(lengths, B, n_s, n_t, "the embeddings", ROWS_TILE)
-    dmeta = _to_device(plan.meta, Es.device)
+    stream = torch.cuda.current_stream().cuda_stream
+    dmeta = _to_device(plan.meta, Es.device, stream)
     inv_s = torch.empty(B * n_s, dtype=torch.float32, device=Es.device)
     inv_t = torch.empty(B * n_t, dtype=torch.float32, device=Es.device)
     _alg.check(_lib().pa_similarity_rows(
         Es.data_ptr(), Et.data_ptr(), B, n_s, n_t, dim, int(normalize), dmeta.data_ptr(), dmeta.data_ptr() + 4 * B,
         dmeta.data_ptr() + 8 * B, plan.tiles, out.data_ptr(), out.stride(0), out.stride(1), inv_s.data_ptr(),
-        inv_t.data_ptr(), _status(Es.device).data_ptr(), torch.cuda.current_stream().cuda_stream))
+        inv_t.data_ptr(), _status(Es.device).data_ptr(), stream))
     return inv_s, inv_t
 
 
@@ -208,7 +222,8 @@ def similarity_bf16(Esb, Etb, lengths, out=None, alpha=1.0, beta=0.0):
     if dim % 16:
         raise ValueError("dim must be a multiple of 16")
     plan = _Plan(lengths, B, n_s, n_t, "the embeddings")
-    dmeta, total = _to_device(plan.meta, Esb.device), plan.tiles  # no host wait for the queued work
+    stream = torch.cuda.current_stream().cuda_stream
+    dmeta, total = _to_device(plan.meta, Esb.device, stream), plan.tiles  # no host wait for the queued work
     if out is None:
         out = torch.empty((B, n_t, n_s), dtype=torch.float32, device=Esb.device)
     elif out.shape != (B, n_t, n_s) or out.dtype != torch.float32 or out.stride(2) != 1 or not out.is_cuda:
@@ -217,8 +232,7 @@ def similarity_bf16(Esb, Etb, lengths, out=None, alpha=1.0, beta=0.0):
     _alg.check(_lib().pa_similarity_bf16(
         Esb.data_ptr(), Etb.data_ptr(), B, n_s, n_t, dim, dmeta.data_ptr(), dmeta.data_ptr() + 4 * B,
         dmeta.data_ptr() + 8 * B, total, out.data_ptr(), out.stride(0), out.stride(1), float(alpha), float(beta),
-        st.data_ptr(),
-        torch.cuda.current_stream().cuda_stream))
+        st.data_ptr(), stream))
     return out.transpose(1, 2)
 
 
@@ -295,7 +309,7 @@ def _forward_paths(S, lengths, gap, locality, direction, dtw, plan=None, rows=0)
     B, n_s, n_t = S.shape
     ss, st_ = S.stride(1), S.stride(2)
     plan = plan or _Plan(lengths, B, n_s, n_t, "the similarity tensor")
-    solver, ln, scores, paths, plen, poff = _path_buffers(B, n_s, n_t, plan, locality, direction, dtw, gap, S.device)
+    solver, ln, scores, paths, plen, poff, stream = _path_buffers(B, n_s, n_t, plan, locality, direction, dtw, gap, S.device)
     pair, first, ptr = S.stride(0), S.storage_offset(), S.data_ptr()
     offsets = _pair_offsets(B, first, pair)
     args = (solver.handle, ptr - 4 * first, offsets.ctypes.data, ss, st_, B, n_s, n_t, ln.ctypes.data,
@@ -312,20 +326,20 @@ def _forward_paths(S, lengths, gap, locality, direction, dtw, plan=None, rows=0)
         torch.cuda.empty_cache()
         status = L.pa_solve_dense_paths(*args)
     _alg.check(status)
-    return scores, paths, plen, _to_device(poff, S.device), ss == 1
+    return scores, paths, plen, _to_device(poff, S.device, stream), ss == 1
 
 
 def _path_buffers(B, n_s, n_t, plan, locality, direction, dtw, gap, device):
     """The solver on the current stream, the (2, B) int32 lengths and the output buffers of a
     paths solve: scores, packed paths (2 (|s| + |t| + 2) entries per pair), path lengths and
-    the host path offsets."""
-    solver = _solver(B, n_s, n_t, locality, direction, dtw, gap)
-    stream = torch.cuda.current_stream()
-    _alg.check(_lib().pa_solver_set_stream(solver.handle, ctypes.c_void_p(stream.cuda_stream)))
+    the host path offsets, and the stream's handle."""
+    stream = torch.cuda.current_stream().cuda_stream
+    solver = _solver(B, n_s, n_t, locality, direction, dtw, gap, stream)
+    _alg.check(_lib().pa_solver_set_stream(solver.handle, ctypes.c_void_p(stream)))
     paths = torch.empty(plan.entries, dtype=torch.int32, device=device)
     plen = torch.zeros(B, dtype=torch.int32, device=device)
     scores = torch.empty(B, dtype=torch.float32, device=device)
-    return solver, plan.ln, scores, paths, plen, plan.poff
+    return solver, plan.ln, scores, paths, plen, plan.poff, stream
 
 
 def _series_paths(x, y, lengths, gap, locality, direction, dtw):
@@ -334,11 +348,11 @@ def _series_paths(x, y, lengths, gap, locality, direction, dtw):
     B, n_s = x.shape
     n_t = y.shape[1]
     plan = _Plan(lengths, B, n_s, n_t, "the series")
-    solver, ln, scores, paths, plen, poff = _path_buffers(B, n_s, n_t, plan, locality, direction, dtw, gap, x.device)
+    solver, ln, scores, paths, plen, poff, stream = _path_buffers(B, n_s, n_t, plan, locality, direction, dtw, gap, x.device)
     _alg.check(_lib().pa_solve_series_paths(
         solver.handle, x.data_ptr(), x.stride(0), y.data_ptr(), y.stride(0), B, n_s, n_t, ln.ctypes.data,
         scores.data_ptr(), paths.data_ptr(), poff.ctypes.data, plen.data_ptr()))
-    return scores, paths, plen, _to_device(poff, x.device)
+    return scores, paths, plen, _to_device(poff, x.device, stream)
 
 
 def _gap_grads(linear, locality, direction, B, paths, plen, poff, grad, device):
@@ -435,7 +449,7 @@ def normalized_bf16(E, normalize=True, lengths=None, tiled=False):
         _alg.check(_lib().pa_normalize_rows_bf16(E.data_ptr(), B * n, dim, int(normalize), Eb.data_ptr(),
                                                  inv.data_ptr(), stream))
     else:
-        ln = _to_device(np.minimum(np.asarray(lengths).reshape(B), n).astype(np.int32), E.device)
+        ln = _to_device(np.minimum(np.asarray(lengths).reshape(B), n).astype(np.int32), E.device, stream)
         if tiled:
             _alg.check(_lib().pa_normalize_rows_bf16_tiled(E.data_ptr(), B, n, dim, int(normalize), ln.data_ptr(),
                                                            SIM_TILE, Eb.data_ptr(), inv.data_ptr(), stream))
