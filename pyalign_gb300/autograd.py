@@ -44,7 +44,9 @@ class _Linear:
         return {"linear": self.g}
 
 
-def _solver(batch, n_s, n_t, locality, direction, dtw, gap, stream):
+def _solver(batch, n_s, n_t, locality, direction, dtw, gap, stream=None):
+    if stream is None:
+        stream = torch.cuda.current_stream().cuda_stream
     key = (batch, n_s, n_t, locality, direction, dtw, gap, stream, threading.get_ident())
     s = _SOLVERS.get(key)
     if s is None:

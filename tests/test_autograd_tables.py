@@ -86,3 +86,10 @@ def test_two_streams_at_once(threads):
     for key, w in want.items():
         for x, y in zip(got[key], w):
             assert torch.equal(x, y), key
+
+
+@pytest.mark.gpu
+def test_the_current_stream_is_the_default():
+    import torch
+    with torch.cuda.stream(torch.cuda.Stream()):
+        assert ag._solver(*ARGS) is ag._solver(*ARGS, torch.cuda.current_stream().cuda_stream)
