@@ -33,7 +33,7 @@ def sources():
 
 
 def _deps():
-    hdr = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".cuh", ".h"))]
+    hdr = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".cuh", ".h", ".inc"))]
     hdr.append(os.path.join(os.path.dirname(HERE), "include", "pyalign_gb300.h"))
     return max(os.path.getmtime(h) for h in hdr)
 
